@@ -39,6 +39,7 @@ _SIGNATURES = {
     },
     "gemm_f32": {
         "ni_gemm_f32": [_P, _P, _P, _I, _I, _I, _P],
+        "ni_gemm_f32_variant": [_I, _P, _P, _P, _I, _I, _I, _P],
         "ni_gemm_f32_heads": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
     },
     "pointwise": {
@@ -458,14 +459,16 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         v_dim, int(chunk or 0), _f32_or_none(sink, "sink"), int(maps), _stream()), "attention_generic")
 
 
-def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = x[M, K] . w[N, K]^T, all float32, plain FP32 arithmetic."""
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, variant: int = 0) -> None:
+    """out[M, N] = x[M, K] . w[N, K]^T, all float32, plain FP32 arithmetic.  ``variant``: one of the kernels of
+    csrc/gemm_f32.cu by its number there (they give the same bits; for tests and measurements), 0: chosen by the sizes."""
     m, k = x.shape
     n = w.shape[0]
     if w.shape[1] != k or out.shape != (m, n):
         raise KernelError("gemm_f32: shapes do not agree")
-    _check(load("gemm_f32").ni_gemm_f32(_dev(x, "x", torch.float32), _dev(w, "w", torch.float32),
-                                        _dev(out, "out", torch.float32), m, n, k, _stream()), "gemm_f32")
+    args = (_dev(x, "x", torch.float32), _dev(w, "w", torch.float32), _dev(out, "out", torch.float32), m, n, k, _stream())
+    lib = load("gemm_f32")
+    _check(lib.ni_gemm_f32_variant(int(variant), *args) if variant else lib.ni_gemm_f32(*args), "gemm_f32")
 
 
 def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

@@ -119,6 +119,42 @@ def test_gemm_f32(m, n, k):
     assert torch.equal(out1[0], out[m - 1])
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (2, 17, 124), (3, 33, 132), (5, 31, 128), (8, 16, 1028), (9, 15, 64), (16, 300, 2052),
+                                   (17, 33, 252), (64, 96, 516), (65, 129, 36), (130, 100, 131), (40, 5, 7)])
+def test_gemm_f32_kernels_agree(m, n, k):
+    """Every kernel of the product (rings for few rows, tiles) at remainders of its tiles and of its k-steps: the same
+    bits, since an element is one ascending chain everywhere, and within a chain's rounding bound of the exact product."""
+    from nanoinfer_b200.kernels import ops
+    x, w = _randn(m, k, seed=1), _randn(n, k, seed=2)
+    want = x.cpu().double() @ w.cpu().double().t()
+    bound = k * 2.0 ** -24 * (x.cpu().double().abs() @ w.cpu().double().abs().t()) + 1e-30     # k roundings of partial sums
+    tile = torch.empty(m, n, dtype=torch.float32, device=DEV)
+    ops.gemm_f32(x, w, tile, variant=6)
+    assert ((tile.cpu().double() - want).abs() <= bound).all()
+    for variant in range(6):
+        out = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
+        if k % 4 and variant:
+            with pytest.raises(ops.KernelError):
+                ops.gemm_f32(x, w, out, variant=variant)          # the rings read 16 bytes at a time
+            continue
+        ops.gemm_f32(x, w, out, variant=variant)
+        assert torch.equal(out, tile), variant
+
+
+@pytest.mark.parametrize("m,k,offset", [(3, 16, 0), (3, 16, 1), (20, 12, 4), (70, 20, 2)])
+def test_gemm_f32_heads_rows_of_a_wider_matrix(m, k, offset):
+    """Rows that start off a 16-byte boundary take the scalar loads; the result is the same."""
+    from nanoinfer_b200.kernels import ops
+    h, n = 3, 37
+    wide, w = _randn(m, h * k + 9, seed=3), _randn(h, n, k, seed=4)
+    x = wide[:, offset:offset + h * k]
+    out, rows = torch.empty(m, h * n, dtype=torch.float32, device=DEV), torch.empty(m, n, dtype=torch.float32, device=DEV)
+    ops.gemm_f32_heads(x, w, out)
+    for i in range(h):
+        ops.gemm_f32(x[:, i * k:(i + 1) * k].contiguous(), w[i], rows)
+        assert torch.equal(out[:, i * n:(i + 1) * n], rows)
+
+
 def _paged_setup(T_per_seq, n_kv, hd, page, dtype, seed):
     """Random k/v for sequences of the given lengths, scattered over shuffled pages."""
     g = torch.Generator().manual_seed(seed)
