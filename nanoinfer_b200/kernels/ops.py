@@ -37,6 +37,11 @@ _SIGNATURES = {
     "attention_generic": {
         "ni_attention_generic": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _F, _I, _I, _P, _I, _P],
     },
+    "attention_f32": {
+        "ni_attention_f32_tiles": [_P, _P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _F, _P],
+        "ni_attention_f32_segments": [_I, _I, _I, _I, _LL],
+        "ni_attention_f32_rows": [_P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _F, _I, _P, _P],
+    },
     "gemm_f32": {
         "ni_gemm_f32": [_P, _P, _P, _I, _I, _I, _P],
         "ni_gemm_f32_variant": [_I, _P, _P, _P, _I, _I, _I, _P],
@@ -426,8 +431,9 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
                       page_size: int, window: Optional[int], scale: float,
                       token_list: Optional[torch.Tensor] = None, head_slopes: Optional[torch.Tensor] = None,
                       score_cap: float = 0.0, value_dim: Optional[int] = None, chunk: int = 0,
-                      sink=None, maps: int = 1) -> None:
-    """The plain attention kernel (any dtype, any head size up to 1,024).  ``token_list``
+                      sink=None, maps: int = 1, tiles=None) -> None:
+    """The plain attention kernel (any dtype, any head size up to 1,024); float32 heads of 64 and 128 with plain scores take
+    the FP32 kernels of csrc/attention_f32.cu instead (same formula; ``tiles``: see attention_f32, only for these).  ``token_list``
     int32 [n] restricts it to those tokens of the step.  ``head_slopes`` float32 [Hq] adds
     slope[h] * (key position - query position) to the scaled scores of head h.  ``score_cap`` c > 0
     bounds the scaled scores: s <- c * tanh(s / c).  ``value_dim``: the size of a value where it differs
@@ -447,6 +453,15 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         raise KernelError(f"attention: head_dim {head_dim} or value_dim {v_dim} beyond 1,024 is not supported")
     if k_pages.shape[-1] != maps * head_dim or v_pages.shape[-1] != v_dim:
         raise KernelError("attention: the pages' rows must have the keys' and the values' sizes")
+    if (q.dtype == torch.float32 and head_slopes is None and not score_cap > 0 and v_dim == head_dim and maps == 1
+            and n_q_heads > 0 and n_kv_heads > 0 and n_q_heads % n_kv_heads == 0 and page_size > 0
+            and attention_f32_supports(n_q_heads, n_kv_heads, head_dim)
+            and all(x.data_ptr() % 16 == 0 for x in (q, k_pages, v_pages, out))):
+        attention_f32(q, k_pages, v_pages, out, positions, seq_of_token, block_table, n_q_heads, n_kv_heads, head_dim, page_size,
+                      window, scale, chunk=chunk, sink=sink, token_list=token_list, tiles=tiles)
+        return
+    if tiles is not None:
+        raise KernelError("attention: tiles are for the FP32 kernels' heads")
     sink = _sinks(sink, n_q_heads, q.device)
     _check(load("attention_generic").ni_attention_generic(
         _dev(q, "q"), _code(q, "q"), _dev(k_pages, "k_pages"), _dev(v_pages, "v_pages"),
@@ -457,6 +472,47 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         int(window) if window else 0, float(scale),
         _dev(head_slopes, "head_slopes", torch.float32) if head_slopes is not None else None, float(score_cap),
         v_dim, int(chunk or 0), _f32_or_none(sink, "sink"), int(maps), _stream()), "attention_generic")
+
+
+ATTENTION_F32_HEAD_DIMS = (64, 128)
+ATTENTION_F32_MAX_GROUP = 16
+
+
+def attention_f32_supports(n_q_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    """Whether the tiled FP32 attention takes these heads (the choice must not depend on the step: its results differ from
+    attention_generic's in the last bits)."""
+    return head_dim in ATTENTION_F32_HEAD_DIMS and n_q_heads // n_kv_heads <= ATTENTION_F32_MAX_GROUP
+
+
+def attention_f32(q, k_pages, v_pages, out, positions, seq_of_token, block_table, n_q_heads, n_kv_heads, head_dim, page_size,
+                  window, scale, chunk: int = 0, sink=None, token_list: Optional[torch.Tensor] = None, tiles=None) -> None:
+    """Causal attention in FP32 (attention_generic's formula with windows, chunks and sinks; heads of 64 and 128).
+    Without ``tiles``: the tokens of ``token_list`` (default: all), one by one.  ``tiles`` = (tile_seq, tile_row0, n_tiles,
+    tile_tokens, cu_q, kv_len): tiles of query tokens of one request each.  A token's result has the same bits either way."""
+    n = q.shape[0]
+    if q.shape != (n, n_q_heads * head_dim) or out.shape != q.shape:
+        raise KernelError("attention_f32: q and out must be [T, Hq * head_dim]")
+    if k_pages.shape[-1] != head_dim or v_pages.shape[-1] != head_dim:
+        raise KernelError("attention_f32: the pages' rows must have the heads' size")
+    f32, i32 = torch.float32, torch.int32
+    operands = (_dev(q, "q", f32), _dev(k_pages, "k_pages", f32), _dev(v_pages, "v_pages", f32), _dev(out, "out", f32))
+    table = (_dev(block_table, "block_table", i32), block_table.shape[1])
+    sink = _sinks(sink, n_q_heads, q.device)
+    masks = (n_q_heads, n_kv_heads, head_dim, page_size, int(window) if window else 0, int(chunk or 0), _f32_or_none(sink, "sink"),
+             float(scale))
+    lib = load("attention_f32")
+    if tiles is not None:
+        tile_seq, tile_row0, n_tiles, tile_tokens, cu_q, kv_len = tiles
+        _check(lib.ni_attention_f32_tiles(*operands, _dev(tile_seq, "tile_seq", i32), _dev(tile_row0, "tile_row0", i32), n_tiles,
+                                          tile_tokens, _dev(cu_q, "cu_q", i32), _dev(kv_len, "kv_len", i32), *table, *masks,
+                                          _stream()), "attention_f32")
+        return
+    n_tokens = n if token_list is None else token_list.numel()
+    segments = lib.ni_attention_f32_segments(n_tokens, n_q_heads, n_kv_heads, head_dim, block_table.shape[1] * page_size)
+    partials = torch.empty(n_tokens * n_q_heads * segments * (head_dim + 2), dtype=f32, device=q.device) if segments > 1 else None
+    _check(lib.ni_attention_f32_rows(*operands, _dev(token_list, "token_list", i32) if token_list is not None else None, n_tokens,
+                                     _dev(positions, "positions", i32), _dev(seq_of_token, "seq_of_token", i32), *table, *masks,
+                                     segments, partials.data_ptr() if partials is not None else None, _stream()), "attention_f32")
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, variant: int = 0) -> None:

@@ -28,7 +28,7 @@ class PagedAttendMixin:
     TILE_ROWS = ops.PREFILL_TILE_ROWS
 
     # libraries of csrc that the attention kernels live in (the second list: on the bfloat16 path only)
-    kernel_modules = ("attention_generic",)
+    kernel_modules = ("attention_generic", "attention_f32")
     kernel_modules_bf16 = ("attention_prefill", "attention_decode")
 
     @staticmethod
@@ -59,7 +59,8 @@ class PagedAttendMixin:
     def _attend(self, q, cache, att, ctx, table) -> None:
         """Attention of every token of the step over its own request's pages.
 
-        float32: the plain kernel.  bfloat16: single query tokens (and portions of at most
+        float32: the plain kernel, which hands heads of 64 and 128 to the FP32 kernels (a token's bits do not depend on
+        which of them takes it).  bfloat16: single query tokens (and portions of at most
         two tokens) go to the split-K kernel, longer portions to the flash-style kernel;
         head sizes those do not take fall back to the plain kernel, never to a wrong result."""
         rt = self.rt
@@ -68,6 +69,18 @@ class PagedAttendMixin:
         slopes = getattr(self.position, "head_slopes", None)
         cap = float(getattr(self, "score_cap", 0.0))       # > 0: scores are bounded by cap * tanh(s / cap)
         chunk, sink = int(getattr(self, "chunk", 0) or 0), getattr(self, "sink", None)
+        if (rt.dtype == torch.float32 and slopes is None and cap == 0.0 and not ctx.decode_only
+                and ops.attention_f32_supports(self.n_heads, self.n_kv, self.head_dim)):
+            # single tokens one by one, portions in tiles (a step that was built without a plan goes token by token, below)
+            plan = next((ctx.plans[c] for c in type(self).__mro__ if c in ctx.plans), None)
+            if plan is not None and "tile_seq" in plan.arrays:
+                args = (q, cache.k_pages, cache.v_pages, att, ctx.positions, ctx.seq_of_token, table, *common)
+                if plan.scalars["n_dec"] > 0:
+                    ops.attention_generic(*args, chunk=chunk, sink=sink, token_list=plan.arrays["dec_tokens"])
+                if plan.scalars["n_tiles"] > 0:
+                    ops.attention_generic(*args, chunk=chunk, sink=sink, tiles=(
+                        plan.arrays["tile_seq"], plan.arrays["tile_row0"], plan.scalars["n_tiles"], self.TILE_ROWS, ctx.cu_q, ctx.kv_len))
+                return
         if rt.dtype != torch.bfloat16 or slopes is not None:
             # float32, or a position encoding that acts on the scores (a bias slope[h] * (k_pos - q_pos)): the plain
             # kernel takes both.  (A chunk mask and a sink are known to the split-K kernel for single tokens and to both

@@ -203,6 +203,72 @@ def test_attention_generic(dtype, n_q, n_kv, hd, page, window):
     torch.testing.assert_close(out.cpu().float(), want, **_tol(dtype))
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,page,window,chunk,sink", [
+    (4, 1, 64, 16, None, 0, False), (3, 1, 128, 8, None, 0, True), (32, 2, 64, 16, 700, 0, False), (16, 1, 128, 16, None, 600, True),
+    (2, 2, 64, 4, 63, 0, True), (10, 2, 128, 16, 65, 0, False)])
+def test_attention_f32_same_bits_one_by_one_and_in_tiles(n_q, n_kv, hd, page, window, chunk, sink):
+    """Tokens around the edges of key blocks (64) and segments (512): against float64, and the same bits whether a token
+    comes in a tile, alone with its segments split over blocks, or alone in one block.  What a token does not see - later
+    keys, keys before its window, unused places of a page - holds NaN and must not touch it."""
+    from nanoinfer_b200.kernels import ops
+    lens, starts = [1100, 1, 64, 513, 640], [1, 0, 0, 511, 600]
+    table, k_pages, v_pages, ks, vs = _paged_setup(lens, n_kv, hd, page, torch.float32, seed=hd + n_q)
+    used = torch.zeros(k_pages.shape[0], page, dtype=torch.bool)
+    for s, t in enumerate(lens):
+        for j in range(t):
+            used[table[s, j // page], j % page] = True
+    for pages in (k_pages, v_pages):
+        pages.permute(0, 2, 1, 3)[~used] = float("nan")
+    last = table[0, (lens[0] - 1) // page], (lens[0] - 1) % page          # the first request's newest key and value too
+    k_pages[last[0], :, last[1]] = float("nan")
+    v_pages[last[0], :, last[1]] = float("inf")
+    g = torch.Generator().manual_seed(5)
+    q_lens = [t - s for t, s in zip(lens, starts)]
+    positions = torch.cat([torch.arange(s, t) for s, t in zip(starts, lens)]).int()
+    seq_of = torch.cat([torch.full((n,), i) for i, n in enumerate(q_lens)]).int()
+    cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0))).int()
+    n = int(cu[-1])
+    q = torch.randn(n, n_q * hd, generator=g)
+    sinks = torch.randn(n_q, generator=g) if sink else None
+    scale = 1.0 / math.sqrt(hd)
+    common = (positions.to(DEV), seq_of.to(DEV), table.to(DEV), n_q, n_kv, hd, page, window, scale)
+    more = dict(chunk=chunk, sink=sinks.to(DEV) if sink else None)
+    qd, kd, vd = q.to(DEV), k_pages.to(DEV), v_pages.to(DEV)
+    tiles = [(i, r) for i, ql in enumerate(q_lens) for r in range(0, ql, 128)]
+    out = torch.full((n, n_q * hd), -7.0, device=DEV)
+    ops.attention_f32(qd, kd, vd, out, *common, **more, tiles=(
+        torch.tensor([t[0] for t in tiles]).int().to(DEV), torch.tensor([t[1] for t in tiles]).int().to(DEV), len(tiles), 128,
+        cu.to(DEV), torch.tensor(lens).int().to(DEV)))
+    alone = torch.full_like(out, -7.0)
+    ops.attention_f32(qd, kd, vd, alone, *common, **more)                                   # many tokens: one block each
+    few = torch.full_like(out, -7.0)
+    pick = torch.tensor([0, 61, 62, 63, 510, 511, 512, 700, 1022, 1023, 1024, 1097, 1099, 1163, 1164, n - 1]).int()
+    assert ops.load("attention_f32").ni_attention_f32_segments(pick.numel(), n_q, n_kv, hd, table.shape[1] * page) > 1
+    ops.attention_f32(qd, kd, vd, few, *common, **more, token_list=pick.to(DEV))            # few tokens: a block per segment
+    newest = q_lens[0] - 1                                      # the token that does see the NaN
+    rest = torch.arange(n) != newest
+    out, alone, few = out.cpu(), alone.cpu(), few.cpu()
+    assert torch.isnan(out[newest]).all() and torch.isnan(alone[newest]).all()
+    assert torch.equal(out[rest], alone[rest])
+    pick = pick.long()
+    assert torch.equal(few[pick[pick != newest]], out[pick[pick != newest]])
+    untouched = torch.ones(n, dtype=torch.bool)
+    untouched[pick] = False
+    assert (few[untouched] == -7.0).all()
+    for t in [i for i in range(0, n, 7) if i != newest] + [t for t in pick.tolist() if t != newest]:
+        s, pos = int(seq_of[t]), int(positions[t])
+        lo = max(0, pos - window + 1) if window else 0
+        lo = max(lo, pos - pos % chunk) if chunk else lo
+        for h in range(n_q):
+            k, v = ks[s][lo:pos + 1, h // (n_q // n_kv)].double(), vs[s][lo:pos + 1, h // (n_q // n_kv)].double()
+            sc = k @ q[t, h * hd:(h + 1) * hd].double() * scale
+            top = max(sc.max().item(), sinks[h].item()) if sink else sc.max().item()
+            e = torch.exp(sc - top)
+            want = (e @ v) / (e.sum() + (math.exp(sinks[h].item() - top) if sink else 0.0))
+            # scores of size up to ~6 rounded to 2^-24 of their terms' sum, 2 ulp of exp, sums of up to 1,100 weights
+            torch.testing.assert_close(out[t, h * hd:(h + 1) * hd].double(), want, rtol=2e-5, atol=2e-6)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,hd,page,window", [(6, 2, 48, 4, None), (5, 1, 80, 16, 33)])
 def test_attention_generic_with_a_slope_per_head(dtype, n_q, n_kv, hd, page, window):
