@@ -349,6 +349,66 @@ def test_rope_kv_write(dtype, pairing, n_q, n_kv, hd, rot, page):
     assert torch.all(vp.permute(0, 2, 1, 3)[~touched] == 7.0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n_q,n_kv,hd,rot,page", [(32, 8, 64, 64, 16), (5, 1, 128, 128, 8), (7, 2, 128, 96, 4), (3, 3, 256, 34, 16),
+                                                  (40, 8, 128, 0, 16), (2, 1, 64, 2, 16)])
+def test_rope_kv_write_a_chunk_column_per_lane(dtype, n_q, n_kv, hd, rot, page):
+    """Adjacent pairs at head sizes whose 16-byte chunks divide a warp: few and many heads, part of a head rotated."""
+    test_rope_kv_write(dtype, "interleaved", n_q, n_kv, hd, rot, page) if rot else _rope_kv_write_unrotated(dtype, n_q, n_kv, hd, page)
+
+
+def _rope_kv_write_unrotated(dtype, n_q, n_kv, hd, page):
+    from nanoinfer_b200.kernels import ops
+    n = 5
+    qkv = _randn(n, (n_q + 2 * n_kv) * hd, dtype=dtype, seed=7)
+    q, kp = torch.empty(n, n_q * hd, dtype=dtype, device=DEV), torch.zeros(1, n_kv, page, hd, dtype=dtype, device=DEV)
+    vp = torch.zeros_like(kp)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    ops.rope_kv_write(qkv, q, kp, vp, torch.arange(n, **i32), torch.zeros(n, **i32), torch.zeros(1, 1, **i32),
+                      torch.zeros(0, device=DEV), n_q, n_kv, hd, 0, True, page)
+    assert torch.equal(q, qkv[:, :n_q * hd])
+    assert torch.equal(kp[0, :, :n].transpose(0, 1).reshape(n, -1), qkv[:, n_q * hd:(n_q + n_kv) * hd])
+    assert torch.equal(vp[0, :, :n].transpose(0, 1).reshape(n, -1), qkv[:, (n_q + n_kv) * hd:])
+
+
+@pytest.mark.parametrize("types", [("f32", "f32"), ("bf16", "bf16"), ("f32", "bf16")])
+@pytest.mark.parametrize("H,G,D,V,rot,norm,unit,temperature,mix,own", [
+    (16, 8, 128, 128, 64, True, False, None, False, True), (32, 8, 128, 128, 128, True, False, (0.1, 8.0), True, True),
+    (3, 1, 48, 16, 16, True, False, None, True, True), (8, 2, 64, 64, 32, True, True, None, False, True),
+    (5, 1, 128, 64, 96, False, True, (0.3, 4.0), False, True), (63, 1, 128, 128, 0, True, True, None, False, True),
+    (4, 4, 256, 256, 256, True, False, None, False, False), (1, 1, 16, 8, 16, False, False, None, True, True)])
+def test_qk_norm_rope_rows_in_registers(types, H, G, D, V, rot, norm, unit, temperature, mix, own):
+    """The kernel that keeps a token's row in registers against the general one, which takes the same numbers where the rows
+    do not start on 16 bytes: every option, one and two items per thread, heads with a number of chunks that is no power of two."""
+    from nanoinfer_b200.kernels import ops
+    t_in, t_out = (torch.float32 if t == "f32" else torch.bfloat16 for t in types)
+    n, page, cols = 7, 4, (H + G) * D + G * V
+    data = _randn(n, cols, seed=H + D, scale=2.0).to(t_in)
+    first = _randn(n, G * V, seed=3).to(t_in)
+    bias = _randn(cols, seed=4, scale=0.5)
+    gains = (1 + _randn(H * D, seed=5, scale=0.3), 1 + _randn(G * D, seed=6, scale=0.3)) if norm else (None, None)
+    inv_freq = (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) * 2 / max(rot, 1))).float().to(DEV)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    positions, seq_of = torch.tensor([0, 1, 2, 3, 9, 10, 900], **i32), torch.tensor([0, 0, 0, 0, 1, 1, 2], **i32)
+    table = torch.zeros(3, 226, **i32)
+    table[0, 0], table[1, 2], table[2, 225] = 3, 1, 2
+    got = []
+    for extra in (8 - cols % 8, 8 - cols % 8 + 1):
+        wide = torch.zeros(n, cols + extra, dtype=t_in, device=DEV)
+        wide[:, :cols] = data
+        q = torch.zeros(n, H * D, dtype=t_out, device=DEV)
+        kp, vp = torch.zeros(5, G, page, D, dtype=t_out, device=DEV), torch.zeros(5, G, page, V, dtype=t_out, device=DEV)
+        ops.qk_norm_rope(wide, bias, *gains, 1e-5, positions, seq_of, table, inv_freq, 1.25, q, kp if own else None, vp if own else None,
+                         H, G, D, V, rot, page, head_unit=unit, temperature=temperature,
+                         first_values=(first, 0, bias[(H + G) * D:].contiguous(), 0.3) if mix else None)
+        got.append((q, kp, vp))
+    for a, b in zip(*got):
+        # the same FP32 formula; sums of squares in another order, then one rounding to the outputs' type
+        tol = dict(rtol=2e-5, atol=2e-5) if t_out == torch.float32 else dict(rtol=2.0 ** -7, atol=1e-3)
+        torch.testing.assert_close(a.float(), b.float(), **tol)
+    assert got[0][0].abs().sum() > 0
+
+
 @pytest.mark.parametrize("mode", ["bf16", "f32", "add"])
 @pytest.mark.parametrize("m,n,k", [(1, 64, 64), (3, 100, 120), (8, 4800, 2048), (9, 333, 200), (16, 520, 8200),
                                    (5, 2048, 8192), (7, 1000, 3072), (8, 600, 4096), (2, 328, 2056),
