@@ -104,6 +104,10 @@ _SIGNATURES = {
         "ni_delta_recurrence": [_P, _P, _P, _I, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "ni_delta_gated_norm": [_P, _P, _I, _I, _P, _F, _F, _I, _I, _I, _I, _I, _I, _I, _P, _I, _I, _P, _I, _I, _P, _LL, _P, _P, _P],
     },
+    "delta_block": {
+        "ni_delta_block": [_P, _I, _P, _P, _P, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P],
+        "ni_delta_block_supports": [_I, _I, _I, _I, _I],
+    },
     "delta_chunk": {
         "ni_delta_chunk_recurrence": [_P, _I, _I, _P, _P, _P, _P, _I, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _LL, _P, _P, _P],
         "ni_delta_chunk_set_wait": [_LL, _I],
@@ -663,6 +667,32 @@ def delta_gated_norm(o, proj, weight, eps, n_q_heads_kv, n_heads, dim, vdim, y, 
         _dev(y, "y") + y_col * y.element_size(), _code(y, "y"), y.shape[1], _dev(proj, "proj") + col0 * proj.element_size(),
         _code(proj, "proj"), proj.shape[1], _dev(state, "state", f32), state.shape[1], _dev(cu_q, "cu_q", torch.int32),
         _dev(slots, "slots", torch.int32), _stream()), "delta_gated_norm")
+
+
+def delta_block_supports(n_q_heads_kv: int, n_heads: int, dim: int, vdim: int, taps: int) -> bool:
+    """Whether delta_block_recurrence takes these sizes."""
+    return dim in (64, 128, 256) and vdim % 4 == 0 and 0 < taps <= 64
+
+
+def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
+                           vdim, taps, out) -> None:
+    """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another
+    order of sums): ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the
+    decay at ``b_col`` and ``a_col``.  delta_gated_norm must follow (it moves the convolution history on)."""
+    f32, i32 = torch.float32, torch.int32
+    n = proj.shape[0]
+    c = 2 * n_q_heads_kv * dim + n_heads * vdim
+    if out.shape != (n, n_heads * vdim) or conv_w.shape != (c, taps) or a_log.numel() != n_heads or dt_bias.numel() != n_heads or \
+            proj.shape[1] < max(col0 + c, b_col + n_heads, a_col + n_heads) or min(b_col, a_col) < col0 or \
+            state.shape[1] != n_heads * dim * vdim + (taps - 1) * c or cu_q.numel() != n_seqs + 1 or slots.numel() != n_seqs:
+        raise KernelError("delta_block_recurrence: shapes do not agree")
+    qkv = torch.empty(n, c, dtype=f32, device=proj.device)
+    coef = torch.empty((n // 4 + n_seqs) * n_heads * 32, dtype=f32, device=proj.device)
+    _check(load("delta_block").ni_delta_block(
+        _dev(proj, "proj") + col0 * proj.element_size(), _code(proj, "proj"), _dev(conv_w, "conv_w", f32), _dev(a_log, "a_log", f32),
+        _dev(dt_bias, "dt_bias", f32), _dev(state, "state", f32), state.shape[1], _dev(cu_q, "cu_q", i32), _dev(slots, "slots", i32), n,
+        n_seqs, n_q_heads_kv, n_heads, dim, vdim, taps, proj.shape[1], b_col - col0, a_col - col0, qkv.data_ptr(), coef.data_ptr(),
+        _dev(out, "out", f32), _stream()), "delta_block_recurrence")
 
 
 DELTA_CHUNK_MAX_DIM = 128      # the largest key size that the chunked delta rule takes

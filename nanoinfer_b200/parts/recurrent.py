@@ -33,7 +33,8 @@ class GatedDeltaRule(Part):
     second, block-diagonal product turns (W_a1 x, W_g1 x) into the logits of decay and gate in FP32.  Everything from there
     to the gated norm is FP32 on the device; in bfloat16 a step of single tokens with both options is one launch (from an
     FP32 projection, thin products included), and portions of CHUNK_FROM tokens and more run in chunks on the tensor cores
-    (csrc/delta_chunk.cu).  A request's state is one FP32 vector: M of every head, then the last
+    (csrc/delta_chunk.cu); with a decay per head portions of BLOCK_FROM tokens and more run by blocks of four tokens
+    (csrc/delta_block.cu).  A request's state is one FP32 vector: M of every head, then the last
     conv_taps - 1 inputs of every convolved channel.  A step's kernels run exactly once, so the state advances by exactly
     the step's tokens.
 
@@ -42,6 +43,7 @@ class GatedDeltaRule(Part):
     kernel_modules = ("delta_rule",)       # libraries of csrc that this part's kernels live in
 
     CHUNK_FROM = 16             # a step whose longest portion has this many tokens takes the chunked recurrence
+    BLOCK_FROM = 8              # ... with a decay per head: the recurrence by blocks of four tokens
 
     JOINS = True                # can be a side of mixers with joined projections
     takes_output_scale = True   # a factor on the output rides in the gated norm, before the output projection
@@ -153,6 +155,10 @@ class GatedDeltaRule(Part):
         self.chunked = rt.dtype == torch.bfloat16 and self.channel and d <= ops.DELTA_CHUNK_MAX_DIM and v <= 512
         if self.chunked:
             self.kernel_modules = ("delta_chunk",)
+        # (FP32 mode walks the tokens one by one: a block's sums depend on where a portion starts)
+        self.in_blocks = rt.dtype == torch.bfloat16 and not self.channel and ops.delta_block_supports(g, h, d, v, taps)
+        if self.in_blocks:
+            self.kernel_modules = ("delta_block",)
 
     def cache_need(self):
         return StateNeed((self.H * self.D * self.V + (self.taps - 1) * self.channels,), "float32")
@@ -213,6 +219,9 @@ class GatedDeltaRule(Part):
             buf = rt.workspace("delta_chunks", -(-need // 4), f32)                 # one buffer for all layers
             ops.delta_chunk_recurrence(proj, col0, col0 + self.b_col, self.conv_w, self.a_log, self.dt_bias, z, cache.state,
                                        ctx.cu_q, ctx.slots, ctx.n_seqs, ctx.max_q_len, g, h, d, v, self.taps, buf, o)
+        elif self.in_blocks and ctx.max_q_len >= self.BLOCK_FROM and proj.shape[1] % 4 == 0 and col0 % 4 == 0:
+            ops.delta_block_recurrence(proj, col0, col0 + self.b_col, col0 + self.b_col + h, self.conv_w, self.a_log, self.dt_bias,
+                                       cache.state, ctx.cu_q, ctx.slots, ctx.n_seqs, g, h, d, v, self.taps, o)
         else:
             qkv = rt.empty(n, self.channels, dtype=f32)
             gates = rt.empty(n, h, 2, dtype=f32)

@@ -202,6 +202,46 @@ def test_delta_kernels_alone(G, H, D, V, taps):
         torch.testing.assert_close(torch.cat(got[k]).double(), want, rtol=2e-4, atol=2e-5)
 
 
+@pytest.mark.parametrize("G, H, D, V, taps, fast", [(1, 1, 128, 128, 4, False), (2, 6, 64, 36, 4, False), (1, 2, 256, 68, 3, False),
+                                                    (4, 4, 128, 32, 1, True), (1, 3, 64, 4, 6, True), (8, 160, 64, 32, 4, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_delta_rule_by_blocks_of_four_tokens(G, H, D, V, taps, fast, dtype):
+    """Portions of every length modulo four, shorter than the convolution's history too, requests without tokens beside them
+    and slots out of order, in two steps: read-outs, states and histories against the kernel that walks the tokens one by one.
+    ``fast``: decays that reach zero within a block (products of stretches only, no quotients)."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(G + 10 * H + D + V)
+    C = 2 * G * D + H * V
+    b_col = C + 4
+    a_col, N = b_col + H, -(-(b_col + 2 * H) // 4) * 4
+    conv_w, i32 = (torch.randn(C, taps, generator=g) * 0.6).to(DEV), dict(dtype=torch.int32, device=DEV)
+    a_log = (torch.randn(H, generator=g) + (4.0 if fast else -2.0)).to(DEV)
+    dt_bias = torch.randn(H, generator=g).to(DEV)
+    states = [torch.zeros(9, H * D * V + (taps - 1) * C, device=DEV) for _ in range(2)]
+    slots = torch.tensor([4, 0, 7, 2, 5, 8], **i32)
+    for lens in ([9, 1, 0, 67, 2, 16], [3, 8, 5, 4, 130, 0]):
+        n = sum(lens)
+        proj = torch.randn(n, N, generator=g).to(DEV, dtype)
+        cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), **i32)
+        seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().to(DEV)
+        o = [torch.empty(n, H * V, device=DEV) for _ in range(2)]
+        qkv, gates = torch.empty(n, C, device=DEV), torch.empty(n, H, 2, device=DEV)
+        ops.delta_prepare(proj, conv_w, a_log, dt_bias, states[0], seq, cu, slots, len(lens), G, H, D, V, taps, qkv, gates, b_col=b_col)
+        ops.delta_recurrence(qkv, gates, states[0], cu, slots, len(lens), G, H, D, V, o[0])
+        ops.delta_block_recurrence(proj, 0, b_col, a_col, conv_w, a_log, dt_bias, states[1], cu, slots, len(lens), G, H, D, V, taps, o[1])
+        norm_w, gate = torch.ones(V, device=DEV), torch.ones(n, H * V, device=DEV)
+        for k in range(2):
+            ops.delta_gated_norm(o[k], proj, norm_w, 1e-5, G, H, D, V, torch.empty(n, H * V, dtype=dtype, device=DEV), states[k], cu, slots,
+                                 len(lens), taps, gate=gate, gate_col=0)
+        # sums of D terms in another order, carried along at most 130 tokens whose state neither rule lets grow
+        scale = o[0].abs().max().item()
+        torch.testing.assert_close(o[1], o[0], rtol=2e-5, atol=2e-5 * scale)
+        assert torch.equal(states[0][:, H * D * V:], states[1][:, H * D * V:])                # the histories
+        torch.testing.assert_close(states[1], states[0], rtol=2e-5, atol=2e-5 * states[0][:, :H * D * V].abs().max().item())
+        states[1].copy_(states[0])
+    assert bool((states[1][[1, 3, 6]] == 0).all())
+
+
 def _one_layer(layer, width=64, vocab=120, side=None):
     raw = {"architecture": "Runevik", "vocab": vocab, "width": width, "norm": {"eps": 1e-5}, "layers": [layer]}
     if side:
