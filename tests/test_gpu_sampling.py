@@ -72,6 +72,43 @@ def test_a_cluster_per_row_selects_the_same_tokens_as_one_block(vocab):
     assert len(set(out_b.tolist())) == 1 and out_b[0] == out_a[0]
 
 
+@pytest.mark.parametrize("vocab", [4096, 4097, 33000, 128256])
+def test_top_k_from_candidates_selects_the_same_tokens_as_one_block(vocab):
+    """Rows with top-k whose blocks send a few candidates, and rows that send too many (large k, equal logits, most of a row
+    masked with -inf) and go the general way: k from 1 to beyond what a block may send, ties at the k-th place and among the
+    probabilities, logits that differ only far behind the leading bits, negative rows, masked rows, with and without top-p."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(vocab)
+    ks = [1, 2, 50, 200, 503, 505, 3000, vocab - 1]
+    tops = [1.0, 0.9, 0.3, 0.9999999]
+    kinds = 8
+    rows = kinds * len(ks)
+    l = torch.randn(rows, vocab, generator=g) * 3.0
+    for i in range(len(ks)):
+        l[kinds * i + 1] = (l[kinds * i + 1] * 2).round() / 2                       # many ties
+        l[kinds * i + 2] = 0.25                                                     # all equal
+        l[kinds * i + 3] = 5.0 + torch.rand(vocab, generator=g) * 1e-4              # one leading value, different tails
+        l[kinds * i + 4] = -100.0 + l[kinds * i + 4]                                # all negative
+        l[kinds * i + 5, torch.randperm(vocab, generator=g)[: vocab - 120]] = -float("inf")      # masked but for 120 tokens
+        l[kinds * i + 6] = l[kinds * i + 6].abs().neg().mul(50)                     # probabilities that round to a mass of zero
+        l[kinds * i + 7, :vocab // 8] += 30.0                                       # everything that counts in the first block's slice
+    l = l.to(DEV)
+    k_t = torch.tensor([ks[r // kinds] for r in range(rows)], dtype=torch.int32, device=DEV)
+    seeds = torch.arange(rows, dtype=torch.int64, device=DEV) * 7919
+    counters = torch.arange(rows, dtype=torch.int64, device=DEV) % 5
+    temps = torch.tensor([[0.7, 1.0, 1.5][r % 3] for r in range(rows)], device=DEV)
+    for p in tops:
+        ps_ = torch.full((rows,), p, device=DEV)
+        outs = []
+        for cluster in (True, False):
+            ops.sample_by_cluster(cluster)
+            out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+            ops.sample(l, out, temps, k_t, ps_, seeds, counters)
+            outs.append(out.cpu())
+        ops.sample_by_cluster(True)
+        assert torch.equal(outs[0], outs[1]), f"rows {torch.nonzero(outs[0] != outs[1]).flatten().tolist()} differ at top-p {p}"
+
+
 @pytest.mark.parametrize("vocab", [384, 1000, 128256])
 def test_sampler_matches_plain_selection(vocab):
     from nanoinfer_b200.sampling import Sampler, SamplingParams
