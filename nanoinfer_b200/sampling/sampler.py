@@ -11,6 +11,7 @@ request's tokens do not depend on what else is in the batch.
 """
 from __future__ import annotations
 
+import struct
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -27,6 +28,7 @@ class Sampler:
         self.h2d_bytes = 0     # bytes of per-row parameters copied to the device so far
         self._dev = None       # the parameters' place on the device, and the pinned buffers they come from
         self._host, self._events, self._used, self._next = [], [], [], 0
+        self._rows, self._parts, self._pairs = -1, (), []      # views of the buffers for a batch of _rows rows
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                token_indices: Sequence[int],
@@ -72,21 +74,31 @@ class Sampler:
             self._host = [torch.empty(cap, dtype=torch.int32, pin_memory=pin) for _ in range(self._RING)]
             self._events = [torch.cuda.Event() if pin else None for _ in range(self._RING)]
             self._used = [False] * self._RING
+            self._rows = -1
         i = self._next
         self._next = (i + 1) % self._RING
         if self._used[i] and self._events[i] is not None:
             self._events[i].synchronize()          # the copy that read this buffer last has run
-        h = self._host[i][:words].numpy()
-        h[0:2 * n].view(np.int64)[:] = np.asarray(seeds, dtype=np.uint64).view(np.int64)
-        h[2 * n:4 * n].view(np.int64)[:] = np.asarray(token_indices, dtype=np.int64)
-        h[4 * n:5 * n].view(np.float32)[:] = [p.temperature for p in params]
-        h[5 * n:6 * n].view(np.float32)[:] = [p.top_p for p in params]
-        h[6 * n:7 * n] = [p.top_k for p in params]
-        d = self._dev[:words]
-        d.copy_(self._host[i][:words], non_blocking=True)
+        if self._rows != n:
+            # the places of n rows' parameters in the buffers: a server's batch stays the same size for many steps
+            d = self._dev[:words]
+            self._parts = (d[0:2 * n].view(torch.int64), d[2 * n:4 * n].view(torch.int64), d[4 * n:5 * n].view(torch.float32),
+                           d[5 * n:6 * n].view(torch.float32), d[6 * n:7 * n])
+            self._pairs = [(d, host[:words], host.numpy()) for host in self._host]
+            self._rows = n
+        d, h, words_of = self._pairs[i]
+        try:
+            struct.pack_into(f"<{n}Q{n}q{n}f{n}f{n}i", words_of, 0, *seeds, *token_indices, *(p.temperature for p in params),
+                             *(p.top_p for p in params), *(p.top_k for p in params))
+        except (OverflowError, struct.error, TypeError):        # what only the conversions of numpy take (or refuse)
+            words_of[0:2 * n].view(np.int64)[:] = np.asarray(seeds, dtype=np.uint64).view(np.int64)
+            words_of[2 * n:4 * n].view(np.int64)[:] = np.asarray(token_indices, dtype=np.int64)
+            words_of[4 * n:5 * n].view(np.float32)[:] = [p.temperature for p in params]
+            words_of[5 * n:6 * n].view(np.float32)[:] = [p.top_p for p in params]
+            words_of[6 * n:7 * n] = [p.top_k for p in params]
+        d.copy_(h, non_blocking=True)
         if self._events[i] is not None:
-            self._events[i].record()
+            self._events[i].record(ops.current_stream_object())
             self._used[i] = True
         self.h2d_bytes += 4 * words
-        return (d[0:2 * n].view(torch.int64), d[2 * n:4 * n].view(torch.int64), d[4 * n:5 * n].view(torch.float32),
-                d[5 * n:6 * n].view(torch.float32), d[6 * n:7 * n])
+        return self._parts
