@@ -574,12 +574,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 at_fence_after();
                 o_waited = true;
 #pragma unroll 1
-                for (int c = 0; c < HD / 64; ++c) {
-                    uint32_t o[32];
-                    at_ld32(t_o + 32 * c, o);
+                for (int c = 0; c < HD / 32; ++c) {     // 16 columns at a time: 32 beside the row's 64 scores spilled 64 registers
+                    uint32_t o[16];
+                    at_ld16(t_o + 16 * c, o);
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-                    at_st32(t_o + 32 * c, o);
+                    for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+                    at_st16(t_o + 16 * c, o);
                 }
             }
             // The exponentials of the two streams take turns (0, 1, 0, 1, ...), so that one
