@@ -187,7 +187,7 @@ __global__ void rope_kv_write_vec_kernel(const T* __restrict__ qkv, T* __restric
 // barrier -, and the loads of all its heads (which need no position) are on their way before the token's position, angles and
 // page are known.  A block is a token; a warp visits 32 / chunks heads at a time, ITEMS times at most before it stores.
 // Bound by the chain position -> angles -> page -> stores of a token (one wave of blocks), not yet by its bytes: 2,048 tokens
-// of 48 heads of 64 (25 MB) 9.9 -> 8.9 us, 1,914 tokens of 48 heads of 128 (47 MB) 22.4 -> 12.9 us against the table.
+// of 48 heads of 64 (25 MB) 9.9 -> 8.6 us, 1,914 tokens of 48 heads of 128 (47 MB) 22.4 -> 12.9 us against the table.
 template <typename T, int ITEMS>
 __global__ void __launch_bounds__(256)
 rope_kv_write_lanes_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages,
@@ -257,16 +257,20 @@ NI_EXPORT int ni_rope_kv_write(const void* qkv, int dtype, void* q_out, void* k_
         return NI_ERR_BAD_ARGUMENT;
     const int chunks = head_dim / 8;
     if (interleaved && head_dim % 8 == 0 && chunks >= 2 && chunks <= 32 && (chunks & (chunks - 1)) == 0) {
-        // two groups of heads per warp (a warp's worth of chunks each), up to 8 warps: four (fewer warps and angles per token)
-        // took 14.6 against 12.9 us for 1,914 tokens of 48 heads of 128, and 8.6 against 8.9 us for 2,048 of 48 heads of 64
+        // groups of heads (a warp's worth of chunks each) per warp: four where that leaves up to four warps, else two over up
+        // to eight warps.  1,914 tokens of 48 heads of 128 (24 groups): 14.6 us with four, 12.9 with two; 2,048 tokens of 48 heads
+        // of 64 (12 groups): 8.6 with four (fewer warps compute the angles), 8.9 with two
         int log_chunks = 0;
         while ((1 << log_chunks) < chunks) ++log_chunks;
         const int groups = ((n_q_heads + 2 * n_kv_heads) * chunks + 31) / 32;
-        const int warps = groups <= 2 ? 1 : (groups + 1) / 2 <= 8 ? (groups + 1) / 2 : 8;
+        const int warps = groups <= 16 ? (groups + 3) / 4 : (groups + 1) / 2 <= 8 ? (groups + 1) / 2 : 8;
 #define LAUNCHL(T)                                                                                     \
-    rope_kv_write_lanes_kernel<T, 2><<<n_tokens, 32 * warps, 0, stream>>>(                              \
-        (const T*)qkv, (T*)q_out, (T*)k_pages, (T*)v_pages, positions, seq_of_token, block_table,     \
-        bt_stride, inv_freq, n_q_heads, n_kv_heads, head_dim, log_chunks, rotary_dim, page_size, write_cache)
+    do {                                                                                               \
+        auto kernel = groups <= 16 ? rope_kv_write_lanes_kernel<T, 4> : rope_kv_write_lanes_kernel<T, 2>; \
+        kernel<<<n_tokens, 32 * warps, 0, stream>>>(                                                   \
+            (const T*)qkv, (T*)q_out, (T*)k_pages, (T*)v_pages, positions, seq_of_token, block_table, \
+            bt_stride, inv_freq, n_q_heads, n_kv_heads, head_dim, log_chunks, rotary_dim, page_size, write_cache); \
+    } while (0)
         if (dtype == NI_DTYPE_F32) LAUNCHL(float);
         else if (dtype == NI_DTYPE_BF16) LAUNCHL(__nv_bfloat16);
         else return NI_ERR_BAD_ARGUMENT;
