@@ -259,6 +259,252 @@ lightning_chunk_out_kernel(const T* __restrict__ proj, int ld, const int* __rest
     }
 }
 
+// ---- FP32 rows of whole 16-byte groups, key sizes up to 128: the same two chunk kernels with packed multiply-adds --------
+// Loads are asynchronous and in the order of their use (the state before the chunk arrives in the keys' place while the
+// scores meet the values), neighbouring dimensions or columns are the two halves of a packed multiply-add (each half an
+// IEEE chain of its own), and two read-out blocks share an SM.  Bound by shared memory (128 bytes per clock whatever lanes
+// share): 12 loads of 16 bytes for 128 multiply-adds.  2,048 tokens in two requests, 8 heads of 128: read-outs 75 -> 43 us, sums
+// 26.5 -> 20 us against blocks of 256 threads that loaded everything first.
+__device__ __forceinline__ void lf_copy16(float* dst, const float* src, bool live) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int n = live ? 16 : 0;                                // 0: sixteen bytes of zeros, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void lf_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long lf_pair(float a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ float2 lf_split(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+// Columns [0, cols) of rows [0, rows) of src into dst, zeros up to rows_pad x cols_pad (multiples of 4); the same thread gets
+// the same pieces in lf_apply, which turns what it copied itself into f(r, value).
+template <int THREADS>
+__device__ __forceinline__ void lf_load(const float* __restrict__ src, size_t ld, int rows, int rows_pad, int cols, int cols_pad,
+                                        float* __restrict__ dst, int dst_stride) {
+    const int per_row = cols_pad / 4;
+    for (int i = threadIdx.x; i < rows_pad * per_row; i += THREADS) {
+        const int r = i / per_row, c = 4 * (i - r * per_row);
+        const bool live = r < rows && c < cols;
+        lf_copy16(dst + r * dst_stride + c, live ? src + (size_t)r * ld + c : src, live);
+    }
+}
+template <int THREADS, typename F>
+__device__ __forceinline__ void lf_apply(int rows, int cols_pad, float* __restrict__ dst, int dst_stride, F f) {
+    const int per_row = cols_pad / 4;
+    for (int i = threadIdx.x; i < rows * per_row; i += THREADS) {
+        const int r = i / per_row, c = 4 * (i - r * per_row);
+        float4 v = *reinterpret_cast<float4*>(dst + r * dst_stride + c);
+        v.x = f(r, v.x); v.y = f(r, v.y); v.z = f(r, v.z); v.w = f(r, v.w);
+        *reinterpret_cast<float4*>(dst + r * dst_stride + c) = v;
+    }
+}
+__device__ __forceinline__ void lf_powers(float* pw, float dec) {
+    float p = 1.0f;
+    for (int i = 0; i <= LT_C; ++i) { pw[i] = p; p *= dec; }
+}
+
+// One 64 x 64 tile of a chunk's sum: 128 threads of 4 x 8.  Grid as lightning_chunk_kv_kernel.
+#define LF_KV_THREADS 128
+template <bool SILU>
+__global__ void __launch_bounds__(LF_KV_THREADS)
+lightning_chunk_kv_f32_kernel(const float* __restrict__ proj, int ld, const int* __restrict__ cu_q, const float* __restrict__ decay,
+                              float* __restrict__ buf, int H, int D, int V, int d_tiles, int v_tiles) {
+    __shared__ __align__(16) float Ks[LT_C][LT_KV_TILE];
+    __shared__ __align__(16) float Vs[LT_C][LT_KV_TILE];
+    __shared__ float pw[LT_C + 1];
+    __shared__ int base_s;
+    const int tid = threadIdx.x, head = blockIdx.y, seq = blockIdx.z;
+    const int chunk = blockIdx.x / (d_tiles * v_tiles), tile = blockIdx.x % (d_tiles * v_tiles);
+    const int d0 = (tile / v_tiles) * LT_KV_TILE, v0 = (tile % v_tiles) * LT_KV_TILE;
+    const int t0 = cu_q[seq], t1 = cu_q[seq + 1];
+    const int c0 = t0 + chunk * LT_C;
+    if (c0 >= t1) return;
+    const int n = min(LT_C, t1 - c0);
+    const float* row0 = proj + (size_t)c0 * ld;
+    lf_load<LF_KV_THREADS>(row0 + (size_t)(H + head) * D + d0, ld, n, n, min(LT_KV_TILE, D - d0), LT_KV_TILE, &Ks[0][0], LT_KV_TILE);
+    lf_load<LF_KV_THREADS>(row0 + (size_t)2 * H * D + (size_t)head * V + v0, ld, n, n, min(LT_KV_TILE, V - v0), LT_KV_TILE, &Vs[0][0], LT_KV_TILE);
+    lt_cp_async_commit();
+    if (tid == 0) lf_powers(pw, decay[head]);
+    const int base = lt_chunk_base(cu_q, seq, &base_s);         // (its barriers publish the powers)
+    lt_cp_async_wait<0>();
+    if (SILU) lf_apply<LF_KV_THREADS>(n, LT_KV_TILE, &Ks[0][0], LT_KV_TILE, [&](int, float x) { return lt_silu(x); });
+    lf_apply<LF_KV_THREADS>(n, LT_KV_TILE, &Vs[0][0], LT_KV_TILE, [&](int r, float x) { return (SILU ? lt_silu(x) : x) * pw[n - 1 - r]; });   // decayed to the chunk's end
+    __syncthreads();
+    const int vg = 4 * (tid & 7), dg = 4 * (tid >> 3);          // columns also 32 further on
+    unsigned long long acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+        const float4 k0 = *reinterpret_cast<const float4*>(&Ks[j][dg]);
+        const ulonglong2 v0p = *reinterpret_cast<const ulonglong2*>(&Vs[j][vg]), v1p = *reinterpret_cast<const ulonglong2*>(&Vs[j][vg + 32]);
+        const float kk[4] = {k0.x, k0.y, k0.z, k0.w};
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const unsigned long long k2 = lf_pair(kk[a]);
+            lf_fma2(acc[a][0], k2, v0p.x);
+            lf_fma2(acc[a][1], k2, v0p.y);
+            lf_fma2(acc[a][2], k2, v1p.x);
+            lf_fma2(acc[a][3], k2, v1p.y);
+        }
+    }
+    float* out = buf + ((size_t)(base + chunk) * H + head) * D * V;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int d = d0 + dg + a;
+        if (d >= D) continue;
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int v = v0 + vg + 32 * g;                     // V is a multiple of 4
+            if (v >= V) continue;
+            const float2 x = lf_split(acc[a][2 * g]), y = lf_split(acc[a][2 * g + 1]);
+            *reinterpret_cast<float4*>(out + (size_t)d * V + v) = make_float4(x.x, x.y, y.x, y.y);
+        }
+    }
+}
+
+// A chunk's read-outs for 64 value columns: 128 threads; a thread owns rows ty + 8 i and keys tx + 16 j of the scores (so that
+// every thread has as many below the diagonal), then the same rows and columns 4 tx .. 4 tx + 3 of the read-out.  (64 threads
+// of 8 x 8 read shared memory less often per multiply-add, but two warps per block wait for one another: 56 us.)
+#define LF_OUT_THREADS 128
+#define LF_VT 64
+template <bool SILU>
+__global__ void __launch_bounds__(LF_OUT_THREADS)
+lightning_chunk_out_f32_kernel(const float* __restrict__ proj, int ld, const int* __restrict__ cu_q, const float* __restrict__ decay,
+                               const float* __restrict__ buf, float* __restrict__ out, int H, int D, int V, int v_tiles) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float pw[LT_C + 1];
+    __shared__ int base_s;
+    constexpr int AS = LT_C + 4;
+    const int QS = D + 4;                    // row stride of Qs / Ks: neighbouring rows start 4 banks apart
+    float* Qs = sm;                          // [LT_C][QS]
+    float* Ks = Qs + LT_C * QS;              // [LT_C][QS], later the state before the chunk [D][LF_VT] (not larger: D + 4 > D)
+    float* Vs = Ks + LT_C * QS;              // [LT_C][LF_VT]
+    float* As = Vs + LT_C * LF_VT;           // [LT_C][AS]
+    const int tid = threadIdx.x, head = blockIdx.y, seq = blockIdx.z;
+    const int chunk = blockIdx.x / v_tiles, v0 = (blockIdx.x % v_tiles) * LF_VT;
+    const int t0 = cu_q[seq], t1 = cu_q[seq + 1];
+    const int c0 = t0 + chunk * LT_C;
+    if (c0 >= t1) return;
+    const int n = min(LT_C, t1 - c0), vt = min(LF_VT, V - v0);
+    const float* row0 = proj + (size_t)c0 * ld;
+    lf_load<LF_OUT_THREADS>(row0 + (size_t)head * D, ld, n, LT_C, D, D, Qs, QS);
+    lf_load<LF_OUT_THREADS>(row0 + (size_t)(H + head) * D, ld, n, LT_C, D, D, Ks, QS);
+    lt_cp_async_commit();
+    lf_load<LF_OUT_THREADS>(row0 + (size_t)2 * H * D + (size_t)head * V + v0, ld, n, LT_C, vt, LF_VT, Vs, LF_VT);
+    lt_cp_async_commit();
+    if (tid == 0) lf_powers(pw, decay[head]);
+    const int base = lt_chunk_base(cu_q, seq, &base_s);         // (its barriers publish the powers)
+    lt_cp_async_wait<1>();
+    if (SILU) {
+        lf_apply<LF_OUT_THREADS>(n, D, Qs, QS, [&](int, float x) { return lt_silu(x); });
+        lf_apply<LF_OUT_THREADS>(n, D, Ks, QS, [&](int, float x) { return lt_silu(x); });
+    }
+    __syncthreads();
+    const int tx = tid & 15, ty = tid >> 4;
+    // ---- scores: A[t, j] = (q_t . k_j) p[t - j], zero above the diagonal; key block j meets rows from 16 j on: i >= 2 j
+    {
+        unsigned long long acc[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        const float* qp = Qs + ty * QS;
+        const float* kp = Ks + tx * QS;
+#pragma unroll 2
+        for (int d = 0; d < D; d += 4) {
+            ulonglong2 kv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const ulonglong2*>(kp + 16 * j * QS + d);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qp + 8 * i * QS + d);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (i >= 2 * j) {
+                        lf_fma2(acc[i][j], qv.x, kv[j].x);
+                        lf_fma2(acc[i][j], qv.y, kv[j].y);
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i >= 2 * j) {
+                    const int t = ty + 8 * i, k = tx + 16 * j;
+                    const float2 x = lf_split(acc[i][j]);
+                    As[t * AS + k] = k <= t ? (x.x + x.y) * pw[t - k] : 0.f;
+                }
+    }
+    lt_cp_async_wait<0>();
+    if (SILU) lf_apply<LF_OUT_THREADS>(n, LF_VT, Vs, LF_VT, [&](int, float x) { return lt_silu(x); });
+    __syncthreads();                                            // scores and values are there, the keys have been read
+    lf_load<LF_OUT_THREADS>(buf + ((size_t)(base + chunk) * H + head) * D * V + v0, V, D, D, vt, LF_VT, Ks, LF_VT);
+    lt_cp_async_commit();
+    // ---- read-out: o_t = sum_(j <= t) A[t, j] v_j + p[t + 1] S0^T q_t
+    unsigned long long intra[8][2], inter[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) intra[i][0] = intra[i][1] = inter[i][0] = inter[i][1] = 0ull;
+#pragma unroll
+    for (int jb = 0; jb < 4; ++jb)
+#pragma unroll 1
+        for (int j = 16 * jb; j < 16 * jb + 16; j += 4) {
+            ulonglong2 wv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) wv[u] = *reinterpret_cast<const ulonglong2*>(Vs + (j + u) * LF_VT + 4 * tx);
+#pragma unroll
+            for (int i = 2 * jb; i < 8; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(As + (ty + 8 * i) * AS + j);
+                const float aa[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned long long a2 = lf_pair(aa[u]);
+                    lf_fma2(intra[i][0], a2, wv[u].x);
+                    lf_fma2(intra[i][1], a2, wv[u].y);
+                }
+            }
+        }
+    lt_cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll 1
+    for (int d = 0; d < D; d += 4) {
+        ulonglong2 sv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sv[u] = *reinterpret_cast<const ulonglong2*>(Ks + (d + u) * LF_VT + 4 * tx);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 q = *reinterpret_cast<const float4*>(Qs + (ty + 8 * i) * QS + d);
+            const float qq[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned long long q2 = lf_pair(qq[u]);
+                lf_fma2(inter[i][0], q2, sv[u].x);
+                lf_fma2(inter[i][1], q2, sv[u].y);
+            }
+        }
+    }
+    if (4 * tx >= vt) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = ty + 8 * i;
+        if (t >= n) continue;
+        const float f = pw[t + 1];
+        const float2 a = lf_split(intra[i][0]), b = lf_split(intra[i][1]), c = lf_split(inter[i][0]), e = lf_split(inter[i][1]);
+        *reinterpret_cast<float4*>(out + (size_t)(c0 + t) * H * V + (size_t)head * V + v0 + 4 * tx) =
+            make_float4(fmaf(f, c.x, a.x), fmaf(f, c.y, a.y), fmaf(f, e.x, b.x), fmaf(f, e.y, b.y));
+    }
+}
+
 // ---- bfloat16 projections: the same two chunk kernels on tensor cores ------------------------------------------------
 // mma.sync m16n8k16 (bfloat16 operands, FP32 accumulation).  q, k and v enter as the bfloat16 roundings of their
 // activations.  Whatever the design keeps in 32 bits and a product has to read again - the decayed scores, the state
@@ -807,6 +1053,26 @@ NI_EXPORT int ni_lightning_recurrence(const void* proj, int dtype, int ld, float
             }
             NI_RETURN_LAUNCH_STATUS();
         }
+    }
+    // FP32 rows on 16 bytes, keys that leave room for two blocks per SM
+    const auto on16 = [](const void* p) { return (reinterpret_cast<size_t>(p) & 15) == 0; };
+    if ((activation == 0 || dtype == NI_DTYPE_F32) && D % 4 == 0 && V % 4 == 0 && D <= 128 && ld % 4 == 0 && on16(proj) && on16(buf) && on16(out)) {
+        const size_t smem_f32 = ((size_t)2 * LT_C * (D + 4) + (size_t)LT_C * LF_VT + (size_t)LT_C * (LT_C + 4)) * sizeof(float);
+        const int out_tiles = (V + LF_VT - 1) / LF_VT;
+        const float* x = (const float*)proj;
+#define LAUNCH_F32(SILU)                                                                                                 \
+    do {                                                                                                                 \
+        const cudaError_t e = cudaFuncSetAttribute(lightning_chunk_out_f32_kernel<SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f32); \
+        if (e != cudaSuccess) return (int)e;                                                                             \
+        lightning_chunk_kv_f32_kernel<SILU><<<grid_kv, LF_KV_THREADS, 0, stream>>>(x, ld, cu_q, decay, buf, H, D, V, d_tiles, kv_tiles); \
+        lightning_scan_kernel<<<grid_scan, LT_THREADS, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, 0, H, D, V); \
+        lightning_chunk_out_f32_kernel<SILU><<<dim3(per_seq * out_tiles, H, n_seqs), LF_OUT_THREADS, smem_f32, stream>>>( \
+            x, ld, cu_q, decay, before, out, H, D, V, out_tiles);                                                        \
+    } while (0)
+        if (activation == 0) LAUNCH_F32(false);
+        else LAUNCH_F32(true);
+#undef LAUNCH_F32
+        NI_RETURN_LAUNCH_STATUS();
     }
 #define LAUNCH(T)                                                                                                        \
     do {                                                                                                                 \

@@ -328,6 +328,13 @@ def test_lightning_recurrence_alone(dtype, H, D, V, pad):
     torch.testing.assert_close(y.double().cpu(), want_y, **_tol(dtype))
 
 
+@pytest.mark.parametrize("H, D, V, pad", [(2, 4, 4, 0), (2, 124, 68, 4), (1, 128, 60, 0), (3, 64, 132, 8)])
+def test_lightning_fp32_chunks_at_the_edges_of_their_tiles(H, D, V, pad):
+    """FP32 rows on 16 bytes take the kernels with packed multiply-adds: the smallest sizes, and tiles that end inside."""
+    test_lightning_recurrence_alone(torch.float32, H, D, V, pad)
+
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rowwise_kernels_and_the_squared_unit(dtype):
     from nanoinfer_b200.config.model_config import FeedForwardSpec
