@@ -164,7 +164,15 @@ gemm_f32_ring_kernel(const float* __restrict__ x, const float* __restrict__ w, f
     const int lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
     const int chunks = (K + KC - 1) / KC;
-    if (threadIdx.x >= 32) {                                    // the fetching warp
+    // Blocks of two warps fill an SM's warp slots, and with them its four schedulers, as 0 1, 2 3, 0 1, 2 3.  A block in slots 4
+    // to 7 (8 to 11 as 0 to 3, and so on) lets its other warp multiply, so that four blocks multiply on four schedulers instead
+    // of two: 177 rows x [2048, 8192] 346 -> 263 us, 16 rows x [16384, 2048] 67 -> 54 us.  (Which warp it is changes no result;
+    // the slot is only read to spread the work.)
+    __shared__ unsigned gr_slot;
+    if (threadIdx.x == 0) asm volatile("mov.u32 %0, %%warpid;" : "=r"(gr_slot));
+    __syncthreads();
+    const int multiplier = (gr_slot >> 2) & 1;
+    if ((int)(threadIdx.x >> 5) != multiplier) {                // the fetching warp
         const int row = lane / GROUPS, col = 4 * (lane % GROUPS);
         const bool whole = n0 + BN <= N && m0 + BM <= M;        // every row of the tile exists
         const float* wp = w + (size_t)(n0 + row) * K + col;
@@ -293,16 +301,16 @@ static int gf_launch_ring(const float* x, const float* w, float* out, int M, int
 
 // Up to 16 rows the narrowest ring that holds them all: weights are read once.  Beyond, the ring's 32 x 16 tiles (three
 // blocks per SM) or the 64 x 128 tiles, whichever is done first by what they measured at K = 2,048 (both go with K):
-// a ring tile takes 34 us alone and 0.1 us each once the SMs are full, a 64 x 128 tile 128 us and 0.64 us.  [2048, K] weights:
-// 64 rows 38 / 130 us, 177 rows 93 / 130 us, 256 rows 110 / 130 us, 512 rows 205 / 130 us; [16384, K]: 17 rows 115 / 130 us,
-// 64 rows 212 / 132 us.  Before (64 x 64 tiles of 4 x 4 outputs per thread, one k-step of 16 at a time): 190 us and up
-// for any few rows, [16384, K] at 2,048 rows 5,863 us against 2,620 us (0.70 of the FMA rate).
+// a ring tile takes 34 us alone and 0.077 us each once the SMs are full, a 64 x 128 tile 128 us and 0.64 us.  [2048, K]
+// weights: 64 rows 37 / 130 us, 177 rows 74 / 130 us, 256 rows 99 / 130 us, 512 rows 200 / 130 us; [16384, K]: 17 rows
+// 103 / 130 us, 64 rows 170 / 132 us.  Before (64 x 64 tiles of 4 x 4 outputs per thread, one k-step of 16 at a time): 190 us and
+// up for any few rows, [16384, K] at 2,048 rows 5,863 us against 2,620 us (0.70 of the FMA rate).
 static int gf_choose(int M, int N, int H, bool vec) {
     if (!vec) return GF_TILE;
     if (M <= 16) return M <= 2 ? GF_RING_2 : M <= 4 ? GF_RING_4 : M <= 8 ? GF_RING_8 : GF_RING_16;
     const double fill = 148.0 / ni_sm_count();
     const double ring = (double)((N + 31) / 32) * ((M + 15) / 16) * H * fill, tile = (double)((N + 127) / 128) * ((M + 63) / 64) * H * fill;
-    const double ring_us = 8.0 + 0.1 * ring, tile_us = 50.0 + 0.64 * tile;
+    const double ring_us = 14.0 + 0.077 * ring, tile_us = 50.0 + 0.64 * tile;
     return (ring_us > 34.0 ? ring_us : 34.0) <= (tile_us > 128.0 ? tile_us : 128.0) ? GF_RING_32x16 : GF_TILE;
 }
 
