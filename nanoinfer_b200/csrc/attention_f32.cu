@@ -29,7 +29,7 @@ struct AfParams {
     float* out;
     const int *block_table, *positions, *seq_of_token;
     const float* sinks;
-    int bt_stride, n_q, n_kv, group, page, window, chunk;
+    int bt_stride, n_q, n_kv, group, page, page_shift, window, chunk;      // page_shift: -1 where the page size is no power of two
     float scale;
 };
 
@@ -76,7 +76,10 @@ __device__ __forceinline__ void af_fetch(const AfParams& p, const int* table, in
         const int row = i / G16, c = 4 * (i % G16), key = b * AF_KB + row;
         const bool live = key >= from && key <= to;
         size_t at = 0;
-        if (live) at = (((size_t)table[key / p.page] * p.n_kv + kvh) * p.page + key % p.page) * HD + c;
+        if (live) {
+            const int page = p.page_shift >= 0 ? key >> p.page_shift : key / p.page;
+            at = (((size_t)table[page] * p.n_kv + kvh) * p.page + (key - page * p.page)) * HD + c;
+        }
         af_copy16(ks + row * PITCH + c, p.k + at, live);
         af_copy16(vs + row * PITCH + c, p.v + at, live);
     }
@@ -163,41 +166,63 @@ attention_f32_tile_kernel(AfParams p, const int* __restrict__ tile_seq, const in
         }
         const int key = b * AF_KB + tx;
         const bool edge = b * AF_KB + AF_KB - 1 > pos_first || b * AF_KB < af_first(p, pos_last) || rows < ROWS;
+        // (the rows side by side in every step: a row's four exchanges and its exponentials are a chain of their own)
+        float s[RM][4], top[RM];
 #pragma unroll
         for (int i = 0; i < RM; ++i) {
-            float s[4];
-            bool seen[4];
-            float top = -INFINITY;
+            top[i] = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                seen[j] = !edge || (key + 16 * j <= pos[i] && key + 16 * j >= lo[i]);
-                s[j] = seen[j] ? af_score(s2[i][j], p.scale) : -INFINITY;
-                top = fmaxf(top, s[j]);
+                const bool seen = !edge || (key + 16 * j <= pos[i] && key + 16 * j >= lo[i]);
+                s[i][j] = seen ? af_score(s2[i][j], p.scale) : -INFINITY;
+                top[i] = fmaxf(top[i], s[i][j]);
             }
+        }
 #pragma unroll
-            for (int o = 1; o < 16; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-            const float m_new = fmaxf(m[i], top), corr = af_factor(m[i], m_new);
+        for (int o = 1; o < 16; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < RM; ++i) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
+        float sum[RM];
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+            const float m_new = fmaxf(m[i], top[i]), corr = af_factor(m[i], m_new);
             float w[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                w[j] = seen[j] ? expf(s[j] - m_new) : 0.f;
+                const bool seen = !edge || (key + 16 * j <= pos[i] && key + 16 * j >= lo[i]);
+                w[j] = seen ? expf(s[i][j] - m_new) : 0.f;
                 ps[(r0 + i) * PP + tx + 16 * j] = w[j];
             }
-            float sum = __fadd_rn(__fadd_rn(w[0], w[1]), __fadd_rn(w[2], w[3]));
-#pragma unroll
-            for (int o = 1; o < 16; o <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
-            l[i] = fmaf(l[i], corr, sum);
+            sum[i] = __fadd_rn(__fadd_rn(w[0], w[1]), __fadd_rn(w[2], w[3]));
             m[i] = m_new;
+            top[i] = corr;
 #pragma unroll
             for (int d = 0; d < 2 * DV; ++d) {
                 const float2 a = af_split(acc[i][d]);
                 acc[i][d] = af_pair(af_scale(a.x, corr), af_scale(a.y, corr));
             }
         }
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < RM; ++i) sum[i] = __fadd_rn(sum[i], __shfl_xor_sync(0xffffffffu, sum[i], o));
+#pragma unroll
+        for (int i = 0; i < RM; ++i) l[i] = fmaf(l[i], top[i], sum[i]);
         __syncwarp();                                      // a half warp reads only the rows it has written itself
         const float* vb = vs + buf * AF_KB * PITCH + 4 * tx;
         const float* pb = ps + r0 * PP;
-        if (!edge) {
+        // a key that a row does not see has the weight 0 there, which leaves the row alone unless its value is not a number or
+        // infinite: then (never, in a sound model) the row must not touch it at all
+        bool plain = true;
+        if (edge) {
+            bool odd = false;
+            for (int i = threadIdx.x; i < AF_KB * (HD / 4); i += AF_THREADS) {
+                const float4 v = *reinterpret_cast<const float4*>(vs + buf * AF_KB * PITCH + (i / (HD / 4)) * PITCH + 4 * (i % (HD / 4)));
+                odd |= !(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w));
+            }
+            plain = !__syncthreads_or(odd);
+        }
+        if (plain) {
 #pragma unroll 2
             for (int j = 0; j < AF_KB; j += 4) {
                 float4 w[RM];
@@ -218,7 +243,6 @@ attention_f32_tile_kernel(AfParams p, const int* __restrict__ tile_seq, const in
                     }
             }
         } else {
-            // a key that a row does not see must not touch it, whatever its value holds (0 times infinity)
             for (int j = 0; j < AF_KB; ++j) {
                 const int at = b * AF_KB + j;
 #pragma unroll
@@ -447,7 +471,8 @@ static int af_params(AfParams& p, const float* q, const float* k, const float* v
     if (n_q <= 0 || n_kv <= 0 || n_q % n_kv || page <= 0 || chunk < 0) return NI_ERR_BAD_ARGUMENT;
     if ((head_dim != 64 && head_dim != 128) || n_q / n_kv > AF_MAX_GROUP || n_kv > 65535) return NI_ERR_UNSUPPORTED_SIZE;
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) % 16) return NI_ERR_BAD_ARGUMENT;
-    p = AfParams{q, k, v, out, block_table, positions, seq_of_token, sinks, bt_stride, n_q, n_kv, n_q / n_kv, page, window, chunk, scale};
+    const int shift = (page & (page - 1)) == 0 ? __builtin_ctz((unsigned)page) : -1;
+    p = AfParams{q, k, v, out, block_table, positions, seq_of_token, sinks, bt_stride, n_q, n_kv, n_q / n_kv, page, shift, window, chunk, scale};
     return NI_OK;
 }
 
