@@ -127,6 +127,62 @@ __global__ void lightning_scan_kernel(float* __restrict__ state, long long state
     *S = s;
 }
 
+// The same with four neighbouring numbers per thread (D V a multiple of 4, everything on 16 bytes): a quarter of the threads
+// with 16 bytes each per load keep more of the chunks' sums on their way.  2,048 tokens of 16 heads of 128 (67 MB through L2):
+// 9.7 us against 16.8 us with one number per thread.
+__global__ void lightning_scan4_kernel(float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
+                                       const int* __restrict__ slots, const float* __restrict__ decay,
+                                       const float* __restrict__ sums, float* __restrict__ before, int split, int H, int D, int V) {
+    constexpr int AHEAD = 8;
+    __shared__ int base_s;
+    const int head = blockIdx.y, seq = blockIdx.z;
+    const int len = cu_q[seq + 1] - cu_q[seq];
+    if (len <= 0) return;
+    const int base = lt_chunk_base(cu_q, seq, &base_s);
+    const int e = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (e >= D * V) return;
+    const float dec = decay[head];
+    float p_full = 1.0f;
+    for (int i = 0; i < LT_C; ++i) p_full *= dec;
+    float4* S = reinterpret_cast<float4*>(state + (size_t)slots[seq] * state_stride + (size_t)head * D * V + e);
+    float4 s = *S;
+    const size_t stride = (size_t)H * D * V, first = ((size_t)base * H + head) * D * V;
+    const float* b = sums + first + e;
+    float* o32 = before + first + e;
+    __nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(before + first) + e;
+    const int chunks = (len + LT_C - 1) / LT_C;
+    for (int c = 0; c < chunks; c += AHEAD) {
+        float4 own[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            own[i] = c + i < chunks ? *reinterpret_cast<const float4*>(b + (size_t)(c + i) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (c + i >= chunks) break;
+            const int n = min(LT_C, len - (c + i) * LT_C);
+            float pn = p_full;
+            if (n < LT_C) {
+                pn = 1.0f;
+                for (int k = 0; k < n; ++k) pn *= dec;
+            }
+            if (split) {                           // what the chunk's read-out starts from
+                uint2 hi, lo;
+                lt_split2(s.x, s.y, hi.x, lo.x);
+                lt_split2(s.z, s.w, hi.y, lo.y);
+                *reinterpret_cast<uint2*>(o16 + (size_t)(c + i) * stride * 2) = hi;
+                *reinterpret_cast<uint2*>(o16 + (size_t)(c + i) * stride * 2 + (size_t)D * V) = lo;
+            } else {
+                *reinterpret_cast<float4*>(o32 + (size_t)(c + i) * stride) = s;
+            }
+            s.x = fmaf(pn, s.x, own[i].x);
+            s.y = fmaf(pn, s.y, own[i].y);
+            s.z = fmaf(pn, s.z, own[i].z);
+            s.w = fmaf(pn, s.w, own[i].w);
+        }
+    }
+    *S = s;
+}
+
 // grid (chunks of the longest request x column tiles of VT, H, requests); buf holds the state before every chunk
 template <typename T, int VT>
 __global__ void __launch_bounds__(LT_THREADS)
@@ -1024,6 +1080,13 @@ NI_EXPORT int ni_lightning_recurrence(const void* proj, int dtype, int ld, float
     const int d_tiles = (D + LT_KV_TILE - 1) / LT_KV_TILE, kv_tiles = (V + LT_KV_TILE - 1) / LT_KV_TILE, v_tiles = (V + VT - 1) / VT;
     dim3 grid_kv(per_seq * d_tiles * kv_tiles, H, n_seqs), grid_scan((D * V + LT_THREADS - 1) / LT_THREADS, H, n_seqs),
         grid_out(per_seq * v_tiles, H, n_seqs);
+    const bool scan4 = D * V % 4 == 0 && state_stride % 4 == 0 && ((reinterpret_cast<size_t>(state) | reinterpret_cast<size_t>(buf)) & 15) == 0;
+    const auto scan = [&](int split) {
+        if (scan4)
+            lightning_scan4_kernel<<<dim3((D * V / 4 + 127) / 128, H, n_seqs), 128, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, split, H, D, V);
+        else
+            lightning_scan_kernel<<<grid_scan, LT_THREADS, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, split, H, D, V);
+    };
     const bool tc = dtype == NI_DTYPE_BF16 && D % 16 == 0 && V % 16 == 0 && ld % 8 == 0 &&
                     (reinterpret_cast<size_t>(proj) & 15) == 0 && (reinterpret_cast<size_t>(buf) & 15) == 0 &&
                     (reinterpret_cast<size_t>(out) & 7) == 0;
@@ -1041,7 +1104,7 @@ NI_EXPORT int ni_lightning_recurrence(const void* proj, int dtype, int ld, float
             const __nv_bfloat16* p = (const __nv_bfloat16*)proj;
             cudaFuncSetAttribute(lightning_chunk_kv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_kv);
             lightning_chunk_kv_tc_kernel<<<dim3(per_seq, H, n_seqs), LT_THREADS, smem_kv, stream>>>(p, ld, cu_q, decay, buf, H, D, V);
-            lightning_scan_kernel<<<grid_scan, LT_THREADS, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, 1, H, D, V);
+            scan(1);
             if (VT == 128) {
                 cudaFuncSetAttribute(lightning_chunk_out_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out);
                 lightning_chunk_out_tc_kernel<128><<<dim3(per_seq * vt_tiles, H, n_seqs), 256, smem_out, stream>>>(
@@ -1065,7 +1128,7 @@ NI_EXPORT int ni_lightning_recurrence(const void* proj, int dtype, int ld, float
         const cudaError_t e = cudaFuncSetAttribute(lightning_chunk_out_f32_kernel<SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f32); \
         if (e != cudaSuccess) return (int)e;                                                                             \
         lightning_chunk_kv_f32_kernel<SILU><<<grid_kv, LF_KV_THREADS, 0, stream>>>(x, ld, cu_q, decay, buf, H, D, V, d_tiles, kv_tiles); \
-        lightning_scan_kernel<<<grid_scan, LT_THREADS, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, 0, H, D, V); \
+        scan(0); \
         lightning_chunk_out_f32_kernel<SILU><<<dim3(per_seq * out_tiles, H, n_seqs), LF_OUT_THREADS, smem_f32, stream>>>( \
             x, ld, cu_q, decay, before, out, H, D, V, out_tiles);                                                        \
     } while (0)
@@ -1078,7 +1141,7 @@ NI_EXPORT int ni_lightning_recurrence(const void* proj, int dtype, int ld, float
     do {                                                                                                                 \
         lightning_chunk_kv_kernel<T><<<grid_kv, LT_THREADS, 0, stream>>>((const T*)proj, ld, cu_q, decay, buf, H, D, V,  \
                                                                          d_tiles, kv_tiles);                             \
-        lightning_scan_kernel<<<grid_scan, LT_THREADS, 0, stream>>>(state, state_stride, cu_q, slots, decay, buf, before, 0, H, D, V); \
+        scan(0); \
         if (VT == 64) {                                                                                                  \
             cudaFuncSetAttribute(lightning_chunk_out_kernel<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             lightning_chunk_out_kernel<T, 64><<<grid_out, LT_THREADS, smem, stream>>>((const T*)proj, ld, cu_q, decay, before, \
@@ -1156,6 +1219,80 @@ linear_attention_prepare_kernel(const T* __restrict__ proj, int ld, const int* _
     for (int i = threadIdx.x; i < nv; i += blockDim.x) o[nqk + i] = ni_to_float(x[nqk + i]);
 }
 
+// The same with 16-byte accesses: a thread turns 8 dimensions of a head's first rotated half and their 8 partners (or 16
+// unrotated ones), the first of which it asks for before the angles are known; values 8 at a time.  D and rotary_dim multiples
+// of 16, V of 8, everything on 16 bytes.  2,048 tokens of 8 heads of 128 (38 MB): 9.3 us
+// against 15 us number by number.
+template <typename T> __device__ __forceinline__ void lp_load8(const T* p, float* v) {
+#pragma unroll
+    for (int k = 0; k < 8; k += NiVec16<T>::N) NiVec16<T>::load(p + k, v + k);
+}
+__device__ __forceinline__ void lp_store8(float* p, const float* v) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+template <typename T>
+__global__ void __launch_bounds__(128)
+linear_attention_prepare_vec_kernel(const T* __restrict__ proj, int ld, const int* __restrict__ positions,
+                                    const float* __restrict__ inv_freq, float k_scale, float* __restrict__ qkv, int H, int D, int V,
+                                    int rotary_dim) {
+    extern __shared__ __align__(16) float cs[];          // [rotary_dim]: cosines, then sines
+    const int t = blockIdx.x, half = rotary_dim >> 1, nqk = 2 * H * D, nv = H * V;
+    const int per_head = D >> 4, rotated = rotary_dim >> 4, items = 2 * H * per_head;
+    const T* x = proj + (size_t)t * ld;
+    float* o = qkv + (size_t)t * (nqk + nv);
+    float a[8], b[8];
+    auto place = [&](int i, int& other) {
+        const int head = i / per_head, c = i - head * per_head;
+        other = c < rotated ? half : 8;
+        return head * D + (c < rotated ? 8 * c : rotary_dim + 16 * (c - rotated));
+    };
+    int other = 0, at = 0;
+    if ((int)threadIdx.x < items) {
+        at = place(threadIdx.x, other);
+        lp_load8<T>(x + at, a);
+        lp_load8<T>(x + at + other, b);
+    }
+    const float pos = (float)positions[t];
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+        float s, c;
+        sincosf(pos * inv_freq[i], &s, &c);
+        cs[i] = c;
+        cs[half + i] = s;
+    }
+    for (int i = threadIdx.x * 8; i < nv; i += blockDim.x * 8) {      // the values wait for nothing
+        float v[8];
+        lp_load8<T>(x + nqk + i, v);
+        lp_store8(o + nqk + i, v);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < items; i += blockDim.x) {
+        if (i != (int)threadIdx.x) {
+            at = place(i, other);
+            lp_load8<T>(x + at, a);
+            lp_load8<T>(x + at + other, b);
+        }
+        const int c = i % per_head;
+        if (c < rotated) {
+            float co[8], si[8];
+            lp_load8<float>(cs + 8 * c, co);
+            lp_load8<float>(cs + half + 8 * c, si);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float p = a[k], q = b[k];
+                a[k] = p * co[k] - q * si[k];
+                b[k] = q * co[k] + p * si[k];
+            }
+        }
+        if (at >= H * D) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { a[k] *= k_scale; b[k] *= k_scale; }
+        }
+        lp_store8(o + at, a);
+        lp_store8(o + at + other, b);
+    }
+}
+
 NI_EXPORT int ni_linear_attention_prepare(const void* proj, int dtype, int ld, const int* positions, const float* inv_freq,
                                           float k_scale, float* qkv, int n_tokens, int H, int D, int V, int rotary_dim,
                                           cudaStream_t stream) {
@@ -1165,7 +1302,15 @@ NI_EXPORT int ni_linear_attention_prepare(const void* proj, int dtype, int ld, c
     const size_t smem = (size_t)(rotary_dim > 0 ? rotary_dim : 1) * sizeof(float);
     if (smem > 48 * 1024) return NI_ERR_UNSUPPORTED_SIZE;
     const int threads = 2 * H * D >= 1024 ? 256 : 128;
-    if (dtype == NI_DTYPE_F32)
+    const bool wide = D % 16 == 0 && rotary_dim % 16 == 0 && V % 8 == 0 && ld % 8 == 0 &&
+                      ((reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(qkv)) & 15) == 0;
+    if (wide && dtype == NI_DTYPE_F32)
+        linear_attention_prepare_vec_kernel<float><<<n_tokens, 128, smem, stream>>>((const float*)proj, ld, positions, inv_freq, k_scale,
+                                                                                    qkv, H, D, V, rotary_dim);
+    else if (wide && dtype == NI_DTYPE_BF16)
+        linear_attention_prepare_vec_kernel<__nv_bfloat16><<<n_tokens, 128, smem, stream>>>((const __nv_bfloat16*)proj, ld, positions,
+                                                                                            inv_freq, k_scale, qkv, H, D, V, rotary_dim);
+    else if (dtype == NI_DTYPE_F32)
         linear_attention_prepare_kernel<float><<<n_tokens, threads, smem, stream>>>((const float*)proj, ld, positions, inv_freq,
                                                                                     k_scale, qkv, H, D, V, rotary_dim);
     else if (dtype == NI_DTYPE_BF16)
@@ -1229,6 +1374,32 @@ __global__ void group_gated_norm_kernel(const float* __restrict__ o, const T* __
     }
 }
 
+// Heads of 128 in bfloat16: four neighbours per lane, a head's numbers, gates and weights asked for together, several heads
+// per warp in flight through the block's warps.  2,048 tokens of 8 heads (16 MB): 6.1 us against 10 us number by number.
+__global__ void __launch_bounds__(256)
+group_gated_norm_128_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ proj, int ld, int col0,
+                            const float* __restrict__ weight, float eps, __nv_bfloat16* __restrict__ y, int n_tokens, int groups,
+                            int gate_act, float scale) {
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= (long long)n_tokens * groups) return;
+    const int t = (int)(item / groups), c = (int)(item - (long long)t * groups) * 128 + 4 * (threadIdx.x & 31);
+    const float4 x = *reinterpret_cast<const float4*>(o + (size_t)t * groups * 128 + c);
+    const uint2 graw = *reinterpret_cast<const uint2*>(proj + (size_t)t * ld + col0 + c);
+    const float4 w = weight ? *reinterpret_cast<const float4*>(weight + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+    const float ss = ni_warp_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))));
+    const float inv = scale / sqrtf(ss / 128.0f + eps);
+    const float2 g0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.x));
+    const float2 g1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&graw.y));
+    const auto gate = [&](float z) {
+        const float sig = 1.0f / (1.0f + expf(-z));
+        return gate_act ? z * sig : sig;
+    };
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(x.x * inv * w.x * gate(g0.x), x.y * inv * w.y * gate(g0.y));
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(x.z * inv * w.z * gate(g1.x), x.w * inv * w.w * gate(g1.y));
+    *reinterpret_cast<uint2*>(y + (size_t)t * groups * 128 + c) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+
 NI_EXPORT int ni_group_gated_norm(const float* o, const void* proj, int dtype, int ld, int col0, const float* weight,
                                   float eps, void* y, int n_tokens, int groups, int V, int gate_act, float scale,
                                   cudaStream_t stream) {
@@ -1236,6 +1407,13 @@ NI_EXPORT int ni_group_gated_norm(const float* o, const void* proj, int dtype, i
     if (groups <= 0 || V <= 0 || col0 < 0 || (long long)col0 + (long long)groups * V > ld || (gate_act != 0 && gate_act != 1))
         return NI_ERR_BAD_ARGUMENT;
     const int threads = groups >= 8 ? 256 : (groups >= 4 ? 128 : 64);
+    const long long blocks128 = ((long long)n_tokens * groups + 7) / 8;
+    if (dtype == NI_DTYPE_BF16 && V == 128 && ld % 8 == 0 && col0 % 8 == 0 && blocks128 <= 2147483647LL &&
+        ((reinterpret_cast<size_t>(o) | reinterpret_cast<size_t>(proj) | reinterpret_cast<size_t>(weight) | reinterpret_cast<size_t>(y)) & 15) == 0) {
+        group_gated_norm_128_kernel<<<(int)blocks128, 256, 0, stream>>>(o, (const __nv_bfloat16*)proj, ld, col0, weight, eps,
+                                                                        (__nv_bfloat16*)y, n_tokens, groups, gate_act, scale);
+        NI_RETURN_LAUNCH_STATUS();
+    }
     if (dtype == NI_DTYPE_F32)
         group_gated_norm_kernel<float><<<n_tokens, threads, 0, stream>>>(o, (const float*)proj, ld, col0, weight, eps, (float*)y,
                                                                          groups, V, gate_act, scale);

@@ -334,6 +334,70 @@ def test_lightning_fp32_chunks_at_the_edges_of_their_tiles(H, D, V, pad):
     test_lightning_recurrence_alone(torch.float32, H, D, V, pad)
 
 
+@pytest.mark.parametrize("H, D, V", [(2, 64, 64), (1, 128, 128), (3, 4, 8), (1, 16, 200)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_chunk_scan_by_four_numbers_is_the_scan_by_one(dtype, H, D, V):
+    """States on 16 bytes are scanned four numbers at a time, others one by one: the same arithmetic, the same bits.  Portions
+    of one chunk, of more chunks than the scan asks for at once, and one that ends inside a chunk."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + V)
+    lens = [64, 700, 5]
+    n, cols = sum(lens), H * (2 * D + 2 * V)
+    proj = torch.randn(n, cols + (-cols) % 8, generator=g).to(dtype).to(DEV)
+    start = torch.randn(3, H * D * V, generator=g)
+    decay = torch.tensor([0.99, 0.6, 1.0][:H], device=DEV)
+    cu = torch.tensor([0, 64, 764, 769], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([2, 0, 1], dtype=torch.int32, device=DEV)
+    got = []
+    for extra in (0, 1):
+        state = torch.zeros(3, H * D * V + extra, device=DEV)
+        state[:, :H * D * V] = start.to(DEV)
+        out = torch.empty(n, H * V, device=DEV)
+        ops.lightning_recurrence(proj, state, cu, slots, 3, decay, H, D, V, out)
+        got.append((out, state[:, :H * D * V]))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("H, D, V, rot", [(2, 16, 8, 16), (3, 128, 40, 64), (1, 48, 16, 0), (10, 128, 128, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rotated_rows_by_16_bytes_are_the_rows_number_by_number(dtype, H, D, V, rot):
+    """Rows on 16 bytes take the wide kernel, others the general one: the same numbers (more items than threads too)."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + V + rot)
+    n, cols = 5, H * (2 * D + V)
+    data = torch.randn(n, cols, generator=g).to(dtype)
+    positions = torch.tensor([0, 1, 77, 5000, 3], dtype=torch.int32, device=DEV)
+    inv_freq = (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) * 2 / max(rot, 1))).float().to(DEV)
+    got = []
+    for pad in ((-cols) % 8, (-cols) % 8 + 1):
+        proj = torch.zeros(n, cols + pad, dtype=dtype, device=DEV)
+        proj[:, :cols] = data.to(DEV)
+        qkv = torch.full((n, cols), float("nan"), device=DEV)
+        ops.linear_attention_prepare(proj, positions, inv_freq, 0.37, qkv, H, D, V, rot)
+        got.append(qkv)
+    torch.testing.assert_close(got[0], got[1], rtol=1e-6, atol=1e-6)          # one rounding: a product contracted or not
+
+
+@pytest.mark.parametrize("groups", [1, 3, 8])
+@pytest.mark.parametrize("gate, weighted", [("silu", False), ("sigmoid", True)])
+def test_group_norm_of_heads_of_128_is_the_general_one(groups, gate, weighted):
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(groups)
+    n, cols = 9, groups * 128
+    o = torch.randn(n, cols, generator=g).to(DEV)
+    w = (1 + 0.3 * torch.randn(cols, generator=g)).to(DEV) if weighted else None
+    z = torch.randn(n, cols, generator=g).to(torch.bfloat16).to(DEV)
+    got = []
+    for col0 in (8, 9):                                                        # 9: the gates do not start on 16 bytes
+        proj = torch.zeros(n, cols + 16, dtype=torch.bfloat16, device=DEV)
+        proj[:, col0:col0 + cols] = z
+        y = torch.empty(n, cols, dtype=torch.bfloat16, device=DEV)
+        ops.group_gated_norm(o, proj, col0, w, 1e-5, y, 128, gate=gate, scale=0.7)
+        got.append(y.float())
+    torch.testing.assert_close(got[0], got[1], rtol=2.0 ** -7, atol=1e-6)      # the last bit of bfloat16
+
+
+
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rowwise_kernels_and_the_squared_unit(dtype):
