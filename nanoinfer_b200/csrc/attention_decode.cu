@@ -129,13 +129,17 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
                         float scale_log2e, float cap_l2, int n_splits, float* __restrict__ scratch,
                         int* __restrict__ tickets, const unsigned char* __restrict__ warm_a, unsigned long long warm_a_bytes,
                         const unsigned char* __restrict__ warm_b, unsigned long long warm_b_bytes, int chunk,
-                        const float* __restrict__ sinks, int share_heads, const DecDiff diff) {
+                        const float* __restrict__ sinks, int share_heads, const DecDiff diff, int n_items) {
     // more than 16 query rows over one page head are dealt over several "kv heads" of at most 16 rows each
     const int share = share_heads > 1 ? share_heads : 1;
     // Weights that the kernels after this one will read (the caller's hint, up to two regions): asked
     // into L2 now, in pieces dealt over the blocks, while this kernel - which waits on latencies
     // more than on bandwidth - leaves the memory system room.  Nothing here depends on the kernel before.
     if (threadIdx.x >= (DEC_WARPS - 1) * 32) dec_warm(warm_a, warm_a_bytes);
+    if ((int)blockIdx.x >= n_items) {        // a block (with CL: a whole cluster) without a token: it only asks (see dec_extra_items)
+        if (threadIdx.x >= (DEC_WARPS - 1) * 32) dec_warm(warm_b, warm_b_bytes);
+        return;
+    }
     constexpr int CH = HD / 8;       // 16-byte chunks per row
     constexpr int KS = HD / 16;      // k-steps over the head size
     constexpr int NT_O = HD / 8;     // output column tiles
@@ -868,6 +872,22 @@ NI_EXPORT int ni_attention_decode_balanced(const void* q, const void* k_pages, c
     }
 }
 
+// Items without a token that a launch with weights to ask for gets besides its own, so that the requests come from as many
+// SMs as the GPU has.  Requests of one SM are served one after the other: 16 MB asked for by the 8 blocks of a lone short
+// request (8 kv heads, one split) kept those blocks - and the product that waits for them - several us beyond their few
+// keys.  Up to three blocks per SM in all, which is what is resident at once, so no block with a token waits for one without.
+// Sixteen tokens generated for one request of 33, ms with 0 / 148 / 296 / 444 blocks: 12.38 / 10.81 / 10.77 / 10.77 (nothing
+// asked for at all: 10.91); four requests of 20 to 60: 12.71 / 11.55 / 11.32 / 11.09 (11.27); eight of 17 to 301: 14.35 /
+// 13.78 / 13.73 / 13.73 (14.08); one of 900, which is cut into four splits: 13.99 / 14.02 / 13.96 / 13.87 (13.70).
+// Only while the launch's own blocks fill at most every second SM: beyond that they ask from enough places, and their longer
+// streams only get company.  A layer of width 4,096 with heads of 128, one token at 500 keys (16 blocks): 40.0 us without,
+// 33.9 with; four at 20 to 3,000 (384 blocks): 39.9 and 42.0.  Eight requests of 700 (128 blocks), sixteen tokens: 21.5 ms
+// without, 21.6 with, which is as far as two runs of one side lie apart.
+static int dec_extra_items(int n_items, int n_kv_heads, int n_splits, unsigned long long warm_bytes) {
+    const long long per_item = (long long)n_kv_heads * n_splits, own = n_items * per_item, sms = ni_sm_count();
+    return warm_bytes && 2 * own <= sms ? (int)((3 * sms - own) / per_item) : 0;
+}
+
 template <int HD, int SEG, bool CL, bool CAP, bool DIFF>
 static int launch_decode_cl(const void* q, const void* k_pages, const void* v_pages, void* out, const int* token_list,
                          int n_items, const int* positions, const int* seq_of_token, const int* block_table,
@@ -889,7 +909,7 @@ static int launch_decode_cl(const void* q, const void* k_pages, const void* v_pa
         configured = smem;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_items, n_kv_heads, n_splits);
+    cfg.gridDim = dim3(n_items + dec_extra_items(n_items, n_kv_heads, n_splits, warm_a_bytes + warm_b_bytes), n_kv_heads, n_splits);
     cfg.blockDim = dim3(DEC_WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -911,7 +931,7 @@ static int launch_decode_cl(const void* q, const void* k_pages, const void* v_pa
                                        (__nv_bfloat16*)out, token_list, positions, seq_of_token, block_table,
                                        bt_stride, n_q_heads, n_kv_heads, page_size, window, scale_log2e, cap_l2, n_splits,
                                        scratch, tickets, (const unsigned char*)warm_a, warm_a_bytes,
-                                       (const unsigned char*)warm_b, warm_b_bytes, chunk, sinks, share, diff);
+                                       (const unsigned char*)warm_b, warm_b_bytes, chunk, sinks, share, diff, n_items);
     return e == cudaSuccess ? NI_OK : (int)e;
 }
 

@@ -594,6 +594,36 @@ def test_a_request_to_warm_l2_changes_no_result():
     assert torch.equal(later, keep)
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,n_splits,cluster", [(32, 8, 64, 1, True), (8, 8, 128, 1, True), (32, 8, 64, 3, True),
+                                                           (32, 8, 64, 3, False), (16, 1, 64, 12, True),
+                                                           (16, 8, 64, 4, True), (16, 8, 64, 5, True)])
+@pytest.mark.parametrize("items", [1, 2])
+def test_attention_decode_with_blocks_that_only_ask(n_q, n_kv, hd, n_splits, cluster, items):
+    """With weights to ask for, a launch of few blocks gets items without a token (whole clusters of them where the splits
+    merge in one; with 2 x 8 x 4 blocks yes and with 2 x 8 x 5 no, on 148 SMs): the same bits, the tickets at zero,
+    rows beyond the items and the weights untouched."""
+    from nanoinfer_b200.kernels import ops
+    lens = [700, 33]
+    spans = [(t - 1, t) for t in lens]
+    table, k_pages, v_pages, _, _, _, q, positions, seq_of = _attention_case(lens, spans, n_q, n_kv, hd, 16, hd + n_splits)
+    dev = [t.to(DEV) for t in (q, k_pages, v_pages, positions, seq_of, table)]
+    weights = torch.arange(3_000_001, dtype=torch.int32, device=DEV)
+    ops.attention_decode_cluster_merge(cluster)
+    outs = []
+    for warm in [(), ((weights, 0, 1 << 30), (weights, 4096, 1 << 20)), (None, (weights, 16, 8208))]:
+        out = torch.full_like(dev[0], 9.0)
+        scratch = torch.full((items * n_q * n_splits * (hd + 2),), float("nan"), dtype=torch.float32, device=DEV)
+        tickets = torch.zeros(items * n_kv, dtype=torch.int32, device=DEV)
+        ops.attention_decode(dev[0], dev[1], dev[2], out, None, items, dev[3], dev[4], dev[5], n_q, n_kv, hd, 16, None, 0.125,
+                             n_splits, scratch, tickets, warm=warm)
+        assert torch.all(tickets == 0) and torch.all(out[items:] == 9.0)
+        outs.append(out)
+    ops.attention_decode_cluster_merge(True)
+    assert torch.isfinite(outs[0].float()).all()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert torch.equal(weights, torch.arange(3_000_001, dtype=torch.int32, device=DEV))
+
+
 def test_gemv_refuses_what_it_cannot_take():
     from nanoinfer_b200.kernels import ops
     x = _randn(17, 64, dtype=torch.bfloat16)
