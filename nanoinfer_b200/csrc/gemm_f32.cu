@@ -311,6 +311,7 @@ static int gf_choose(int M, int N, int H, bool vec) {
     const double fill = 148.0 / ni_sm_count();
     const double ring = (double)((N + 31) / 32) * ((M + 15) / 16) * H * fill, tile = (double)((N + 127) / 128) * ((M + 63) / 64) * H * fill;
     const double ring_us = 14.0 + 0.077 * ring, tile_us = 50.0 + 0.64 * tile;
+    if ((M + 15) / 16 > 65535) return GF_TILE;                  // more row tiles of 16 than a grid has room for
     return (ring_us > 34.0 ? ring_us : 34.0) <= (tile_us > 128.0 ? tile_us : 128.0) ? GF_RING_32x16 : GF_TILE;
 }
 

@@ -141,6 +141,23 @@ def test_gemm_f32_kernels_agree(m, n, k):
         assert torch.equal(out, tile), variant
 
 
+@pytest.mark.parametrize("m", [1_048_560, 1_048_561, 1_048_577])
+@pytest.mark.parametrize("heads", [None, 2])
+def test_gemm_f32_narrow_products_of_very_many_rows(m, heads):
+    """Few columns go to the ring of 32 x 16 tiles as long as its row tiles fit a grid, and to the wider tiles beyond."""
+    from nanoinfer_b200.kernels import ops
+    k, h = 4, heads or 1
+    x, w = _randn(m, h * k, seed=1), _randn(h, 1, k, seed=2)
+    out = torch.full((m, h), float("nan"), dtype=torch.float32, device=DEV)
+    if heads:
+        ops.gemm_f32_heads(x, w, out)
+    else:
+        ops.gemm_f32(x, w[0], out)
+    want = (x.view(m, h, k).double() * w[:, 0].double()).sum(-1)
+    bound = k * 2.0 ** -24 * (x.view(m, h, k).double() * w[:, 0].double()).abs().sum(-1) + 1e-30      # k roundings of partial sums
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("m,k,offset", [(3, 16, 0), (3, 16, 1), (20, 12, 4), (70, 20, 2)])
 def test_gemm_f32_heads_rows_of_a_wider_matrix(m, k, offset):
     """Rows that start off a 16-byte boundary take the scalar loads; the result is the same."""
