@@ -272,15 +272,17 @@ def _stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-_stream_objects: Dict[int, "torch.cuda.Stream"] = {}
+_stream_objects: Dict[tuple, "torch.cuda.Stream"] = {}
 
 
 def current_stream_object() -> "torch.cuda.Stream":
-    """torch's current stream as an object (for Event.record), cached by raw handle."""
-    raw = _stream()
-    obj = _stream_objects.get(raw)
+    """torch's current stream of the current device as an object (for Event.record), cached by device and raw handle (the
+    default stream's handle is 0 on every device)."""
+    device = torch._C._cuda_getDevice()
+    key = (device, torch._C._cuda_getCurrentRawStream(device))
+    obj = _stream_objects.get(key)
     if obj is None:
-        obj = _stream_objects[raw] = torch.cuda.current_stream()
+        obj = _stream_objects[key] = torch.cuda.current_stream(device)
     return obj
 
 

@@ -45,3 +45,16 @@ def test_tensor_core_prefill_attention_cases():
     assert not ops.attention_prefill_tc_supports(8, 2, 96, 16)      # head size
     assert not ops.attention_prefill_tc_supports(8, 2, 64, 4)       # page size
     assert not ops.attention_prefill_tc_supports(8, 2, 64, 48)
+
+
+def test_stream_objects_belong_to_their_device(monkeypatch):
+    """The default stream has the raw handle 0 on every device: an event must be recorded on the current device's stream."""
+    import torch
+    place = {"device": 0, "raw": 0}
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: place["device"], raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: place["raw"], raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: (place["device"], place["raw"]))
+    monkeypatch.setattr(ops, "_stream_objects", {})
+    for device, raw in [(0, 0), (1, 0), (1, 77), (0, 77), (0, 0), (1, 0)]:
+        place.update(device=device, raw=raw)
+        assert ops.current_stream_object() == (device, raw)
