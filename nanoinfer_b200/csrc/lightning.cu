@@ -329,6 +329,10 @@ __device__ __forceinline__ void lf_copy16(float* dst, const float* src, bool liv
 __device__ __forceinline__ void lf_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+// The same where `live`, as a predicate of the instruction: no branch, and nothing of a or b reaches acc otherwise.
+__device__ __forceinline__ void lf_fma2_if(unsigned long long& acc, unsigned long long a, unsigned long long b, bool live) {
+    asm("{\n.reg .pred p;\nsetp.ne.s32 p, %3, 0;\n@p fma.rn.f32x2 %0, %1, %2, %0;\n}" : "+l"(acc) : "l"(a), "l"(b), "r"((int)live));
+}
 __device__ __forceinline__ unsigned long long lf_pair(float a) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
@@ -525,8 +529,14 @@ lightning_chunk_out_f32_kernel(const float* __restrict__ proj, int ld, const int
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const unsigned long long a2 = lf_pair(aa[u]);
-                    lf_fma2(intra[i][0], a2, wv[u].x);
-                    lf_fma2(intra[i][1], a2, wv[u].y);
+                    if (i < 2 * jb + 2) {                       // the two row groups that the diagonal crosses: beyond it the weight is
+                        const bool live = j + u <= ty + 8 * i;  // 0, but 0 times a later token's infinity is not
+                        lf_fma2_if(intra[i][0], a2, wv[u].x, live);
+                        lf_fma2_if(intra[i][1], a2, wv[u].y, live);
+                    } else {
+                        lf_fma2(intra[i][0], a2, wv[u].x);
+                        lf_fma2(intra[i][1], a2, wv[u].y);
+                    }
                 }
             }
         }

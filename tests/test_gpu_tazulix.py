@@ -334,6 +334,29 @@ def test_lightning_fp32_chunks_at_the_edges_of_their_tiles(H, D, V, pad):
     test_lightning_recurrence_alone(torch.float32, H, D, V, pad)
 
 
+@pytest.mark.parametrize("activation", [True, False])
+@pytest.mark.parametrize("at", [0, 3, 17, 40, 63, 64, 79])
+def test_lightning_fp32_values_that_are_not_finite_leave_earlier_tokens_alone(activation, at):
+    """A token whose value is infinite or no number touches its own and later read-outs only, wherever it stands in a chunk."""
+    from nanoinfer_b200.kernels import ops
+    H, D, V, n = 2, 64, 68, 90
+    proj = torch.randn(n, H * (2 * D + V), generator=torch.Generator().manual_seed(at)).to(DEV)
+    decay = torch.tensor([0.99, 0.8], device=DEV)
+    cu, slots = torch.tensor([0, n], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for value in (None, float("inf"), float("nan")):
+        x = proj.clone()
+        if value is not None:
+            x[at, 2 * H * D:] = value
+        state, out = torch.zeros(1, H * D * V, device=DEV), torch.empty(n, H * V, device=DEV)
+        ops.lightning_recurrence(x, state, cu, slots, 1, decay, H, D, V, out, activation=activation)
+        outs.append(out)
+    assert bool(torch.isfinite(outs[0]).all())
+    for out in outs[1:]:
+        assert torch.equal(out[:at], outs[0][:at])
+        assert not bool(torch.isfinite(out[at]).any())
+
+
 @pytest.mark.parametrize("H, D, V", [(2, 64, 64), (1, 128, 128), (3, 4, 8), (1, 16, 200)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_chunk_scan_by_four_numbers_is_the_scan_by_one(dtype, H, D, V):
