@@ -456,7 +456,7 @@ delta_block_recurrence_kernel(const float* __restrict__ qkv, const float* __rest
 }
 
 // Whether these sizes are taken: key heads of 64, 128 or 256, whole 16-byte groups everywhere.
-NI_EXPORT int ni_delta_block_supports(int G, int H, int D, int V, int taps) {
+static int db_supports(int G, int H, int D, int V, int taps) {
     return G > 0 && H > 0 && H % G == 0 && (D == 64 || D == 128 || D == 256) && V > 0 && V % 4 == 0 && taps > 0 && taps <= 64;
 }
 // Floats of the coefficients of n_tokens tokens of n_seqs requests.
@@ -471,11 +471,12 @@ NI_EXPORT int ni_delta_block(const void* proj, int proj_dtype, const float* conv
                              int G, int H, int D, int V, int taps, int ld, int b_off, int a_off, float* qkv, float* coef,
                              float* out, cudaStream_t stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return NI_OK;
-    if (!ni_delta_block_supports(G, H, D, V, taps)) return NI_ERR_UNSUPPORTED_SIZE;
+    if (!db_supports(G, H, D, V, taps)) return NI_ERR_UNSUPPORTED_SIZE;
     DbDims dm{G, H, D, V, taps, ld, b_off, a_off};
     const auto aligned = [](const void* q) { return (reinterpret_cast<size_t>(q) & 15) == 0; };
     if (b_off < 0 || a_off < 0 || ld < dm.C() || ld < b_off + H || ld < a_off + H) return NI_ERR_BAD_ARGUMENT;
-    if (ld % 4 || state_stride % 4 || !aligned(proj) || !aligned(state) || !aligned(qkv) || !aligned(coef)) return NI_ERR_BAD_ARGUMENT;
+    if (state_stride % 4 || !aligned(state) || !aligned(qkv) || !aligned(coef)) return NI_ERR_BAD_ARGUMENT;
+    if (proj_dtype == NI_DTYPE_F32 && (ld % 4 || !aligned(proj))) return NI_ERR_BAD_ARGUMENT;      // (bfloat16 rows are read number by number)
     if (H > 65535 || n_seqs > 65535) return NI_ERR_UNSUPPORTED_SIZE;
     const int units = G + (H * V + 127) / 128;
     const dim3 pgrid(n_tokens / DB_T + n_seqs, (units + DB_WARPS - 1) / DB_WARPS);

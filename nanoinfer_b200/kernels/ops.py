@@ -106,7 +106,6 @@ _SIGNATURES = {
     },
     "delta_block": {
         "ni_delta_block": [_P, _I, _P, _P, _P, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P],
-        "ni_delta_block_supports": [_I, _I, _I, _I, _I],
     },
     "delta_chunk": {
         "ni_delta_chunk_recurrence": [_P, _I, _I, _P, _P, _P, _P, _I, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _LL, _P, _P, _P],
@@ -676,6 +675,13 @@ def delta_block_supports(n_q_heads_kv: int, n_heads: int, dim: int, vdim: int, t
     return dim in (64, 128, 256) and vdim % 4 == 0 and 0 < taps <= 64
 
 
+def delta_block_takes(proj: torch.Tensor, col0: int, state: torch.Tensor) -> bool:
+    """Whether delta_block_recurrence takes these rows: float32 rows are read 16 bytes at a time from column ``col0`` on,
+    bfloat16 rows number by number; a request's state lies on 16 bytes."""
+    on16 = proj.dtype != torch.float32 or (proj.shape[1] % 4 == 0 and (proj.data_ptr() + 4 * col0) % 16 == 0)
+    return on16 and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0
+
+
 def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
                            vdim, taps, out) -> None:
     """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another
@@ -689,8 +695,10 @@ def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, sta
             state.shape[1] != n_heads * dim * vdim + (taps - 1) * c or cu_q.numel() != n_seqs + 1 or slots.numel() != n_seqs:
         raise KernelError("delta_block_recurrence: shapes do not agree")
     qkv = torch.empty(n, c, dtype=f32, device=proj.device)
-    coef = torch.empty((n // 4 + n_seqs) * n_heads * 32, dtype=f32, device=proj.device)
-    _check(load("delta_block").ni_delta_block(
+    lib = load("delta_block")
+    lib.ni_delta_block_coefs.restype, lib.ni_delta_block_coefs.argtypes = _LL, [_I] * 3
+    coef = torch.empty(lib.ni_delta_block_coefs(n, n_seqs, n_heads), dtype=f32, device=proj.device)
+    _check(lib.ni_delta_block(
         _dev(proj, "proj") + col0 * proj.element_size(), _code(proj, "proj"), _dev(conv_w, "conv_w", f32), _dev(a_log, "a_log", f32),
         _dev(dt_bias, "dt_bias", f32), _dev(state, "state", f32), state.shape[1], _dev(cu_q, "cu_q", i32), _dev(slots, "slots", i32), n,
         n_seqs, n_q_heads_kv, n_heads, dim, vdim, taps, proj.shape[1], b_col - col0, a_col - col0, qkv.data_ptr(), coef.data_ptr(),

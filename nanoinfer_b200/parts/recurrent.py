@@ -139,8 +139,11 @@ class GatedDeltaRule(Part):
             self.w_second = [rt.weight(x) for x in second]
             self.w_thin = rt.weight(torch.block_diag(*[x.float() for x in second]).to(like.dtype))        # [H D (+ H V), ranks]
             at = self.thin_col + self.thin_k
-        if joined and at % 8:
-            rows.append(zeros(-at % 8, hidden_size))
+        # (FP32 mode walks the tokens one by one: a block's sums depend on where a portion starts)
+        self.in_blocks = rt.dtype == torch.bfloat16 and not self.channel and ops.delta_block_supports(g, h, d, v, taps)
+        pad = -at % (8 if joined else 4 if self.in_blocks else 1)      # (whole groups of 16 bytes: delta_block_takes)
+        if pad:
+            rows.append(zeros(pad, hidden_size))
         if joined:
             self.in_rows, self.out_matrix = torch.cat(rows, dim=0), weights["o"]
         else:
@@ -155,8 +158,6 @@ class GatedDeltaRule(Part):
         self.chunked = rt.dtype == torch.bfloat16 and self.channel and d <= ops.DELTA_CHUNK_MAX_DIM and v <= 512
         if self.chunked:
             self.kernel_modules = ("delta_chunk",)
-        # (FP32 mode walks the tokens one by one: a block's sums depend on where a portion starts)
-        self.in_blocks = rt.dtype == torch.bfloat16 and not self.channel and ops.delta_block_supports(g, h, d, v, taps)
         if self.in_blocks:
             self.kernel_modules = ("delta_block",)
 
@@ -219,7 +220,7 @@ class GatedDeltaRule(Part):
             buf = rt.workspace("delta_chunks", -(-need // 4), f32)                 # one buffer for all layers
             ops.delta_chunk_recurrence(proj, col0, col0 + self.b_col, self.conv_w, self.a_log, self.dt_bias, z, cache.state,
                                        ctx.cu_q, ctx.slots, ctx.n_seqs, ctx.max_q_len, g, h, d, v, self.taps, buf, o)
-        elif self.in_blocks and ctx.max_q_len >= self.BLOCK_FROM and proj.shape[1] % 4 == 0 and col0 % 4 == 0:
+        elif self.in_blocks and ctx.max_q_len >= self.BLOCK_FROM and ops.delta_block_takes(proj, col0, cache.state):
             ops.delta_block_recurrence(proj, col0, col0 + self.b_col, col0 + self.b_col + h, self.conv_w, self.a_log, self.dt_bias,
                                        cache.state, ctx.cu_q, ctx.slots, ctx.n_seqs, g, h, d, v, self.taps, o)
         else:

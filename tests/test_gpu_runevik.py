@@ -242,6 +242,37 @@ def test_delta_rule_by_blocks_of_four_tokens(G, H, D, V, taps, fast, dtype):
     assert bool((states[1][[1, 3, 6]] == 0).all())
 
 
+@pytest.mark.parametrize("dtype, col0, extra, taken", [(torch.bfloat16, 4, 0, True), (torch.bfloat16, 1, 0, True), (torch.bfloat16, 0, 1, True),
+                                                       (torch.float32, 4, 0, True), (torch.float32, 2, 0, False), (torch.float32, 0, 2, False)])
+def test_delta_blocks_of_rows_that_start_anywhere(dtype, col0, extra, taken):
+    """The rule that picks the blocks takes exactly the rows that the launcher takes: bfloat16 rows from any column on (a
+    side of joined mixers starts where the other one ends), float32 rows on 16 bytes."""
+    from nanoinfer_b200.kernels import ops
+    G, H, D, V, taps, n = 1, 2, 64, 8, 4, 13
+    C = 2 * G * D + H * V
+    N = col0 + C + 2 * H + (-(col0 + C + 2 * H)) % 8 + extra
+    g = torch.Generator().manual_seed(col0 + extra)
+    proj, state = torch.randn(n, N, generator=g).to(DEV, dtype), torch.randn(1, H * D * V + (taps - 1) * C, generator=g).to(DEV)
+    conv_w, a_log, dt_bias = (torch.randn(*s, generator=g).to(DEV) for s in ((C, taps), (H,), (H,)))
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cu, slots, seq = torch.tensor([0, n], **i32), torch.zeros(1, **i32), torch.zeros(n, **i32)
+    assert ops.delta_block_takes(proj, col0, state) == taken
+    states, o = [state.clone(), state.clone()], [torch.empty(n, H * V, device=DEV) for _ in range(2)]
+    block = lambda: ops.delta_block_recurrence(proj, col0, col0 + C, col0 + C + H, conv_w, a_log, dt_bias, states[1], cu, slots, 1, G, H, D, V,
+                                               taps, o[1])
+    if not taken:
+        with pytest.raises(ops.KernelError):
+            block()
+        return
+    block()
+    qkv, gates = torch.empty(n, C, device=DEV), torch.empty(n, H, 2, device=DEV)
+    ops.delta_prepare(proj, conv_w, a_log, dt_bias, states[0], seq, cu, slots, 1, G, H, D, V, taps, qkv, gates, col0=col0, b_col=col0 + C)
+    ops.delta_recurrence(qkv, gates, states[0], cu, slots, 1, G, H, D, V, o[0])
+    # sums of D terms in another order, along 13 tokens
+    torch.testing.assert_close(o[1], o[0], rtol=2e-5, atol=2e-5 * o[0].abs().max().item())
+    torch.testing.assert_close(states[1], states[0], rtol=2e-5, atol=2e-5 * states[0].abs().max().item())
+
+
 def _one_layer(layer, width=64, vocab=120, side=None):
     raw = {"architecture": "Runevik", "vocab": vocab, "width": width, "norm": {"eps": 1e-5}, "layers": [layer]}
     if side:

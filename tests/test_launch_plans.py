@@ -1,6 +1,7 @@
 """Host-side launch decisions that need no GPU: how the decode attention cuts a context into
 splits, and which prefill attention kernel takes which head layout."""
 import itertools
+from types import SimpleNamespace
 
 import pytest
 
@@ -58,3 +59,24 @@ def test_stream_objects_belong_to_their_device(monkeypatch):
     for device, raw in [(0, 0), (1, 0), (1, 77), (0, 77), (0, 0), (1, 0)]:
         place.update(device=device, raw=raw)
         assert ops.current_stream_object() == (device, raw)
+
+
+@pytest.mark.parametrize("heads, kv_heads", [(3, 3), (1, 1), (4, 2), (6, 3)])
+def test_the_delta_rules_projection_has_whole_groups_of_16_bytes(heads, kv_heads):
+    """An odd number of heads leaves the logits of beta and decay off a multiple of four columns: zero rows make up for it,
+    so that the FP32 projection of a layer by itself can take the blocks of four tokens."""
+    import torch
+    from nanoinfer_b200.config import MixerSpec
+    from nanoinfer_b200.parts.recurrent import GatedDeltaRule
+    runtime = lambda dtype: SimpleNamespace(dtype=dtype, weight=lambda t: t.to(dtype).contiguous(), gain=lambda t: t.float().contiguous())
+    width, d, v = 8, 64, 4
+    spec = MixerSpec(kind="gated_delta", num_heads=heads, num_kv_heads=kv_heads, head_dim=d, extra=(("value_dim", v), ("conv_taps", 4)))
+    weights = {s: torch.randn(*w.shape) for s, w in GatedDeltaRule.weight_slots(spec, width).items()}
+    part = GatedDeltaRule(spec, width, weights, runtime(torch.bfloat16))
+    cols = part.b_col + 2 * heads
+    assert part.in_blocks and part.w_in.shape[0] == cols + -cols % 4
+    assert torch.equal(part.w_in[cols - heads:cols], weights["a"].to(torch.bfloat16)) and not bool(part.w_in[cols:].any())
+    state = torch.zeros(1, part.cache_need().shape[0])
+    assert ops.delta_block_takes(torch.zeros(2, part.w_in.shape[0]), 0, state)
+    plain = GatedDeltaRule(spec, width, weights, runtime(torch.float32))
+    assert not plain.in_blocks and plain.w_in.shape[0] == cols
