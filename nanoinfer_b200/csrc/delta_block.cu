@@ -264,6 +264,22 @@ __device__ __forceinline__ float2 db_split(unsigned long long v) {
     return r;
 }
 
+// A lane's COLS (2 or 4) neighbouring columns of a row of S: one access.  (V is a multiple of 4 and a lane's first column one of
+// COLS, so they lie on 4 COLS bytes.)
+template <int COLS> __device__ __forceinline__ void db_load(const float* p, float* v) {
+    if (COLS == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[0] = x.x; v[1] = x.y;
+    }
+}
+template <int COLS> __device__ __forceinline__ void db_store(float* p, const float* v) {
+    if (COLS == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+}
+
 #define DB_STAGES 4
 // ROWS rows of COLS columns per lane: row quads 64 j + 4 (lane % 16) .. + 3, columns of half warp lane / 16.
 template <int ROWS, int COLS>
@@ -331,9 +347,15 @@ delta_block_recurrence_kernel(const float* __restrict__ qkv, const float* __rest
 #pragma unroll
     for (int r = 0; r < ROWS / 2; ++r) {
         const size_t row = 64 * (r / 2) + 2 * (r & 1);
+        float a[COLS], b[COLS];
 #pragma unroll
-        for (int c = 0; c < COLS; ++c)
-            s2[r][c] = there ? db_pair(S[row * dm.V + c], S[(row + 1) * dm.V + c]) : 0ull;
+        for (int c = 0; c < COLS; ++c) a[c] = b[c] = 0.f;
+        if (there) {
+            db_load<COLS>(S + row * dm.V, a);
+            db_load<COLS>(S + (row + 1) * dm.V, b);
+        }
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) s2[r][c] = db_pair(a[c], b[c]);
     }
     const float* stage = db_smem;
     for (int b = 0; b < blocks; ++b) {
@@ -445,12 +467,15 @@ delta_block_recurrence_kernel(const float* __restrict__ qkv, const float* __rest
 #pragma unroll
         for (int r = 0; r < ROWS / 2; ++r) {
             const size_t row = 64 * (r / 2) + 2 * (r & 1);
+            float a[COLS], b[COLS];
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
                 const float2 x = db_split(s2[r][c]);
-                S[row * dm.V + c] = x.x;
-                S[(row + 1) * dm.V + c] = x.y;
+                a[c] = x.x;
+                b[c] = x.y;
             }
+            db_store<COLS>(S + row * dm.V, a);
+            db_store<COLS>(S + (row + 1) * dm.V, b);
         }
     }
 }
@@ -496,9 +521,11 @@ NI_EXPORT int ni_delta_block(const void* proj, int proj_dtype, const float* conv
 #undef PREPARE
 #undef PREPARE_T
     if (cudaError_t e = cudaGetLastError()) return (int)e;
-    // Four columns per lane read a k and q from shared memory for twice as many columns; two give twice the warps, for
-    // launches that would not fill the SMs otherwise.
-    const bool few = (long long)((V + 31) / 32) * H * n_seqs < ni_sm_count();
+    // Four columns per lane read a k and q from shared memory for twice as many columns; two halve what a lane does for a block
+    // of tokens, which is faster as long as twice the blocks still have an SM each.  Heads of 128, us with four / two columns: 64
+    // blocks of four columns (one portion of 512, 16 heads) 102.9 / 89.5, 96 (3 x 256 tokens, 8 heads) 56.8 / 63.6, 128 (2 x 256,
+    // 16 heads) 58.5 / 65.2, 256 89.8 / 105.4; heads of 64: 64 blocks 47.9 / 46.7, 96 49.7 / 56.6.
+    const bool few = 2LL * ((V + 31) / 32) * H * n_seqs <= ni_sm_count();
 #define LAUNCH(ROWS, COLS)                                                                                                \
     do {                                                                                                                  \
         constexpr int B = DB_WARPS * 2 * (COLS);                                                                          \

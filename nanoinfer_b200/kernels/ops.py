@@ -682,6 +682,19 @@ def delta_block_takes(proj: torch.Tensor, col0: int, state: torch.Tensor) -> boo
     return on16 and state.shape[1] % 4 == 0 and state.data_ptr() % 16 == 0
 
 
+def delta_block_pays(n_tokens: int, n_seqs: int, max_q_len: int, n_heads: int, dim: int, vdim: int) -> bool:
+    """Whether blocks of four tokens are done before the kernel that walks the tokens, for a step of ``n_tokens`` tokens of
+    ``n_seqs`` requests.  A block saves half of the chain of the longest portion, but costs a request a whole block however
+    few its tokens are, and more to start.  Measured, us token by token / in blocks (16 heads of 128 unless said): one portion
+    of 8 10.4 / 12.2, of 24 15.4 / 14.8, of 64 28.4 / 20.6, of 512 182 / 89; that of 64 beside 64 single tokens 50 / 61, of
+    128 74 / 65; a portion of 256 beside 200 168 / 190, of 512 266 / 204; 16 portions of 8 27.3 / 26.0, 32 of 12 61 / 52.  Heads
+    of 256 (8 of them), whose single tokens cost both kernels alike: 64 beside 64 single tokens 188 / 188, 128 217 / 195."""
+    size = n_heads * dim * vdim / 2 ** 18                      # a request's state, in 16 heads of 128
+    single, full = (2.0, 16) if dim <= 128 else (0.5, 8)
+    return max_q_len >= 26 + single * n_seqs * size ** 0.5 or \
+        (n_tokens >= 8 * n_seqs and (max_q_len >= 26 or n_seqs * size >= full))
+
+
 def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
                            vdim, taps, out) -> None:
     """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another

@@ -33,8 +33,8 @@ class GatedDeltaRule(Part):
     second, block-diagonal product turns (W_a1 x, W_g1 x) into the logits of decay and gate in FP32.  Everything from there
     to the gated norm is FP32 on the device; in bfloat16 a step of single tokens with both options is one launch (from an
     FP32 projection, thin products included), and portions of CHUNK_FROM tokens and more run in chunks on the tensor cores
-    (csrc/delta_chunk.cu); with a decay per head portions of BLOCK_FROM tokens and more run by blocks of four tokens
-    (csrc/delta_block.cu).  A request's state is one FP32 vector: M of every head, then the last
+    (csrc/delta_chunk.cu); with a decay per head steps of long portions run by blocks of four tokens (csrc/delta_block.cu,
+    ops.delta_block_pays).  A request's state is one FP32 vector: M of every head, then the last
     conv_taps - 1 inputs of every convolved channel.  A step's kernels run exactly once, so the state advances by exactly
     the step's tokens.
 
@@ -43,7 +43,6 @@ class GatedDeltaRule(Part):
     kernel_modules = ("delta_rule",)       # libraries of csrc that this part's kernels live in
 
     CHUNK_FROM = 16             # a step whose longest portion has this many tokens takes the chunked recurrence
-    BLOCK_FROM = 8              # ... with a decay per head: the recurrence by blocks of four tokens
 
     JOINS = True                # can be a side of mixers with joined projections
     takes_output_scale = True   # a factor on the output rides in the gated norm, before the output projection
@@ -220,7 +219,8 @@ class GatedDeltaRule(Part):
             buf = rt.workspace("delta_chunks", -(-need // 4), f32)                 # one buffer for all layers
             ops.delta_chunk_recurrence(proj, col0, col0 + self.b_col, self.conv_w, self.a_log, self.dt_bias, z, cache.state,
                                        ctx.cu_q, ctx.slots, ctx.n_seqs, ctx.max_q_len, g, h, d, v, self.taps, buf, o)
-        elif self.in_blocks and ctx.max_q_len >= self.BLOCK_FROM and ops.delta_block_takes(proj, col0, cache.state):
+        elif self.in_blocks and ops.delta_block_takes(proj, col0, cache.state) and \
+                ops.delta_block_pays(n, ctx.n_seqs, ctx.max_q_len, h, d, v):
             ops.delta_block_recurrence(proj, col0, col0 + self.b_col, col0 + self.b_col + h, self.conv_w, self.a_log, self.dt_bias,
                                        cache.state, ctx.cu_q, ctx.slots, ctx.n_seqs, g, h, d, v, self.taps, o)
         else:

@@ -80,3 +80,14 @@ def test_the_delta_rules_projection_has_whole_groups_of_16_bytes(heads, kv_heads
     assert ops.delta_block_takes(torch.zeros(2, part.w_in.shape[0]), 0, state)
     plain = GatedDeltaRule(spec, width, weights, runtime(torch.float32))
     assert not plain.in_blocks and plain.w_in.shape[0] == cols
+
+
+@pytest.mark.parametrize("heads, dim, lens, blocks", [
+    (16, 128, [8], False), (16, 128, [24], False), (16, 128, [64], True), (16, 128, [8] + [1] * 8, False), (16, 128, [32] + [1] * 32, False),
+    (16, 128, [64] + [1] * 64, False), (16, 128, [256] + [1] * 64, True), (16, 128, [256] + [1] * 200, False), (16, 128, [1024] + [1] * 200, True),
+    (16, 128, [8] * 8, False), (16, 128, [16] * 32, True), (8, 64, [8] + [1] * 200, False), (8, 64, [256] + [1] * 200, True),
+    (8, 64, [16] * 16, False), (8, 256, [16], False), (8, 256, [16] * 8, True), (8, 256, [128] + [1] * 64, True), (8, 256, [64] + [1] * 200, False),
+    (16, 128, [1201, 847], True), (16, 128, [2048], True)])
+def test_the_delta_rule_goes_by_blocks_where_they_are_done_first(heads, dim, lens, blocks):
+    """Points of the measured table on both sides of the line: short portions and steps of mostly single tokens token by token."""
+    assert ops.delta_block_pays(sum(lens), len(lens), max(lens), heads, dim, dim) == blocks
