@@ -194,6 +194,20 @@ def with_sub_parts(part) -> list:
     return out
 
 
+def kernel_libraries(parts, bf16: bool) -> set:
+    """The libraries of csrc that these parts name: ``kernel_modules``, and ``kernel_modules_bf16`` or ``kernel_modules_f32``
+    for one of the two paths only; a class inherits its bases' lists, and a part may name more of its own."""
+    needed = set()
+    for part in parts:
+        if part is None:
+            continue
+        needed |= set(getattr(part, "__dict__", {}).get("kernel_modules", ()))            # set on the instance
+        for cls in type(part).__mro__:
+            needed |= set(cls.__dict__.get("kernel_modules", ()))
+            needed |= set(cls.__dict__.get("kernel_modules_bf16" if bf16 else "kernel_modules_f32", ()))
+    return needed
+
+
 class ModelRunner:
     def __init__(self, config: ModelConfig, weights: Dict[str, torch.Tensor], *, dtype,
                  page_size: int = 16, num_pages=1024, max_requests: int = 8,
@@ -217,22 +231,13 @@ class ModelRunner:
         from ..kernels import ops
         self.model = DecoderModel(config, weights, self.rt)
         # Compile (in parallel) and load what THIS model needs in this precision before the first step: the
-        # libraries every model uses, and those its parts name (``kernel_modules``, and ``kernel_modules_bf16``
-        # for the bfloat16 path only; a class inherits its bases' lists).  Anything else is built when first used.
+        # libraries every model uses, and those its parts name.  Anything else is built when first used.
         bf16 = self.rt.dtype == torch.bfloat16
         needed = {"elementwise"} | ({"gemv_bf16", "gemv_ksplit"} if bf16 else {"gemm_f32"}) | ({"decode_fused"} if fused_decode else set())
         all_parts = [q for b in self.model.blocks if b is not None
                      for p in (b, getattr(b, "mixer", None), getattr(b, "feed_forward", None)) for q in with_sub_parts(p)] \
             + [self.model.embedding, self.model.head, self.model]
-        for part in all_parts:
-            if part is None:
-                continue
-            needed |= set(getattr(part, "__dict__", {}).get("kernel_modules", ()))            # set on the instance
-            for cls in type(part).__mro__:
-                needed |= set(cls.__dict__.get("kernel_modules", ()))
-                if bf16:
-                    needed |= set(cls.__dict__.get("kernel_modules_bf16", ()))
-        ops.preload(sorted(needed))
+        ops.preload(sorted(needed | kernel_libraries(all_parts, bf16)))
 
         # cache groups: one per distinct need among the runs that own a cache
         needs = self.model.cache_needs()

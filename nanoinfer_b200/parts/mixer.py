@@ -27,9 +27,10 @@ class PagedAttendMixin:
     SHORT_PORTION = ops.DECODE_FRESH_KEYS
     TILE_ROWS = ops.PREFILL_TILE_ROWS
 
-    # libraries of csrc that the attention kernels live in (the second list: on the bfloat16 path only)
-    kernel_modules = ("attention_generic", "attention_f32")
+    # libraries of csrc that the attention kernels live in (the second list: on the bfloat16 path only; the third: float32)
+    kernel_modules = ("attention_generic",)
     kernel_modules_bf16 = ("attention_prefill", "attention_decode")
+    kernel_modules_f32 = ("attention_f32",)
 
     @staticmethod
     def plan_step(q_lens: List[int], starts: List[int]) -> StepPlan:

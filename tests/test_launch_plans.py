@@ -91,3 +91,15 @@ def test_the_delta_rules_projection_has_whole_groups_of_16_bytes(heads, kv_heads
 def test_the_delta_rule_goes_by_blocks_where_they_are_done_first(heads, dim, lens, blocks):
     """Points of the measured table on both sides of the line: short portions and steps of mostly single tokens token by token."""
     assert ops.delta_block_pays(sum(lens), len(lens), max(lens), heads, dim, dim) == blocks
+
+
+def test_each_path_loads_the_libraries_that_it_launches():
+    """The FP32 attention kernels belong to float32 models: a bfloat16 one neither builds nor loads them, and the other way round."""
+    from nanoinfer_b200.engine.step import kernel_libraries
+    from nanoinfer_b200.parts.mixer import PagedAttention
+    part = object.__new__(PagedAttention)
+    part.kernel_modules = ("pointwise",)
+    f32, bf16 = kernel_libraries([part, None], False), kernel_libraries([part, None], True)
+    assert {"attention_generic", "rope_kv", "pointwise"} <= f32 & bf16
+    assert "attention_f32" in f32 and "attention_f32" not in bf16
+    assert "attention_decode" in bf16 and "attention_decode" not in f32
