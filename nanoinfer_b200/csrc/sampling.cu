@@ -435,6 +435,8 @@ struct ScScratch {
 // Of a block; the first block's list [SC_RANKS][SC_CANDIDATES] and every block's two numbers of every block lie where the general
 // path has its histograms and its first gather buffer, the coarse counts where it has its second.
 #define SC_CANDIDATES 504
+#define SC_PAIRS 256
+static_assert(SC_RANKS * SC_MAX_SLICE <= 1 << 24, "an id fits the 24 bits of sc_mass_select");
 static_assert(SC_RANKS * (SC_CANDIDATES + 2) <= SC_HISTS * 256 + SC_RANKS * 256, "the candidates and the blocks' numbers fit");
 static_assert(SC_COARSE * 4 <= SC_RANKS * 256 * 8, "the coarse counts fit");
 static_assert(SC_COARSE % SC_THREADS == 0, "every thread sums the same number of coarse counts");
@@ -482,7 +484,61 @@ __device__ void sc_send_candidates(const float* z, int n, int lo, int k, const u
     __syncthreads();
 }
 
-// The first block's part: list [SC_RANKS][SC_CANDIDATES] of (key << 32) | id, counts[2 c + 1] of them per block.
+// Of the n entries (bits of e << 32) | id with bits >= e_floor, the largest bits - or, by_id, the smallest id - such that the masses
+// from it upwards - of it and the ids before it - exceed `remaining`, which the mass of all of them does.  Passes of 8 bits over
+// the list, whatever its length; an id counts as 0xffffff - id, so that both look for a largest key.
+__device__ uint32_t sc_mass_select(const unsigned long long* list, int n, uint32_t e_floor, bool by_id, unsigned long long remaining,
+                                   unsigned long long* bins, ScScratch& s) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t prefix = 0u, mask = 0u;
+    for (int shift = by_id ? 16 : 24; shift >= 0; shift -= 8) {
+        if (tid < 256) bins[tid] = 0ull;
+        __syncthreads();
+        for (int i = tid; i - lane < n; i += blockDim.x) {
+            const uint32_t bits = i < n ? (uint32_t)(list[i] >> 32) : 0u, key = by_id && i < n ? 0xffffffu - (uint32_t)list[i] : bits;
+            const bool in = i < n && bits >= e_floor && (key & mask) == prefix;
+            unsigned long long v = in ? mass_of(__uint_as_float(bits)) : 0ull;
+            const uint32_t bin = (key >> shift) & 255u;
+            const unsigned who = __ballot_sync(0xffffffffu, in);
+            const uint32_t first = __shfl_sync(0xffffffffu, bin, who ? __ffs(who) - 1 : 0);
+            if (__all_sync(0xffffffffu, !in || bin == first)) {          // (tied tokens: one addition per warp)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0 && who) atomicAdd(&bins[first], v);
+            } else if (in) {
+                atomicAdd(&bins[bin], v);
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {                                     // lane l holds bins 8 l .. 8 l + 7
+            unsigned long long mine = 0ull;
+            for (int j = 0; j < 8; ++j) mine += bins[8 * lane + j];
+            unsigned long long incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long nb = __shfl_down_sync(0xffffffffu, incl, o);
+                if (lane + o < 32) incl += nb;
+            }
+            unsigned long long above = incl - mine;
+            if (above <= remaining && above + mine > remaining) {
+                int j = 7;
+                while (above + bins[8 * lane + j] <= remaining) above += bins[8 * lane + j--];
+                s.digit_rest[0] = (unsigned long long)(8 * lane + j);
+                s.digit_rest[1] = remaining - above;
+            }
+        }
+        __syncthreads();
+        prefix |= (uint32_t)s.digit_rest[0] << shift;
+        mask |= 255u << shift;
+        remaining = s.digit_rest[1];
+    }
+    return prefix;
+}
+
+// The first block's part: list [SC_RANKS][SC_CANDIDATES] of (key << 32) | id, counts[2 c + 1] of them per block.  Up to SC_PAIRS
+// tokens that stay are compared with one another; more (ties at the k-th place: up to 4,032 stay) go by passes over their bits.
+// 8 rows, k = 50, top-p 0.9, us in pairs / in passes / as passes of the cluster over the row: 170 that stay 28.7 (without ties
+// 22.6) / - / 178, 520 58.3 / 47.7 / 179, 1,060 141 / 60.3 / 182, 3,960 1,317 / 93.8 / 197; without top-p 520 39.0 / 27.9 / 154.
 __device__ void sc_pick(unsigned long long* list, const unsigned long long* counts, uint32_t* work, ScScratch& s, float m, int k, float p,
                         unsigned long long seed, unsigned long long counter, int* out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -563,21 +619,26 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
     if (tid == 0) s.digit_rest[0] = 0ull;
     total = block_sum(total);                                // (its barriers publish the list)
     const int n = s.chosen;
+    const bool pairs = n <= SC_PAIRS;
     // top-p: the largest probability such that the masses from it upwards exceed p * total (none: everything stays)
     uint32_t e_floor = 0u;
     if (p > 0.f && p < 1.f) {
         const unsigned long long limit = (unsigned long long)((double)p * (double)total);
-        for (int i = tid; i < n; i += blockDim.x) {
-            const uint32_t bits = (uint32_t)(list[i] >> 32);
-            unsigned long long upward = 0ull;
-            for (int j = 0; j < n; ++j) {
-                const uint32_t other = (uint32_t)(list[j] >> 32);
-                if (other >= bits) upward += mass_of(__uint_as_float(other));
+        if (pairs) {
+            for (int i = tid; i < n; i += blockDim.x) {
+                const uint32_t bits = (uint32_t)(list[i] >> 32);
+                unsigned long long upward = 0ull;
+                for (int j = 0; j < n; ++j) {
+                    const uint32_t other = (uint32_t)(list[j] >> 32);
+                    if (other >= bits) upward += mass_of(__uint_as_float(other));
+                }
+                if (upward > limit) atomicMax(&s.digit_rest[0], (unsigned long long)bits);
             }
-            if (upward > limit) atomicMax(&s.digit_rest[0], (unsigned long long)bits);
+            __syncthreads();
+            e_floor = (uint32_t)s.digit_rest[0];
+        } else if (total > limit) {
+            e_floor = sc_mass_select(list, n, 0u, false, limit, reinterpret_cast<unsigned long long*>(work), s);
         }
-        __syncthreads();
-        e_floor = (uint32_t)s.digit_rest[0];
         unsigned long long local = 0ull;
         for (int i = tid; i < n; i += blockDim.x) {
             const uint32_t bits = (uint32_t)(list[i] >> 32);
@@ -592,6 +653,11 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
     if (total > 0ull && target >= total) target = total - 1ull;
     if (total == 0ull) {
         if (tid == 0) *out = 0;
+        return;
+    }
+    if (!pairs) {
+        const uint32_t key = sc_mass_select(list, n, e_floor, true, target, reinterpret_cast<unsigned long long*>(work), s);
+        if (tid == 0) *out = (int)(0xffffffu - key);
         return;
     }
     for (int i = tid; i < n; i += blockDim.x) {

@@ -72,6 +72,68 @@ def test_a_cluster_per_row_selects_the_same_tokens_as_one_block(vocab):
     assert len(set(out_b.tolist())) == 1 and out_b[0] == out_a[0]
 
 
+def _tied_rows(vocab, ties, rows, seed):
+    """40 tokens at 5, ``ties`` per eighth of the row at 4, the rest far below."""
+    g = torch.Generator().manual_seed(seed)
+    l = torch.randn(rows, vocab, generator=g) - 50.0
+    for r in range(rows):
+        for c in range(8):
+            lo, hi = c * vocab // 8, (c + 1) * vocab // 8
+            l[r, lo + torch.randperm(hi - lo, generator=g)[:ties]] = 4.0
+        l[r, torch.randperm(vocab, generator=g)[:40]] = 5.0
+    return l
+
+
+@pytest.mark.parametrize("vocab, ties", [(4104, 20), (4104, 33), (33000, 120), (33000, 480), (128256, 250), (128256, 495)])
+def test_top_k_with_thousands_tied_at_the_kth_place(vocab, ties):
+    """All tokens that tie with the k-th stay: from a few more than are compared pair by pair to thousands; probabilities that
+    tie at the top-p place too, one that takes a few of them, temperatures that round most masses to zero."""
+    from nanoinfer_b200.kernels import ops
+    rows = 12
+    l = _tied_rows(vocab, ties, rows, vocab + ties)
+    l[1] += torch.rand(vocab, generator=torch.Generator().manual_seed(1)) * 1e-6 * (l[1] > 4.5)           # masses that differ in the last bits
+    l[2, l[2] == 4.0] = -40.0                                                                              # tied at a mass of nearly nothing
+    l = l.to(DEV)
+    k_t = torch.tensor([41 + 3 * (r % 3) for r in range(rows)], dtype=torch.int32, device=DEV)
+    seeds, counters = torch.arange(rows, device=DEV) * 104729, torch.arange(rows, device=DEV) % 3
+    for temp, p in [(0.8, 1.0), (0.8, 0.9), (0.8, 0.05), (0.03, 0.9999), (0.004, 0.9), (3.0, 0.5)]:
+        temps, ps_ = torch.full((rows,), temp, device=DEV), torch.full((rows,), p, device=DEV)
+        outs = []
+        for cluster in (True, False):
+            ops.sample_by_cluster(cluster)
+            out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+            ops.sample(l, out, temps, k_t, ps_, seeds, counters)
+            outs.append(out.cpu())
+        ops.sample_by_cluster(True)
+        assert torch.equal(outs[0], outs[1]), (temp, p)
+
+
+def test_tied_rows_take_no_comparisons_of_all_pairs():
+    """Thousands of tied tokens may cost passes over them (as long as a row without candidates, about five times the plain
+    row's), not a comparison of each with each (about sixty times)."""
+    from nanoinfer_b200.kernels import ops
+    rows, vocab = 8, 128256
+
+    def best_of(l):
+        l = l.to(DEV)
+        out = torch.empty(rows, dtype=torch.int32, device=DEV)
+        k_t, ps_ = torch.full((rows,), 50, dtype=torch.int32, device=DEV), torch.full((rows,), 0.9, device=DEV)
+        temps, seeds = torch.full((rows,), 0.8, device=DEV), torch.arange(rows, device=DEV)
+        times = []
+        for _ in range(20):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                ops.sample(l, out, temps, k_t, ps_, seeds, seeds)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    plain, tied = best_of(torch.randn(rows, vocab, generator=torch.Generator().manual_seed(2)) * 3), best_of(_tied_rows(vocab, 490, rows, 3))
+    assert tied < 15 * plain, (tied, plain)
+
+
 @pytest.mark.parametrize("vocab", [4096, 4097, 33000, 128256])
 def test_top_k_from_candidates_selects_the_same_tokens_as_one_block(vocab):
     """Rows with top-k whose blocks send a few candidates, and rows that send too many (large k, equal logits, most of a row
