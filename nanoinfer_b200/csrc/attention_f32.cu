@@ -5,7 +5,8 @@
 // kv head that read the same keys (tokens x heads of the group) and multiplies tiles.  To keep a token's result independent
 // of the cut, the order of every operation on it follows from absolute key positions alone and is the same in both kernels:
 //     keys in blocks of 64 [64 b, 64 b + 63], blocks in segments of 8 [512 s, 512 s + 511];
-//     score: two chains of multiply-adds over the even and the odd dimensions, added, times the scale (a masked key: -inf);
+//     score: for every 32 dimensions two chains of multiply-adds, over the even and the odd ones, added; these sums one after the
+//            other; times the scale (a masked key: -inf);
 //     block: m' = max(m, its scores), p = exp(s - m'), l = l exp(m - m') + sum p, acc = acc exp(m - m') then + p v key by key;
 //            the sum of p: keys j, j + 16, j + 32, j + 48 as (+) + (+), then a binary tree over j from its lowest bit up;
 //     segment: from (-inf, 0, 0), merged into the running (m, l, acc) when it ends; the sink is where the running sums start.
@@ -14,7 +15,8 @@
 //
 // Portions (attention_f32_tile): 64 rows (32 at heads of 128) x 64 keys per step, 128 threads of 8 x 4 scores and 8 x 4
 // outputs, packed multiply-adds, keys and values through two buffers of asynchronous copies.  Bound by shared memory (12
-// loads of 16 bytes for 128 multiply-adds) and by two blocks of 255 registers per SM.  Single tokens (attention_f32_rows): a
+// loads of 16 bytes for 128 multiply-adds) and by the blocks that an SM holds: two at heads of 64 (255 registers), one at heads of
+// 128 (161 KB of shared memory).  Single tokens (attention_f32_rows): a
 // block per (token, kv head, segment), partial results merged by a second launch - or per (token, kv head) where the segments
 // would not fill the GPU any better.  1,087 tokens in three portions, 32 heads of 64: 191 us against 2,054 us of
 // attention_generic.cu; two single tokens over 130 keys: 8.6 against 134 us.
@@ -22,6 +24,7 @@
 
 #define AF_KB 64                    // keys of a block
 #define AF_SEG 512                  // keys of a segment
+#define AF_CHAIN 32                 // dimensions of a score's chains
 #define AF_THREADS 128
 #define AF_MAX_GROUP 16
 
@@ -57,10 +60,10 @@ __device__ __forceinline__ float2 af_split(unsigned long long v) {
 // exp(a - b) where a <= b, and 1 where they are the same (both may be -inf).
 __device__ __forceinline__ float af_factor(float a, float b) { return a == b ? 1.f : expf(a - b); }
 __device__ __forceinline__ float af_scale(float a, float f) { return __fmul_rn(a, f); }
-// The score of two chains: rounded before it is scaled, and never contracted into what follows.
-__device__ __forceinline__ float af_score(unsigned long long chains, float scale) {
+// A score's next two chains added to what came before them: rounded, never contracted into what follows.
+__device__ __forceinline__ float af_score(float before, unsigned long long chains) {
     const float2 c = af_split(chains);
-    return __fmul_rn(__fadd_rn(c.x, c.y), scale);
+    return __fadd_rn(before, __fadd_rn(c.x, c.y));
 }
 // First key that the token at position pos sees.
 __device__ __forceinline__ int af_first(const AfParams& p, int pos) {
@@ -145,37 +148,49 @@ attention_f32_tile_kernel(AfParams p, const int* __restrict__ tile_seq, const in
         __syncthreads();
         const float* kb = ks + buf * AF_KB * PITCH + tx * PITCH;
         const float* qb = qs + r0 * PITCH;
-        unsigned long long s2[RM][4];
+        float s[RM][4];
 #pragma unroll
         for (int i = 0; i < RM; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 1
+        for (int d0 = 0; d0 < HD; d0 += AF_CHAIN) {
+            unsigned long long s2[RM][4];
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
 #pragma unroll 4
-        for (int d = 0; d < HD; d += 4) {
-            ulonglong2 kk[4];
+            for (int d = d0; d < d0 + AF_CHAIN; d += 4) {
+                ulonglong2 kk[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(kb + 16 * j * PITCH + d);
+                for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(kb + 16 * j * PITCH + d);
 #pragma unroll
-            for (int i = 0; i < RM; ++i) {
-                const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qb + i * PITCH + d);
+                for (int i = 0; i < RM; ++i) {
+                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qb + i * PITCH + d);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    af_fma2(s2[i][j], qq.x, kk[j].x);
-                    af_fma2(s2[i][j], qq.y, kk[j].y);
+                    for (int j = 0; j < 4; ++j) {
+                        af_fma2(s2[i][j], qq.x, kk[j].x);
+                        af_fma2(s2[i][j], qq.y, kk[j].y);
+                    }
                 }
             }
+#pragma unroll
+            for (int i = 0; i < RM; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = af_score(s[i][j], s2[i][j]);
         }
         const int key = b * AF_KB + tx;
         const bool edge = b * AF_KB + AF_KB - 1 > pos_first || b * AF_KB < af_first(p, pos_last) || rows < ROWS;
         // (the rows side by side in every step: a row's four exchanges and its exponentials are a chain of their own)
-        float s[RM][4], top[RM];
+        float top[RM];
 #pragma unroll
         for (int i = 0; i < RM; ++i) {
             top[i] = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const bool seen = !edge || (key + 16 * j <= pos[i] && key + 16 * j >= lo[i]);
-                s[i][j] = seen ? af_score(s2[i][j], p.scale) : -INFINITY;
+                s[i][j] = seen ? af_scale(s[i][j], p.scale) : -INFINITY;
                 top[i] = fmaxf(top[i], s[i][j]);
             }
         }
@@ -344,25 +359,33 @@ attention_f32_rows_kernel(AfParams p, const int* __restrict__ token_list, float*
         __syncthreads();
         const int kj = tid & 63, q0 = tid >> 6;
         const float* kb = ks + buf * AF_KB * PITCH + kj * PITCH;
-        unsigned long long s2[QR];
+        float s1[QR];
 #pragma unroll
-        for (int i = 0; i < QR; ++i) s2[i] = 0ull;
+        for (int i = 0; i < QR; ++i) s1[i] = 0.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < HD; c0 += AF_CHAIN) {
+            unsigned long long s2[QR];
+#pragma unroll
+            for (int i = 0; i < QR; ++i) s2[i] = 0ull;
 #pragma unroll 4
-        for (int c = 0; c < HD; c += 4) {
-            const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(kb + c);
+            for (int c = c0; c < c0 + AF_CHAIN; c += 4) {
+                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(kb + c);
 #pragma unroll
-            for (int i = 0; i < QR; ++i)
-                if (q0 + 2 * i < G) {
-                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (q0 + 2 * i) * PITCH + c);
-                    af_fma2(s2[i], qq.x, kk.x);
-                    af_fma2(s2[i], qq.y, kk.y);
-                }
+                for (int i = 0; i < QR; ++i)
+                    if (q0 + 2 * i < G) {
+                        const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (q0 + 2 * i) * PITCH + c);
+                        af_fma2(s2[i], qq.x, kk.x);
+                        af_fma2(s2[i], qq.y, kk.y);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < QR; ++i) s1[i] = af_score(s1[i], s2[i]);
         }
         const int key = b * AF_KB + kj;
         const bool seen = key <= pos && key >= lo;
 #pragma unroll
         for (int i = 0; i < QR; ++i)
-            if (q0 + 2 * i < G) ps[(q0 + 2 * i) * PP + kj] = seen ? af_score(s2[i], p.scale) : -INFINITY;
+            if (q0 + 2 * i < G) ps[(q0 + 2 * i) * PP + kj] = seen ? af_scale(s1[i], p.scale) : -INFINITY;
         __syncthreads();
         for (int r = warp; r < G; r += AF_THREADS / 32) {  // a warp per row; its halves do the same
             const int j0 = lane & 15, k0 = b * AF_KB + j0;

@@ -366,6 +366,45 @@ def test_rope_kv_write(dtype, pairing, n_q, n_kv, hd, rot, page):
     assert torch.all(vp.permute(0, 2, 1, 3)[~touched] == 7.0)
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd", [(8, 2, 64), (6, 2, 128)])
+@pytest.mark.parametrize("lens,starts", [([120, 57, 33], [0, 0, 0]), ([500], [300]), ([1500], [1400])])
+def test_attention_f32_is_as_close_to_the_exact_result_as_key_by_key(n_q, n_kv, hd, lens, starts):
+    """The FP32 tiles against float64 beside the kernel that walks the keys one by one: the error (2-norm, four inputs) is no
+    larger, from short prompts, where the scores' own sums decide it, to long contexts, where the keys' do."""
+    from nanoinfer_b200.kernels import ops
+    page, scale, wrong, size = 16, hd ** -0.5, [0.0, 0.0], 0.0
+    for seed in range(4):
+        table, k_pages, v_pages, ks, vs = _paged_setup(lens, n_kv, hd, page, torch.float32, seed=seed)
+        q_lens = [t - s for t, s in zip(lens, starts)]
+        n = sum(q_lens)
+        q = torch.randn(n, n_q * hd, generator=torch.Generator().manual_seed(90 + seed)).to(DEV)
+        positions = torch.cat([torch.arange(s, t) for s, t in zip(starts, lens)]).int().to(DEV)
+        seq_of = torch.cat([torch.full((c,), i) for i, c in enumerate(q_lens)]).int().to(DEV)
+        cu = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0))).int().to(DEV)
+        kd, vd, td = k_pages.to(DEV), v_pages.to(DEV), table.to(DEV)
+        tiles = [(i, r) for i, c in enumerate(q_lens) for r in range(0, c, 128)]
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        outs = [torch.empty_like(q), torch.empty_like(q)]
+        assert 0 == ops.load("attention_generic").ni_attention_generic(
+            q.data_ptr(), 0, kd.data_ptr(), vd.data_ptr(), outs[0].data_ptr(), 0, None, positions.data_ptr(), seq_of.data_ptr(),
+            td.data_ptr(), td.shape[1], n, n_q, n_kv, hd, page, 0, scale, None, 0.0, hd, 0, None, 1, ops._stream())
+        ops.attention_f32(q, kd, vd, outs[1], positions, seq_of, td, n_q, n_kv, hd, page, None, scale, tiles=(
+            i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), len(tiles), 128, cu, i32(lens)))
+        want, at = torch.empty(n, n_q * hd, dtype=torch.float64, device=DEV), 0
+        for i, c in enumerate(q_lens):
+            hidden = torch.arange(lens[i], device=DEV)[None, :] > starts[i] + torch.arange(c, device=DEV)[:, None]
+            for h in range(n_q):
+                k, v = (x[i][:lens[i], h // (n_q // n_kv)].to(DEV).double() for x in (ks, vs))
+                sc = (q[at:at + c, h * hd:(h + 1) * hd].double() @ k.T * scale).masked_fill(hidden, -math.inf)
+                want[at:at + c, h * hd:(h + 1) * hd] = torch.softmax(sc, dim=-1) @ v
+            at += c
+        for j in range(2):
+            wrong[j] += (outs[j].double() - want).pow(2).sum().item()
+        size += want.pow(2).sum().item()
+    plain, tiled = ((w / size) ** 0.5 for w in wrong)
+    assert tiled <= 1.03 * plain, (tiled, plain)          # (the scatter of such sums over inputs: within 1 %)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n_q,n_kv,hd,rot,page", [(32, 8, 64, 64, 16), (5, 1, 128, 128, 8), (7, 2, 128, 96, 4), (3, 3, 256, 34, 16),
                                                   (40, 8, 128, 0, 16), (2, 1, 64, 2, 16)])
