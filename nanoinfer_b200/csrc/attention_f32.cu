@@ -181,7 +181,8 @@ attention_f32_tile_kernel(AfParams p, const int* __restrict__ tile_seq, const in
                 for (int j = 0; j < 4; ++j) s[i][j] = af_score(s[i][j], s2[i][j]);
         }
         const int key = b * AF_KB + tx;
-        const bool edge = b * AF_KB + AF_KB - 1 > pos_first || b * AF_KB < af_first(p, pos_last) || rows < ROWS;
+        // (a row that is not there counts as one that sees everything: it is never stored)
+        const bool edge = b * AF_KB + AF_KB - 1 > pos_first || b * AF_KB < af_first(p, pos_last);
         // (the rows side by side in every step: a row's four exchanges and its exponentials are a chain of their own)
         float top[RM];
 #pragma unroll
