@@ -187,7 +187,8 @@ __global__ void rope_kv_write_vec_kernel(const T* __restrict__ qkv, T* __restric
 // barrier -, and the loads of all its heads (which need no position) are on their way before the token's position, angles and
 // page are known.  A block is a token; a warp visits 32 / chunks heads at a time, ITEMS times at most before it stores.
 // Bound by the chain position -> angles -> page -> stores of a token (one wave of blocks), not yet by its bytes: 2,048 tokens
-// of 48 heads of 64 (25 MB) 9.9 -> 8.6 us, 1,914 tokens of 48 heads of 128 (47 MB) 22.4 -> 12.9 us against the table.
+// of 48 heads of 64 (25 MB) 8.1 -> 7.4 us, 1,914 tokens of 48 heads of 128 (47 MB) 17.0 -> 10.9 us against the table (replayed
+// launches, the cache warm).
 template <typename T, int ITEMS>
 __global__ void __launch_bounds__(256)
 rope_kv_write_lanes_kernel(const T* __restrict__ qkv, T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages,
@@ -257,22 +258,23 @@ NI_EXPORT int ni_rope_kv_write(const void* qkv, int dtype, void* q_out, void* k_
         return NI_ERR_BAD_ARGUMENT;
     const int chunks = head_dim / 8;
     if (interleaved && head_dim % 8 == 0 && chunks >= 2 && chunks <= 32 && (chunks & (chunks - 1)) == 0) {
-        // groups of heads (a warp's worth of chunks each) per warp: four where that leaves up to four warps, else two over up
-        // to eight warps.  1,914 tokens of 48 heads of 128 (24 groups): 14.6 us with four, 12.9 with two; 2,048 tokens of 48 heads
-        // of 64 (12 groups): 8.6 with four (fewer warps compute the angles), 8.9 with two
+        // Groups of heads (a warp's worth of chunks each) per warp: two, over up to eight warps.  Four, where up to four warps then
+        // hold them all and the launch has tokens enough to keep the SMs busy with fewer warps, half of which compute the angles:
+        // 12 groups x 2,048 tokens 7.7 us with two, 7.4 with four, x 1,024 (heads of 128) 5.5 / 4.8, 8 groups x 2,048 5.8 / 5.4; but 12
+        // groups x 512 3.6 / 4.2, x 8 3.0 / 3.8, 3 groups x 2,048 3.8 / 4.3, and 24 groups x 1,914 10.2 / 14.6.  In bfloat16 alone: the
+        // two are separate compilations of the rotation, and a float32 token's bits must not depend on the step's size.
         int log_chunks = 0;
         while ((1 << log_chunks) < chunks) ++log_chunks;
-        const int groups = ((n_q_heads + 2 * n_kv_heads) * chunks + 31) / 32;
-        const int warps = groups <= 16 ? (groups + 3) / 4 : (groups + 1) / 2 <= 8 ? (groups + 1) / 2 : 8;
-#define LAUNCHL(T)                                                                                     \
-    do {                                                                                               \
-        auto kernel = groups <= 16 ? rope_kv_write_lanes_kernel<T, 4> : rope_kv_write_lanes_kernel<T, 2>; \
-        kernel<<<n_tokens, 32 * warps, 0, stream>>>(                                                   \
-            (const T*)qkv, (T*)q_out, (T*)k_pages, (T*)v_pages, positions, seq_of_token, block_table, \
-            bt_stride, inv_freq, n_q_heads, n_kv_heads, head_dim, log_chunks, rotary_dim, page_size, write_cache); \
-    } while (0)
-        if (dtype == NI_DTYPE_F32) LAUNCHL(float);
-        else if (dtype == NI_DTYPE_BF16) LAUNCHL(__nv_bfloat16);
+        const int groups = ((n_q_heads + 2 * n_kv_heads) * chunks + 31) / 32, halves = (groups + 1) / 2;
+        const bool four = dtype == NI_DTYPE_BF16 && groups <= 16 && (long long)n_tokens * halves >= 32LL * ni_sm_count();
+        const int warps = four ? (groups + 3) / 4 : halves <= 8 ? halves : 8;
+#define LAUNCHL(T, ITEMS)                                                                              \
+    rope_kv_write_lanes_kernel<T, ITEMS><<<n_tokens, 32 * warps, 0, stream>>>(                         \
+        (const T*)qkv, (T*)q_out, (T*)k_pages, (T*)v_pages, positions, seq_of_token, block_table,      \
+        bt_stride, inv_freq, n_q_heads, n_kv_heads, head_dim, log_chunks, rotary_dim, page_size, write_cache)
+        if (dtype == NI_DTYPE_F32) LAUNCHL(float, 2);
+        else if (dtype == NI_DTYPE_BF16 && four) LAUNCHL(__nv_bfloat16, 4);
+        else if (dtype == NI_DTYPE_BF16) LAUNCHL(__nv_bfloat16, 2);
         else return NI_ERR_BAD_ARGUMENT;
 #undef LAUNCHL
         NI_RETURN_LAUNCH_STATUS();

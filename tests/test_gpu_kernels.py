@@ -413,6 +413,34 @@ def test_rope_kv_write_a_chunk_column_per_lane(dtype, n_q, n_kv, hd, rot, page):
     test_rope_kv_write(dtype, "interleaved", n_q, n_kv, hd, rot, page) if rot else _rope_kv_write_unrotated(dtype, n_q, n_kv, hd, page)
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,rot,many,few", [(32, 8, 64, 64, 1000, 150), (16, 4, 128, 96, 1025, 100), (5, 1, 64, 64, 5000, 1000),
+                                                      (32, 8, 128, 128, 700, 350)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_rope_kv_write_of_many_tokens_is_that_of_few(dtype, n_q, n_kv, hd, rot, many, few):
+    """Steps of many tokens keep more heads per warp than steps of few (by the launcher's rule 32 warps per SM lie between the
+    two): the same numbers, in float32 the same bits."""
+    from nanoinfer_b200.kernels import ops
+    page = 16
+    qkv = _randn(many, (n_q + 2 * n_kv) * hd, dtype=dtype, seed=rot)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    positions, seq_of = torch.arange(many, **i32), torch.zeros(many, **i32)
+    table = torch.arange(-(-many // page), **i32).flip(0)[None].contiguous()
+    inv_freq = plain.rope_inv_freq(rot, 10000.0, None).to(DEV)
+    outs = []
+    for step in (many, few):
+        q = torch.empty(many, n_q * hd, dtype=dtype, device=DEV)
+        kp, vp = (torch.zeros(table.shape[1], n_kv, page, hd, dtype=dtype, device=DEV) for _ in range(2))
+        for a in range(0, many, step):
+            b = min(a + step, many)
+            ops.rope_kv_write(qkv[a:b], q[a:b], kp, vp, positions[a:b], seq_of[a:b], table, inv_freq, n_q, n_kv, hd, rot, True, page)
+        outs.append((q, kp, vp))
+    for x, y in zip(*outs):
+        if dtype == torch.float32:
+            assert torch.equal(x, y)
+        torch.testing.assert_close(x.float(), y.float(), rtol=2.0 ** -7, atol=1e-6)          # the last bit of bfloat16
+    assert torch.equal(outs[0][2], outs[1][2]) and bool(outs[0][1].any())
+
+
 def _rope_kv_write_unrotated(dtype, n_q, n_kv, hd, page):
     from nanoinfer_b200.kernels import ops
     n = 5
