@@ -136,7 +136,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     // into L2 now, in pieces dealt over the blocks, while this kernel - which waits on latencies
     // more than on bandwidth - leaves the memory system room.  Nothing here depends on the kernel before.
     if (threadIdx.x >= (DEC_WARPS - 1) * 32) dec_warm(warm_a, warm_a_bytes);
-    if ((int)blockIdx.x >= n_items) {        // a block (with CL: a whole cluster) without a token: it only asks (see dec_extra_items)
+    if ((int)blockIdx.x >= n_items || (int)blockIdx.z >= n_splits) {      // a block (with CL: a whole cluster) that only asks (see dec_extra)
         if (threadIdx.x >= (DEC_WARPS - 1) * 32) dec_warm(warm_b, warm_b_bytes);
         return;
     }
@@ -872,20 +872,34 @@ NI_EXPORT int ni_attention_decode_balanced(const void* q, const void* k_pages, c
     }
 }
 
-// Items without a token that a launch with weights to ask for gets besides its own, so that the requests come from as many
+// Blocks without a token that a launch with weights to ask for gets besides its own, so that the requests come from as many
 // SMs as the GPU has.  Requests of one SM are served one after the other: 16 MB asked for by the 8 blocks of a lone short
 // request (8 kv heads, one split) kept those blocks - and the product that waits for them - several us beyond their few
-// keys.  Up to three blocks per SM in all, which is what is resident at once, so no block with a token waits for one without.
-// Sixteen tokens generated for one request of 33, ms with 0 / 148 / 296 / 444 blocks: 12.38 / 10.81 / 10.77 / 10.77 (nothing
+// keys.  Sixteen tokens generated for one request of 33, ms with 0 / 148 / 296 / 444 blocks: 12.38 / 10.81 / 10.77 / 10.77 (nothing
 // asked for at all: 10.91); four requests of 20 to 60: 12.71 / 11.55 / 11.32 / 11.09 (11.27); eight of 17 to 301: 14.35 /
-// 13.78 / 13.73 / 13.73 (14.08); one of 900, which is cut into four splits: 13.99 / 14.02 / 13.96 / 13.87 (13.70).
+// 13.78 / 13.73 / 13.73 (14.08).
 // Only while the launch's own blocks fill at most every second SM: beyond that they ask from enough places, and their longer
 // streams only get company.  A layer of width 4,096 with heads of 128, one token at 500 keys (16 blocks): 40.0 us without,
 // 33.9 with; four at 20 to 3,000 (384 blocks): 39.9 and 42.0.  Eight requests of 700 (128 blocks), sixteen tokens: 21.5 ms
 // without, 21.6 with, which is as far as two runs of one side lie apart.
-static int dec_extra_items(int n_items, int n_kv_heads, int n_splits, unsigned long long warm_bytes) {
-    const long long per_item = (long long)n_kv_heads * n_splits, own = n_items * per_item, sms = ni_sm_count();
-    return warm_bytes && 2 * own <= sms ? (int)((3 * sms - own) / per_item) : 0;
+// Where they stand: blocks go out item first, then kv head, then split.  With several splits they are further splits (whole
+// clusters of them where the splits merge in one) and so come after every block that has a token: the merge's slots leave room
+// for two blocks per SM, or one, and clusters that only ask would otherwise hold up those of the later kv heads.  One request
+// of the 3B shape at 2,048 keys (8 splits), us per step without them / as further items / as further splits: 1,834 / 1,881 / 1,835, at
+// 900 1,822 / 1,813 / 1,777, at 300 1,953 / 1,802 / 1,772; 1B shape 702 / 707 / 696, 696 / 697 / 685, 738 / 704 / 680.  With one split
+// all of up to three blocks per SM are resident at once, and further items it is: 3B shape, one request of 33 2,705 /
+// 1,605 / 1,634, two 2,504 / 1,642 / 1,666; 1B 706 / 607 / 604, 755 / 612 / 606.
+// Returns how many further splits (n_splits > 1) or further items (one split).
+static int dec_extra(int n_items, int n_kv_heads, int n_splits, bool cluster, unsigned long long warm_bytes, int sms) {
+    const long long own = (long long)n_items * n_kv_heads * n_splits;
+    if (!warm_bytes || 2 * own > sms) return 0;
+    if (n_splits == 1) return (int)((3LL * sms - own) / n_kv_heads);
+    const int step = cluster ? n_splits : 1;
+    return (int)((3LL * sms - own) / ((long long)n_items * n_kv_heads * step)) * step;
+}
+NI_EXPORT int ni_attention_decode_extra(int n_items, int n_kv_heads, int n_splits, int cluster, long long warm_bytes, int sms) {      // for tests
+    if (n_items <= 0 || n_kv_heads <= 0 || n_splits <= 0 || sms <= 0) return 0;
+    return dec_extra(n_items, n_kv_heads, n_splits, cluster != 0, (unsigned long long)warm_bytes, sms);
 }
 
 template <int HD, int SEG, bool CL, bool CAP, bool DIFF>
@@ -909,7 +923,8 @@ static int launch_decode_cl(const void* q, const void* k_pages, const void* v_pa
         configured = smem;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(n_items + dec_extra_items(n_items, n_kv_heads, n_splits, warm_a_bytes + warm_b_bytes), n_kv_heads, n_splits);
+    const int extra = dec_extra(n_items, n_kv_heads, n_splits, CL, warm_a_bytes + warm_b_bytes, ni_sm_count());
+    cfg.gridDim = dim3(n_items + (n_splits == 1 ? extra : 0), n_kv_heads, n_splits + (n_splits == 1 ? 0 : extra));
     cfg.blockDim = dim3(DEC_WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

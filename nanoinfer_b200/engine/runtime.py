@@ -110,7 +110,7 @@ class Runtime:
     # starts and, once a block's own stream has ended, for the first warm_attention_bytes of the matrix
     # after that (a third of that for a lone token, whose attention is over too soon for more); the
     # output projection goes on from there for warm_bytes.  (A launch of few blocks asks with more of
-    # them: dec_extra_items in csrc/attention_decode.cu.)  Measured on the 1B sizes at context 2,048
+    # them: dec_extra in csrc/attention_decode.cu.)  Measured on the 1B sizes at context 2,048
     # (ms per step, without / with): batch 1 0.801 / 0.791, 2 0.836 / 0.814, 4 0.854 / 0.829,
     # 8 0.865 / 0.838.  More does not help (32 MiB: 0.842; 40 MiB: 0.848), nor does the same request at
     # the end of gate/up (for the down projection: 0.855 - that kernel runs at its register limit and

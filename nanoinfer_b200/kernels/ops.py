@@ -138,6 +138,7 @@ _SIGNATURES = {
         "ni_attention_decode_difference": [_P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _F, _F, _I, _I, _P, _P, _P, _LL, _P, _LL, _P],
         "ni_attention_decode_balanced": [_P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P, _P, _P, _LL, _P, _LL, _P],
         "ni_attention_decode_fresh_keys": [],
+        "ni_attention_decode_extra": [_I, _I, _I, _I, _LL, _I],
         "ni_attention_decode_set_cluster_merge": [_I],
         # the variant whose scratch lies in the library's own image (attention_decode_noalloc.h)
         "ni_attention_decode_noalloc": [_P, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P],

@@ -103,3 +103,31 @@ def test_each_path_loads_the_libraries_that_it_launches():
     assert {"attention_generic", "rope_kv", "pointwise"} <= f32 & bf16
     assert "attention_f32" in f32 and "attention_f32" not in bf16
     assert "attention_decode" in bf16 and "attention_decode" not in f32
+
+
+@pytest.mark.parametrize("cluster", [False, True])
+def test_blocks_that_only_ask_for_weights_hold_nobody_up(cluster):
+    """The decode attention's blocks go out item first, then kv head, then split.  Beside several splits, whose merge may leave
+    an SM room for one block, those without a token are further splits: all of them come behind all that have one, in whole
+    clusters.  Beside one split they are further items, and three blocks per SM hold all there are."""
+    extra = ops.load("attention_decode").ni_attention_decode_extra
+    sms, some = 148, 0
+    for items, n_kv, splits in itertools.product([1, 2, 3, 8, 19], [1, 2, 8], range(1, 17)):
+        if cluster and splits < 2:
+            continue
+        more = extra(items, n_kv, splits, cluster, 1 << 20, sms)
+        assert extra(items, n_kv, splits, cluster, 0, sms) == 0
+        own = items * n_kv * splits
+        if 2 * own > sms:
+            assert more == 0
+            continue
+        assert more > 0
+        some += 1
+        if splits == 1:
+            assert (items + more) * n_kv <= 3 * sms < (items + more + 1) * n_kv
+            continue
+        number = lambda x, y, z: (z * n_kv + y) * items + x
+        assert more % (splits if cluster else 1) == 0
+        assert number(items - 1, n_kv - 1, splits - 1) == own - 1 and number(0, 0, splits) == own
+        assert items * n_kv * (splits + more) <= 3 * sms < items * n_kv * (splits + more + (splits if cluster else 1))
+    assert some > 20
