@@ -18,8 +18,9 @@
 // loads of 16 bytes for 128 multiply-adds) and by the blocks that an SM holds: two at heads of 64 (255 registers), one at heads of
 // 128 (161 KB of shared memory).  Single tokens (attention_f32_rows): a
 // block per (token, kv head, segment), partial results merged by a second launch - or per (token, kv head) where the segments
-// would not fill the GPU any better.  1,087 tokens in three portions, 32 heads of 64: 191 us against 2,054 us of
-// attention_generic.cu; two single tokens over 130 keys: 8.6 against 134 us.
+// would not fill the GPU any better.  1,087 tokens in three portions, 32 heads of 64: 188 us against 2,054 us of
+// attention_generic.cu; two single tokens over 130 keys: 8.6 against 134 us.  2,048 tokens of 24/8 heads of 128: 1,423 us (1,673 with
+// chains over the whole head and empty rows that made every key block an edge).
 #include "common.cuh"
 
 #define AF_KB 64                    // keys of a block

@@ -7,9 +7,9 @@
 //     o_t = c_t S^T q_t + sum_{s<=t} P(t, s) (q_t . k_s) u_s
 //     S  <- c_3 S + sum_s P(3, s) k_s u_s^T
 // so a block's eight products with S do not wait for one another, and one exchange between lanes serves four tokens: what
-// bounds a portion is the chain of its blocks (about 1,150 clocks: 330 instructions of a lone warp per scheduler), no longer
-// the chain of its tokens (about 680 clocks each).  2,048 tokens, 16 heads of 128: 350 us with the preparation against 690;
-// portions of 1,201 and 847 tokens 255 against 505 us; 8 portions of 512 tokens 340 against 536 us.
+// bounds a portion is the chain of its blocks (0.64 us each, measured from 512 to 2,048 tokens of one request with 128 thread blocks of
+// 4 warps: 1,270 clocks at 1,965 MHz), no longer the chain of its tokens (0.35 us each).  2,048 tokens, 16 heads of 128: 337 us with
+// the preparation against 715; portions of 1,201 and 847 tokens 245 against 502 us; 8 portions of 512 tokens 329 against 536 us.
 // Only products of decays over stretches of a block appear, never quotients.  Tokens that a last block lacks have beta 0,
 // decay 1 and zeros for k, q and v, which leaves S alone.
 //
