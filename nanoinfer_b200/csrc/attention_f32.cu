@@ -99,6 +99,7 @@ attention_f32_tile_kernel(AfParams p, const int* __restrict__ tile_seq, const in
                           const int* __restrict__ cu_q, const int* __restrict__ kv_len, int slices) {
     constexpr int ROWS = 8 * RM, PITCH = HD + 4, PP = AF_KB + 4, DV = HD / 64;       // DV: groups of four output columns per thread
     extern __shared__ __align__(16) float af_smem[];
+    ni_launch_dependents();                                // the output projection asks for its weights meanwhile
     float* qs = af_smem;                                   // [ROWS][PITCH]
     float* ks = qs + ROWS * PITCH;                         // [2][64][PITCH]
     float* vs = ks + 2 * AF_KB * PITCH;                    // [2][64][PITCH]
@@ -318,6 +319,7 @@ attention_f32_rows_kernel(AfParams p, const int* __restrict__ token_list, float*
     constexpr int PITCH = HD + 4, PP = AF_KB + 4, STEP = AF_THREADS / HD, OUTS = (GM + STEP - 1) / STEP;
     constexpr int QR = GM / 2 > 0 ? (GM + 1) / 2 : 1;      // rows of scores per thread (64 keys x 2)
     extern __shared__ __align__(16) float af_smem[];
+    ni_launch_dependents();
     float* qs = af_smem;                                   // [GM][PITCH]
     float* ks = qs + GM * PITCH;
     float* vs = ks + 2 * AF_KB * PITCH;
@@ -476,6 +478,7 @@ attention_f32_rows_kernel(AfParams p, const int* __restrict__ token_list, float*
 template <int HD>
 __global__ void __launch_bounds__(HD)
 attention_f32_merge_kernel(AfParams p, const int* __restrict__ token_list, const float* __restrict__ partials, int segments) {
+    ni_launch_dependents();
     const int ti = blockIdx.x / p.n_q, head = blockIdx.x % p.n_q, kvh = head / p.group, r = head % p.group, d = threadIdx.x;
     const int t = token_list ? token_list[ti] : ti;
     const int pos = p.positions[t], s0 = af_first(p, pos) / AF_SEG, s1 = pos / AF_SEG;

@@ -23,6 +23,10 @@
         return e__ == cudaSuccess ? NI_OK : (int)e__;  \
     } while (0)
 
+// A kernel launched with programmatic serialisation behind the calling one may begin its preparations (it waits for the calling
+// one's results by itself).
+__device__ __forceinline__ void ni_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
+
 // Streaming multiprocessors of the current device (asked once per device; 148 on a B200).
 // Grid sizes and work splits are derived from it, never from a literal.
 static inline int ni_sm_count() {

@@ -120,6 +120,7 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const TD* __restri
                                        const int* __restrict__ rows, int d, const float* __restrict__ dscale,
                                        const float* __restrict__ dshift) {
     __shared__ float scratch[32];
+    if (sizeof(TO) == 4) ni_launch_dependents();       // the product behind it asks for its weights meanwhile (gemm_f32_tc.cu)
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
     float* hr = h + (size_t)src * d;
@@ -335,6 +336,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out
 template <typename T>
 __global__ void swiglu_blocked_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int n_tokens,
                                       int inter, float c1, float c2) {
+    if (sizeof(T) == 4) ni_launch_dependents();
     const int blocks_per_row = inter >> 3;
     const size_t total = (size_t)n_tokens * blocks_per_row;
     size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

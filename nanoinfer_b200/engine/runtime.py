@@ -175,7 +175,7 @@ class Runtime:
         out_dtype = out_dtype or self.dtype
         if self.dtype == torch.float32:
             out = self.empty(m, n, dtype=torch.float32)
-            ops.gemm_f32(x, w, out)
+            ops.linear_f32(x, w, out)
             return out if affine is None else ops.ScaledAddition(out, *affine)
         if residual is None and self.swapped_gemm(m, n, x.shape[1]):
             out = self.empty(m, n, dtype=out_dtype)
@@ -185,13 +185,13 @@ class Runtime:
 
     def heads_linear(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """One product per head: y[t, h, :] = x[t, h, :] . w[h]^T for x [T, H K] (some columns of a wider
-        matrix will do) and w [H, N, K]; returns [T, H N] in the compute dtype.  float32: the package's FFMA kernel, one ascending chain per
-        element; bfloat16: a library batched product (FP32 accumulation) written straight into y."""
+        matrix will do) and w [H, N, K]; returns [T, H N] in the compute dtype.  float32: the package's own kernels, an order
+        of sums that the row's length fixes; bfloat16: a library batched product (FP32 accumulation) written straight into y."""
         n_heads, n, k = w.shape
         t = x.shape[0]
         y = self.empty(t, n_heads * n)
         if self.dtype == torch.float32:
-            ops.gemm_f32_heads(x, w, y)
+            ops.linear_f32(x, w, y)
         else:
             torch.bmm(x.view(t, n_heads, k).transpose(0, 1), w.transpose(1, 2), out=y.view(t, n_heads, n).transpose(0, 1))
         return y

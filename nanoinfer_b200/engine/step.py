@@ -233,7 +233,7 @@ class ModelRunner:
         # Compile (in parallel) and load what THIS model needs in this precision before the first step: the
         # libraries every model uses, and those its parts name.  Anything else is built when first used.
         bf16 = self.rt.dtype == torch.bfloat16
-        needed = {"elementwise"} | ({"gemv_bf16", "gemv_ksplit"} if bf16 else {"gemm_f32"}) | ({"decode_fused"} if fused_decode else set())
+        needed = {"elementwise"} | ({"gemv_bf16", "gemv_ksplit"} if bf16 else {"gemm_f32", "gemm_f32_tc"}) | ({"decode_fused"} if fused_decode else set())
         all_parts = [q for b in self.model.blocks if b is not None
                      for p in (b, getattr(b, "mixer", None), getattr(b, "feed_forward", None)) for q in with_sub_parts(p)] \
             + [self.model.embedding, self.model.head, self.model]

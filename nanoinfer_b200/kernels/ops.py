@@ -47,6 +47,10 @@ _SIGNATURES = {
         "ni_gemm_f32_variant": [_I, _P, _P, _P, _I, _I, _I, _P],
         "ni_gemm_f32_heads": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
     },
+    "gemm_f32_tc": {
+        "ni_gemm_f32_tc": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+        "ni_gemm_f32_tc_set_wait": [_LL, _I],
+    },
     "pointwise": {
         "ni_embedding_sinusoid": [_P, _P, _P, _I, _P, _P, _I, _I, _I, _P],
         "ni_cast_bf16": [_P, _P, _LL, _P],
@@ -522,8 +526,8 @@ def attention_f32(q, k_pages, v_pages, out, positions, seq_of_token, block_table
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, variant: int = 0) -> None:
-    """out[M, N] = x[M, K] . w[N, K]^T, all float32, plain FP32 arithmetic.  ``variant``: one of the kernels of
-    csrc/gemm_f32.cu by its number there (they give the same bits; for tests and measurements), 0: chosen by the sizes."""
+    """out[M, N] = x[M, K] . w[N, K]^T, all float32, every element one ascending chain of multiply-adds.  ``variant``: one of the
+    kernels of csrc/gemm_f32.cu by its number there (they give the same bits; for tests and measurements), 0: chosen by the sizes."""
     m, k = x.shape
     n = w.shape[0]
     if w.shape[1] != k or out.shape != (m, n):
@@ -533,17 +537,47 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, variant: int =
     _check(lib.ni_gemm_f32_variant(int(variant), *args) if variant else lib.ni_gemm_f32(*args), "gemm_f32")
 
 
-def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """One product per head, plain FP32: out[m, h, :] = x[m, h, :] . w[h]^T with x [M, H K] (its rows may
-    be some columns of a wider matrix), w [H, N, K], out [M, H N], all float32."""
+def _heads_of(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, what: str):
+    """Arguments of a product per head, looked over."""
     h, n, k = w.shape
     m = x.shape[0]
     if x.shape != (m, h * k) or out.shape != (m, h * n):
-        raise KernelError("gemm_f32_heads: shapes do not agree")
+        raise KernelError(f"{what}: shapes do not agree")
     if not x.is_cuda or x.dtype != torch.float32 or x.stride(1) != 1 or x.stride(0) < h * k:
-        raise KernelError("gemm_f32_heads: x must be float32 rows on the device, each row contiguous")
-    _check(load("gemm_f32").ni_gemm_f32_heads(x.data_ptr(), x.stride(0), _dev(w, "w", torch.float32),
-                                              _dev(out, "out", torch.float32), m, n, k, h, _stream()), "gemm_f32_heads")
+        raise KernelError(f"{what}: x must be float32 rows on the device, each row contiguous")
+    return x.data_ptr(), x.stride(0), _dev(w, "w", torch.float32), _dev(out, "out", torch.float32), m, n, k, h
+
+
+def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """One product per head, plain FP32: out[m, h, :] = x[m, h, :] . w[h]^T with x [M, H K] (its rows may
+    be some columns of a wider matrix), w [H, N, K], out [M, H N], all float32."""
+    _check(load("gemm_f32").ni_gemm_f32_heads(*_heads_of(x, w, out, "gemm_f32_heads"), _stream()), "gemm_f32_heads")
+
+
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int = 0, splits: int = 0) -> None:
+    """gemm_f32_heads on the tensor cores, every number cut in two (csrc/gemm_f32_tc.cu); w may be [N, K] for one head.  ``rows`` (16,
+    32, 64, 128: rows of x in a tile) and ``splits`` (blocks that share K, up to 8): 0 leaves them to the sizes; the bits are the
+    same."""
+    args = _heads_of(x, w if w.dim() == 3 else w.unsqueeze(0), out, "gemm_f32_tc")
+    _check(load("gemm_f32_tc").ni_gemm_f32_tc(*args, int(rows), int(splits), _error_word(x.device).data_ptr(), _stream()), "gemm_f32_tc")
+
+
+# Rows of at least this many columns go to the tensor cores as numbers cut in two, shorter ones to the chains of csrc/gemm_f32.cu.  The
+# rule looks at nothing but the row's length, so that a row's bits depend on no other row.  Relative error against 64 bits, cut in
+# two / as a chain: normal numbers 3.0e-7 / 4.1e-7 at 512 columns, 3.0e-7 / 5.7e-7 at 1,024, 3.1e-7 / 1.6e-6 at 8,192; positive numbers
+# 3.6e-7 / 3.1e-7, 3.7e-7 / 4.9e-7, 3.6e-7 / 1.3e-6.  Below the line the chain is as close, and short rows have little to gain.
+F32_CUT_COLUMNS = 1024
+
+
+def linear_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """The 32-bit path's product: out = x . w^T with w [N, K], or one per head with w [H, N, K] (see gemm_f32_heads).  A row of out
+    depends on its row of x alone, whatever lies beside it."""
+    if w.shape[-1] >= F32_CUT_COLUMNS:
+        gemm_f32_tc(x, w, out)
+    elif w.dim() == 3:
+        gemm_f32_heads(x, w, out)
+    else:
+        gemm_f32(x, w, out)
 
 
 def embedding_sinusoid(tokens: torch.Tensor, positions: torch.Tensor, table: torch.Tensor, inv_freq: torch.Tensor,
@@ -1646,6 +1680,10 @@ DEVICE_ERROR_CODES = {
     31: "fused decode step (decode_fused): a grid barrier was not reached by every block in time",
     32: "fused decode step (decode_fused): the weight loader gave up waiting for a free stage",
     33: "fused decode step (decode_fused): a consumer gave up waiting for its weights",
+    51: "FP32 product on the tensor cores (gemm_f32_tc): the loader gave up waiting",
+    52: "FP32 product on the tensor cores (gemm_f32_tc): the cutting warps gave up waiting",
+    53: "FP32 product on the tensor cores (gemm_f32_tc): the MMA issuer gave up waiting",
+    54: "FP32 product on the tensor cores (gemm_f32_tc): the sums gave up waiting",
     41: "delta rule in chunks (delta_chunk): the scan gave up waiting for a chunk's operands",
 }
 
@@ -1683,7 +1721,7 @@ def check_device_errors(device=None) -> None:
 
 
 _WAIT_SETTERS = {"gemm_tc": "ni_gemm_tc_set_wait", "gemm_tc2": "ni_gemm_tc2_set_wait",
-                 "gemm_swap_tc": "ni_gemm_swap_tc_set_wait",
+                 "gemm_swap_tc": "ni_gemm_swap_tc_set_wait", "gemm_f32_tc": "ni_gemm_f32_tc_set_wait",
                  "attention_prefill_tc": "ni_attention_prefill_tc_set_wait", "delta_chunk": "ni_delta_chunk_set_wait"}
 
 
