@@ -18,6 +18,8 @@
 //  * the uniform number is Philox4x32-10 keyed by the request's seed with the index of the
 //    generated token as counter: it does not depend on batching;
 //  * the draw walks the vocabulary in id order: first id whose inclusive mass exceeds u * total.
+#include <string.h>
+
 #include "common.cuh"
 
 #define SAMPLE_THREADS 1024
@@ -402,6 +404,8 @@ __device__ __forceinline__ void sc_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
+__device__ __forceinline__ void sc_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void sc_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void sc_st_remote(const unsigned long long* local_addr, uint32_t rank, unsigned long long v) {
     uint32_t a = (uint32_t)__cvta_generic_to_shared(local_addr), remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(a), "r"(rank));
@@ -421,17 +425,34 @@ struct ScScratch {
     unsigned long long red[SC_WARPS];
     unsigned long long digit_rest[2];    // the chosen digit and what is left of the count or mass
     int chosen;
+    uint32_t low[SC_WARPS];              // ordered keys of the warps' least, then of the block's (in low[0])
 };
 
 // ---- rows with top-k: a few candidates instead of passes over the vocabulary --------------------------------------
-// The k largest of a row are among the k largest of each block's slice.  While a block loads its slice it counts the ordered
-// keys by their leading 12 bits; from the coarse value that at least k of its tokens reach (usually a few dozen more than k) it
-// sends its tokens to the cluster's first block, which finds the k-th largest, the top-p floor and the draw among those alone -
-// with the same keys, the same 64-bit masses and the same rules, so the same token.  A slice with more than SC_CANDIDATES
-// tokens from its coarse value on (a large k, rows of equal logits) sends the whole row down the general path below.
-// 8 rows of 128,256 logits, top-k 50 and top-p 0.9: 21 us, against 102 us as eleven passes of the cluster over the row.
-#define SC_COARSE_BITS 12
-#define SC_COARSE (1 << SC_COARSE_BITS)
+// The k largest of a row are among the k largest of each block's slice.  Every thread keeps the largest of its tokens while the
+// slice is loaded; these are counted by coarse value, 4,096 equal steps between the least and the largest of them.  From the coarse
+// value that the largest tokens of at least k threads reach (few threads have two of the k) the block sends its tokens to the
+// cluster's first block, which finds the k-th largest, the top-p floor and the draw among those alone - with the same keys, the
+// same 64-bit masses and the same rules, so the same token.  (Before, every token was counted by the leading 12 bits of its key while
+// it was loaded: 32 shared-memory additions per thread instead of one, and half again as many candidates.)  A slice with fewer than
+// four tokens per thread counts them all.  A slice with more than SC_CANDIDATES tokens from its coarse value on (a large k, rows of
+// equal logits), or fewer than k threads with a finite token, sends the whole row down the general path below.
+// 8 rows of 128,256 logits, top-k 50 and top-p 0.9: 14.3 us (21.2 as above), against 102 us as eleven passes of the cluster over the
+// row; k = 200 21.7 (27.0); 64 rows, k = 50 40.6 (49.6).
+#define SC_COARSE 4096
+// The coarse value of a number: -1 below `lo`.  (Monotonic in v, which is all that counts.)
+struct ScScale {
+    float lo, scale;
+    __device__ __forceinline__ ScScale(float least, float largest) : lo(least), scale((SC_COARSE - 1) / (largest - least)) {
+        if (!(scale < INFINITY)) scale = 0.f;                // all of them equal
+    }
+    __device__ __forceinline__ int operator()(float v) const {
+        if (!(v >= lo)) return -1;
+        const int c = (int)((v - lo) * scale);
+        return c < SC_COARSE - 1 ? c : SC_COARSE - 1;
+    }
+};
+__device__ __forceinline__ float value_of(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key); }
 // Of a block; the first block's list [SC_RANKS][SC_CANDIDATES] and every block's two numbers of every block lie where the general
 // path has its histograms and its first gather buffer, the coarse counts where it has its second.
 #define SC_CANDIDATES 504
@@ -439,11 +460,12 @@ struct ScScratch {
 static_assert(SC_RANKS * SC_MAX_SLICE <= 1 << 24, "an id fits the 24 bits of sc_mass_select");
 static_assert(SC_RANKS * (SC_CANDIDATES + 2) <= SC_HISTS * 256 + SC_RANKS * 256, "the candidates and the blocks' numbers fit");
 static_assert(SC_COARSE * 4 <= SC_RANKS * 256 * 8, "the coarse counts fit");
+static_assert(SC_PAIRS <= SC_THREADS && 2 * 256 >= SC_THREADS && (SC_WARPS & (SC_WARPS - 1)) == 0, "a thread per token");
 static_assert(SC_COARSE % SC_THREADS == 0, "every thread sums the same number of coarse counts");
 
-// s.hist[1] <- how many (more than SC_CANDIDATES: nothing was sent).  s.chosen is 0 before.
-__device__ void sc_send_candidates(const float* z, int n, int lo, int k, const uint32_t* coarse, unsigned long long* list, ScScratch& s,
-                                   uint32_t rank) {
+// s.digit_rest <- the largest coarse value that at least k of the counted tokens reach, and how many do; -1 and `all` if fewer than k
+// were counted.
+__device__ void sc_reach(const uint32_t* coarse, int k, unsigned long long all, ScScratch& s) {
     constexpr int PER = SC_COARSE / SC_THREADS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // thread t holds counts [PER t, PER t + PER); `above` counts everything beyond them
@@ -460,7 +482,6 @@ __device__ void sc_send_candidates(const float* z, int n, int lo, int k, const u
     __syncthreads();
     uint32_t above = incl - mine;
     for (int w = warp + 1; w < SC_WARPS; ++w) above += (uint32_t)s.red[w];
-    // the coarse value: the largest one that at least k tokens reach, or 0
     if (above < (uint32_t)k && above + mine >= (uint32_t)k) {
         uint32_t reach = above;
         for (int j = PER - 1; j >= 0; --j) {
@@ -468,18 +489,39 @@ __device__ void sc_send_candidates(const float* z, int n, int lo, int k, const u
             if (reach >= (uint32_t)k) { s.digit_rest[0] = (unsigned long long)(PER * tid + j); s.digit_rest[1] = reach; break; }
         }
     }
-    if (tid == 0 && above + mine < (uint32_t)k) { s.digit_rest[0] = 0ull; s.digit_rest[1] = (unsigned long long)n; }
+    if (tid == 0 && above + mine < (uint32_t)k) { s.digit_rest[0] = ~0ull; s.digit_rest[1] = all; }     // (tid 0: all are above + mine)
     __syncthreads();
-    const uint32_t from = (uint32_t)s.digit_rest[0];
-    if (tid == 0) s.hist[1] = s.digit_rest[1];
-    if (s.digit_rest[1] <= SC_CANDIDATES) {
-        for (int i = tid; i < n; i += blockDim.x) {
-            const uint32_t key = ordered_key(z[i]);
-            if ((key >> (32 - SC_COARSE_BITS)) >= from) {
-                const int at = atomicAdd(&s.chosen, 1);
-                sc_st_remote(list + rank * SC_CANDIDATES + at, 0u, ((unsigned long long)key << 32) | (unsigned long long)(uint32_t)(lo + i));
+}
+
+// s.hist[1] <- how many (more than SC_CANDIDATES: not all were sent).  s.chosen is 0 before.
+__device__ void sc_send_candidates(const float* z, int n, int lo, int k, const uint32_t* coarse, unsigned long long* list, ScScratch& s,
+                                   uint32_t rank, const ScScale& coarse_of, bool sparse) {
+    const int tid = threadIdx.x;
+    // (fewer than k: if all tokens were counted, they all go)
+    sc_reach(coarse, k, sparse ? (unsigned long long)SC_CANDIDATES + 1ull : (unsigned long long)n, s);
+    const int from = (int)s.digit_rest[0];
+    if (s.digit_rest[1] <= SC_CANDIDATES) {                  // (what was counted: with one count per thread there may be more)
+        for (int i0 = tid; i0 < n; i0 += 32 * SC_THREADS) {
+            uint32_t hits = 0u;                              // which of this thread's next 32 tokens go: no branch per token
+#pragma unroll 8
+            for (int u = 0; u < 32; ++u) {
+                const int i = i0 + u * SC_THREADS;
+                if (i < n) hits |= (uint32_t)(coarse_of(z[i]) >= from) << u;
+            }
+            if (hits) {
+                int at = atomicAdd(&s.chosen, __popc(hits));
+                for (; hits; hits &= hits - 1u, ++at) {
+                    const int i = i0 + (__ffs(hits) - 1) * SC_THREADS;
+                    if (at < SC_CANDIDATES)
+                        sc_st_remote(list + rank * SC_CANDIDATES + at, 0u,
+                                     ((unsigned long long)ordered_key(z[i]) << 32) | (unsigned long long)(uint32_t)(lo + i));
+                }
             }
         }
+        __syncthreads();
+        if (tid == 0) s.hist[1] = (unsigned long long)s.chosen;
+    } else if (tid == 0) {
+        s.hist[1] = s.digit_rest[1];
     }
     __syncthreads();
 }
@@ -535,77 +577,190 @@ __device__ uint32_t sc_mass_select(const unsigned long long* list, int n, uint32
     return prefix;
 }
 
-// The first block's part: list [SC_RANKS][SC_CANDIDATES] of (key << 32) | id, counts[2 c + 1] of them per block.  Up to SC_PAIRS
-// tokens that stay are compared with one another; more (ties at the k-th place: up to 4,032 stay) go by passes over their bits.
-// 8 rows, k = 50, top-p 0.9, us in pairs / in passes / as passes of the cluster over the row: 170 that stay 28.7 (without ties
-// 22.6) / - / 178, 520 58.3 / 47.7 / 179, 1,060 141 / 60.3 / 182, 3,960 1,317 / 93.8 / 197; without top-p 520 39.0 / 27.9 / 154.
+// The first block's part: list [SC_RANKS][SC_CANDIDATES] of (key << 32) | id, counts[2 c + 1] of them per block.  The candidates are
+// counted by coarse value once more: those above the value of the k-th largest stay, those of that value (a few) are compared with
+// one another - or, if they are many, all go by passes over their bits.  Up to SC_PAIRS tokens that stay are compared with one
+// another; more (ties at the k-th place: up to 4,032 stay) go by passes over their bits.
+// 8 rows, k = 50, top-p 0.9, us now / every candidate by passes over its bits / as passes of the cluster over the row: without ties
+// 14.3 / 21.2 / 102; 128 tied at the k-th place 22.6 / 28.8 / 178, 480 49.3 / 47.9 / 179, 1,024 63 / 60.5 / 182, 3,920 107 / 94 / 197.
 __device__ void sc_pick(unsigned long long* list, const unsigned long long* counts, uint32_t* work, ScScratch& s, float m, int k, float p,
                         unsigned long long seed, unsigned long long counter, int* out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int SLOTS = SC_RANKS * SC_CANDIDATES;
-    // the k-th largest key: four passes of 8 bits, 256 counts
-    uint32_t* bins = work;
-    uint32_t prefix = 0u, mask = 0u, remaining = (uint32_t)k;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        if (tid < 256) bins[tid] = 0u;
-        __syncthreads();
-        for (int i = tid; i < SLOTS; i += blockDim.x) {
-            if ((unsigned long long)(i % SC_CANDIDATES) >= counts[2 * (i / SC_CANDIDATES) + 1]) continue;
-            const uint32_t key = (uint32_t)(list[i] >> 32);
-            if ((key & mask) == prefix) atomicAdd(&bins[(key >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (warp == 0) {                                     // lane l holds bins 8 l .. 8 l + 7
-            uint32_t mine = 0u;
-            for (int j = 0; j < 8; ++j) mine += bins[8 * lane + j];
-            uint32_t incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t nb = __shfl_down_sync(0xffffffffu, incl, o);
-                if (lane + o < 32) incl += nb;
-            }
-            uint32_t above = incl - mine;
-            if (above < remaining && above + mine >= remaining) {
-                int j = 7;
-                while (above + bins[8 * lane + j] < remaining) above += bins[8 * lane + j--];
-                s.digit_rest[0] = (unsigned long long)(8 * lane + j);
-                s.digit_rest[1] = (unsigned long long)(remaining - above);
-            }
-        }
-        __syncthreads();
-        prefix |= (uint32_t)s.digit_rest[0] << shift;
-        mask |= 255u << shift;
-        remaining = (uint32_t)s.digit_rest[1];
-    }
-    const uint32_t key_floor = prefix;
-    // those that stay, side by side: (bits of exp(z - m) << 32) | id, and their masses
-    __syncthreads();
-    if (tid == 0) s.chosen = 0;
-    __syncthreads();
     constexpr int EACH = (SLOTS + SC_THREADS - 1) / SC_THREADS;
     unsigned long long kept[EACH];
     int n_kept = 0;
+    int sent = 0;                                            // candidates in all
+    for (int c = 0; c < SC_RANKS; ++c) sent += (int)counts[2 * c + 1];
+    const ScScale coarse_of(value_of(s.low[0]), m);          // (less than this block's least: value 0)
+    const auto coarse = [&](unsigned long long entry) { return max(0, coarse_of(value_of((uint32_t)(entry >> 32)))); };
+    for (int b = tid; b < SC_COARSE; b += SC_THREADS) work[b] = 0u;
+    if (tid == 0) s.chosen = 0;
+    unsigned long long mine[EACH];                           // candidates tid, tid + SC_THREADS, .. of all blocks' one after the other
+    int have = 0;
 #pragma unroll
     for (int u = 0; u < EACH; ++u) {
-        const int i = tid + u * SC_THREADS;
-        kept[u] = 0ull;
-        if (i < SLOTS && (unsigned long long)(i % SC_CANDIDATES) < counts[2 * (i / SC_CANDIDATES) + 1]) {
-            const uint32_t key = (uint32_t)(list[i] >> 32);
-            if (key >= key_floor) {
-                const float v = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
-                kept[u] = ((unsigned long long)__float_as_uint(expf(v - m)) << 32) | (list[i] & 0xffffffffull);
-                n_kept |= 1 << u;
+        mine[u] = 0ull;
+        if (u * SC_THREADS >= sent) continue;                // (the same for all threads: few candidates cost one turn)
+        int at = tid + u * SC_THREADS, place = at;
+        if (at < sent) {
+            have |= 1 << u;
+#pragma unroll
+            for (int c = 0; c < SC_RANKS - 1; ++c) {
+                const int here = (int)counts[2 * c + 1];
+                if (at >= here) { at -= here; place = (c + 1) * SC_CANDIDATES + at; } else at = -1;
             }
+            mine[u] = list[place];
         }
     }
-    __syncthreads();                                         // the list and the counts have been read
-    unsigned long long total = 0ull;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < EACH; ++u) {
+        if (u * SC_THREADS >= sent) continue;
+        const bool in = have >> u & 1;
+        const int value = coarse(mine[u]);
+        const unsigned who = __ballot_sync(0xffffffffu, in);
+        const int first = __shfl_sync(0xffffffffu, value, who ? __ffs(who) - 1 : 0);
+        if (__all_sync(0xffffffffu, !in || value == first)) {                    // (tied tokens: one addition per warp)
+            if (lane == 0 && who) atomicAdd(&work[first], (uint32_t)__popc(who));
+        } else if (in) {
+            atomicAdd(&work[value], 1u);
+        }
+    }
+    __syncthreads();
+    sc_reach(work, k, (unsigned long long)sent, s);
+    const int from = max(0, (int)s.digit_rest[0]), tied = (int)work[from], rest = k - ((int)s.digit_rest[1] - tied);       // of `tied`, `rest` stay
+    uint32_t* same = reinterpret_cast<uint32_t*>(s.hist);    // the keys of that value, if they are no more than the block's threads
+    uint32_t key_floor = 0u;
+    if (tied <= SC_THREADS) {
+#pragma unroll
+        for (int u = 0; u < EACH; ++u)
+            if (u * SC_THREADS < sent && have >> u & 1 && coarse(mine[u]) == from)
+                same[atomicAdd(&s.chosen, 1)] = (uint32_t)(mine[u] >> 32);
+        __syncthreads();
+    } else {
+        // the k-th largest key: four passes of 8 bits, 256 counts
+        uint32_t* bins = work;
+        uint32_t prefix = 0u, mask = 0u, remaining = (uint32_t)k;
+        for (int shift = 24; shift >= 0; shift -= 8) {
+            if (tid < 256) bins[tid] = 0u;
+            __syncthreads();
+            for (int i = tid; i < SLOTS; i += blockDim.x) {
+                if ((unsigned long long)(i % SC_CANDIDATES) >= counts[2 * (i / SC_CANDIDATES) + 1]) continue;
+                const uint32_t key = (uint32_t)(list[i] >> 32);
+                if ((key & mask) == prefix) atomicAdd(&bins[(key >> shift) & 255u], 1u);
+            }
+            __syncthreads();
+            if (warp == 0) {                                 // lane l holds bins 8 l .. 8 l + 7
+                uint32_t mine = 0u;
+                for (int j = 0; j < 8; ++j) mine += bins[8 * lane + j];
+                uint32_t incl = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t nb = __shfl_down_sync(0xffffffffu, incl, o);
+                    if (lane + o < 32) incl += nb;
+                }
+                uint32_t above = incl - mine;
+                if (above < remaining && above + mine >= remaining) {
+                    int j = 7;
+                    while (above + bins[8 * lane + j] < remaining) above += bins[8 * lane + j--];
+                    s.digit_rest[0] = (unsigned long long)(8 * lane + j);
+                    s.digit_rest[1] = (unsigned long long)(remaining - above);
+                }
+            }
+            __syncthreads();
+            prefix |= (uint32_t)s.digit_rest[0] << shift;
+            mask |= 255u << shift;
+            remaining = (uint32_t)s.digit_rest[1];
+        }
+        key_floor = prefix;
+    }
+#pragma unroll
+    for (int u = 0; u < EACH; ++u) {
+        if (u * SC_THREADS >= sent || !(have >> u & 1)) continue;
+        const uint32_t key = (uint32_t)(mine[u] >> 32);
+        const int value = coarse(mine[u]);
+        bool stays = tied <= SC_THREADS ? value > from : key >= key_floor;
+        if (tied <= SC_THREADS && value == from) {           // fewer than `rest` of its value are larger
+            int larger = 0;
+            for (int j = 0; j < tied; ++j) larger += same[j] > key;
+            stays = larger < rest;
+        }
+        if (stays) {
+            const float v = value_of(key);
+            kept[u] = ((unsigned long long)__float_as_uint(expf(v - m)) << 32) | (mine[u] & 0xffffffffull);
+            n_kept |= 1 << u;
+        }
+    }
+    __syncthreads();                                         // the list, the counts and what was chosen so far have been read
+    // those that stay, side by side: (bits of exp(z - m) << 32) | id
+    if (tid == 0) { s.digit_rest[0] = 0ull; s.chosen = 0; }
+    __syncthreads();
 #pragma unroll
     for (int u = 0; u < EACH; ++u)
-        if (n_kept >> u & 1) {
-            list[atomicAdd(&s.chosen, 1)] = kept[u];
-            total += mass_of(__uint_as_float((uint32_t)(kept[u] >> 32)));
+        if (u * SC_THREADS < sent && n_kept >> u & 1) list[atomicAdd(&s.chosen, 1)] = kept[u];
+    __syncthreads();
+    const int n = s.chosen;
+    const bool nucleus = p > 0.f && p < 1.f;
+    const uint32_t word = philox_first_word(seed, counter);
+    const double uniform = ((double)(word >> 8) + 0.5) * (1.0 / 16777216.0);
+    auto target_of = [&](unsigned long long total) -> unsigned long long {
+        const unsigned long long t = (unsigned long long)(uniform * (double)total);
+        return total > 0ull && t >= total ? total - 1ull : t;
+    };
+    if (n <= SC_PAIRS) {
+        // masses side by side; four threads share a token
+        unsigned long long* masses = list + SC_PAIRS;
+        if (tid < n) masses[tid] = mass_of(__uint_as_float((uint32_t)(list[tid] >> 32)));
+        __syncthreads();
+        constexpr int TOKENS = SC_THREADS / 4;
+        const int part = tid & 3, n_up = (n + TOKENS - 1) & -TOKENS;
+        const auto quad = [](unsigned long long v) {
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            return v + __shfl_xor_sync(0xffffffffu, v, 2);
+        };
+        // top-p: the largest probability such that the masses from it upwards exceed p * total (none: everything stays)
+        uint32_t e_floor = 0u;
+        if (nucleus) {
+            for (int i = tid >> 2; i < n_up; i += TOKENS) {
+                const uint32_t bits = i < n ? (uint32_t)(list[i] >> 32) : 0u;
+                unsigned long long upward = 0ull, total = 0ull;
+#pragma unroll 4
+                for (int j = part; j < n; j += 4) {
+                    const unsigned long long x = masses[j];
+                    total += x;
+                    if ((uint32_t)(list[j] >> 32) >= bits) upward += x;
+                }
+                upward = quad(upward);
+                total = quad(total);
+                if (part == 0 && i < n && upward > (unsigned long long)((double)p * (double)total))
+                    atomicMax(&s.digit_rest[0], (unsigned long long)bits);
+            }
+            __syncthreads();
+            e_floor = (uint32_t)s.digit_rest[0];
         }
+        // the draw: the token whose stretch of the masses in id order holds the target
+        for (int i = tid >> 2; i < n_up; i += TOKENS) {
+            const uint32_t bits = i < n ? (uint32_t)(list[i] >> 32) : 0u, id = i < n ? (uint32_t)list[i] : 0u;
+            unsigned long long before = 0ull, total = 0ull;
+#pragma unroll 4
+            for (int j = part; j < n; j += 4) {
+                const unsigned long long other = list[j], x = (uint32_t)(other >> 32) >= e_floor ? masses[j] : 0ull;
+                total += x;
+                if ((uint32_t)other < id) before += x;
+            }
+            before = quad(before);
+            total = quad(total);
+            if (part || i >= n) continue;
+            const unsigned long long target = target_of(total);
+            if (total == 0ull) {
+                if (i == 0) *out = 0;
+            } else if (bits >= e_floor && before <= target && target < before + masses[i]) {
+                *out = (int)id;
+            }
+        }
+        return;
+    }
     auto block_sum = [&](unsigned long long v) -> unsigned long long {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -616,67 +771,47 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
         for (int w = 0; w < SC_WARPS; ++w) t += s.red[w];
         return t;
     };
-    if (tid == 0) s.digit_rest[0] = 0ull;
-    total = block_sum(total);                                // (its barriers publish the list)
-    const int n = s.chosen;
-    const bool pairs = n <= SC_PAIRS;
-    // top-p: the largest probability such that the masses from it upwards exceed p * total (none: everything stays)
-    uint32_t e_floor = 0u;
-    if (p > 0.f && p < 1.f) {
-        const unsigned long long limit = (unsigned long long)((double)p * (double)total);
-        if (pairs) {
-            for (int i = tid; i < n; i += blockDim.x) {
-                const uint32_t bits = (uint32_t)(list[i] >> 32);
-                unsigned long long upward = 0ull;
-                for (int j = 0; j < n; ++j) {
-                    const uint32_t other = (uint32_t)(list[j] >> 32);
-                    if (other >= bits) upward += mass_of(__uint_as_float(other));
-                }
-                if (upward > limit) atomicMax(&s.digit_rest[0], (unsigned long long)bits);
-            }
-            __syncthreads();
-            e_floor = (uint32_t)s.digit_rest[0];
-        } else if (total > limit) {
-            e_floor = sc_mass_select(list, n, 0u, false, limit, reinterpret_cast<unsigned long long*>(work), s);
-        }
+    auto kept_mass = [&](uint32_t e_floor) -> unsigned long long {
         unsigned long long local = 0ull;
         for (int i = tid; i < n; i += blockDim.x) {
             const uint32_t bits = (uint32_t)(list[i] >> 32);
             if (bits >= e_floor) local += mass_of(__uint_as_float(bits));
         }
-        total = block_sum(local);
+        return block_sum(local);
+    };
+    unsigned long long total = kept_mass(0u);
+    uint32_t e_floor = 0u;
+    if (nucleus) {
+        const unsigned long long limit = (unsigned long long)((double)p * (double)total);
+        if (total > limit) e_floor = sc_mass_select(list, n, 0u, false, limit, reinterpret_cast<unsigned long long*>(work), s);
+        total = kept_mass(e_floor);
     }
-    // the draw: the token whose stretch of the masses in id order holds the target
-    const uint32_t word = philox_first_word(seed, counter);
-    const double u = ((double)(word >> 8) + 0.5) * (1.0 / 16777216.0);
-    unsigned long long target = (unsigned long long)(u * (double)total);
-    if (total > 0ull && target >= total) target = total - 1ull;
     if (total == 0ull) {
         if (tid == 0) *out = 0;
         return;
     }
-    if (!pairs) {
-        const uint32_t key = sc_mass_select(list, n, e_floor, true, target, reinterpret_cast<unsigned long long*>(work), s);
-        if (tid == 0) *out = (int)(0xffffffu - key);
-        return;
-    }
-    for (int i = tid; i < n; i += blockDim.x) {
-        const uint32_t bits = (uint32_t)(list[i] >> 32), id = (uint32_t)list[i];
-        if (bits < e_floor) continue;
-        unsigned long long before = 0ull;
-        for (int j = 0; j < n; ++j) {
-            const uint32_t other = (uint32_t)(list[j] >> 32);
-            if ((uint32_t)list[j] < id && other >= e_floor) before += mass_of(__uint_as_float(other));
-        }
-        if (before <= target && target < before + mass_of(__uint_as_float(bits))) *out = (int)id;
-    }
+    const uint32_t key = sc_mass_select(list, n, e_floor, true, target_of(total), reinterpret_cast<unsigned long long*>(work), s);
+    if (tid == 0) *out = (int)(0xffffffu - key);
 }
 
+// The rows' parameters: arrays on the device, or - up to SC_VALUE_ROWS rows - the numbers themselves among the launch's arguments.
+#define SC_VALUE_ROWS 64
+struct ScArrays {
+    const float* temperatures;
+    const int* top_ks;
+    const float* top_ps;
+    const unsigned long long* seeds;
+    const unsigned long long* counters;
+};
+struct ScValues {
+    unsigned long long seeds[SC_VALUE_ROWS], counters[SC_VALUE_ROWS];
+    float temperatures[SC_VALUE_ROWS], top_ps[SC_VALUE_ROWS];
+    int top_ks[SC_VALUE_ROWS];
+};
+
+template <typename ARGS>
 __global__ void __launch_bounds__(SC_THREADS, 2)
-sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
-                      const float* __restrict__ temperatures, const int* __restrict__ top_ks,
-                      const float* __restrict__ top_ps, const unsigned long long* __restrict__ seeds,
-                      const unsigned long long* __restrict__ counters, int vocab, int slice) {
+sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out, const __grid_constant__ ARGS args, int vocab, int slice) {
     extern __shared__ __align__(16) unsigned char sc_smem[];
     float* z = reinterpret_cast<float*>(sc_smem);                                              // [slice]
     unsigned long long* warp_hists = reinterpret_cast<unsigned long long*>(z + slice);       // [SC_HISTS][256]
@@ -690,14 +825,14 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
     const int lo = (int)rank * slice;
     const int n = max(0, min(vocab, lo + slice) - lo);       // this block's ids: lo .. lo + n
     const int n_up = (n + 31) & ~31;
-    const float temp = temperatures[r];
+    const float temp = args.temperatures[r];
     const bool greedy = temp <= 0.f;
     const float inv_t = greedy ? 1.0f : 1.0f / temp;
-    sc_cluster_sync();                                       // every block of the cluster runs: its shared memory may be written
+    sc_cluster_arrive();                                     // this block runs: its shared memory may be written (waited for below)
     int pass = 0;                                            // which of the two gather buffers is next
     auto next_buf = [&]() { unsigned long long* b = gather + (size_t)(pass & 1) * SC_RANKS * 256; ++pass; return b; };
 
-    const int k = top_ks[r];
+    const int k = args.top_ks[r];
     const bool picks = !greedy && k > 0 && k < vocab;        // a row with top-k: its candidates are collected on the way
     uint32_t* coarse = reinterpret_cast<uint32_t*>(gather + SC_RANKS * 256);       // [4096], where the second gather buffer lies
     if (picks) {
@@ -707,16 +842,20 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
     }
 
     // ---- the slice into shared memory; its maximum (with the lowest id that has it) ----
-    unsigned long long best = 0ull;                          // (ordered key << 32) | (0xffffffff - id): larger is better
+    const bool wide = (vocab & 3) == 0 && (reinterpret_cast<size_t>(logits) & 15) == 0;         // rows and slices start on 16 bytes
+    const bool sparse = n >= 4 * SC_THREADS;                 // every thread has tokens: only its largest is counted
+    uint32_t least = 0xffffffffu;                            // ordered key of what is counted and finite
+    uint32_t largest = 0u;                                   // ordered key of this thread's largest, the lowest id that has it
+    int largest_at = -1;
     auto take = [&](int i, float logit) {
         const float v = logit * inv_t;
         z[i] = v;
         // (-0 and +0 are one value to a comparison, but not to the ordered key)
-        const unsigned long long cand = ((unsigned long long)ordered_key(v == 0.f ? 0.f : v) << 32) | (unsigned long long)(0xffffffffu - (uint32_t)(lo + i));
-        best = cand > best ? cand : best;
-        if (picks) atomicAdd(&coarse[ordered_key(v) >> (32 - SC_COARSE_BITS)], 1u);
+        const uint32_t key = ordered_key(v == 0.f ? 0.f : v);
+        if (key > largest || largest_at < 0) { largest = key; largest_at = i; }                  // (ids ascend)
+        if (!sparse && v > -INFINITY) least = min(least, key);
     };
-    if ((vocab & 3) == 0 && (reinterpret_cast<size_t>(logits) & 15) == 0) {       // rows and slices start on 16 bytes
+    if (wide) {
         constexpr int AHEAD = 4;
         for (int i0 = 4 * tid; i0 < n; i0 += 4 * AHEAD * SC_THREADS) {
             float4 v[AHEAD];
@@ -732,20 +871,46 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
     } else {
         for (int i = tid; i < n; i += blockDim.x) take(i, row[lo + i]);
     }
+    // (ordered key << 32) | (0xffffffff - id): larger is better
+    unsigned long long best = largest_at < 0 ? 0ull : ((unsigned long long)largest << 32) | (unsigned long long)(0xffffffffu - (uint32_t)(lo + largest_at));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         best = other > best ? other : best;
     }
-    if (lane == 0) s.red[warp] = best;
+    if (sparse && value_of(largest) > -INFINITY) least = largest;
+    least = __reduce_min_sync(0xffffffffu, least);
+    if (lane == 0) { s.red[warp] = best; s.low[warp] = least; }
     __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < SC_WARPS; ++w) best = s.red[w] > best ? s.red[w] : best;
-        s.hist[0] = best;
+    if (warp == 0) {
+        least = __reduce_min_sync(0xffffffffu, s.low[lane & (SC_WARPS - 1)]);
+        if (lane == 0) s.low[0] = least;
+        best = s.red[lane & (SC_WARPS - 1)];
+#pragma unroll
+        for (int o = SC_WARPS / 2; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+            best = other > best ? other : best;
+        }
+        if (lane == 0) s.hist[0] = best;
     }
+    sc_cluster_wait();                                       // every block of the cluster runs
     __syncthreads();
     if (picks) {
-        sc_send_candidates(z, n, lo, k, coarse, warp_hists, s, rank);              // (and their number into s.hist[1])
+        const float top = value_of((uint32_t)(s.hist[0] >> 32));
+        const ScScale coarse_of(value_of(s.low[0]), top);
+        const auto count = [&](float v) {
+            const int c = coarse_of(v);
+            if (c >= 0) atomicAdd(&coarse[c], 1u);
+        };
+        if (top < INFINITY) {                                // (an infinite or NaN logit: nothing counted, so the general path)
+            if (sparse) {
+                count(z[largest_at]);
+            } else {
+                for (int i = tid; i < n; i += blockDim.x) count(z[i]);
+            }
+        }
+        __syncthreads();
+        sc_send_candidates(z, n, lo, k, coarse, warp_hists, s, rank, coarse_of, sparse);              // (and their number into s.hist[1])
         unsigned long long* both = warp_hists + SC_RANKS * SC_CANDIDATES;          // every block's best and number
         if (tid < 2 * SC_RANKS) sc_st_remote(both + 2 * rank + (tid & 1), (uint32_t)(tid >> 1), s.hist[tid & 1]);
         sc_cluster_sync();
@@ -758,8 +923,8 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
         if (all_sent) {                                      // (the same in every block) the first block has all that can be drawn
             const uint32_t top = (uint32_t)(best >> 32);
             if (rank == 0)
-                sc_pick(warp_hists, both, coarse, s, __uint_as_float((top & 0x80000000u) ? (top & 0x7fffffffu) : ~top), k, top_ps[r],
-                        seeds[r], counters[r], out + r);
+                sc_pick(warp_hists, both, coarse, s, __uint_as_float((top & 0x80000000u) ? (top & 0x7fffffffu) : ~top), k, args.top_ps[r],
+                        args.seeds[r], args.counters[r], out + r);
             return;
         }
         pass = 1;                                            // a slow block may still read the numbers in the first buffer
@@ -876,14 +1041,14 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out,
     uint32_t key_floor = 0u, e_floor = 0u;
     if (picks) key_floor = radix_select(false, 0u, (unsigned long long)k, false);
     unsigned long long total = kept_total(key_floor, 0u);
-    const float p = top_ps[r];
+    const float p = args.top_ps[r];
     if (p > 0.f && p < 1.f) {
         e_floor = radix_select(true, key_floor, (unsigned long long)((double)p * (double)total), true);
         total = kept_total(key_floor, e_floor);
     }
 
     // ---- draw: first id (in id order) whose inclusive mass exceeds u * total ----
-    const uint32_t word = philox_first_word(seeds[r], counters[r]);
+    const uint32_t word = philox_first_word(args.seeds[r], args.counters[r]);
     const double u = ((double)(word >> 8) + 0.5) * (1.0 / 16777216.0);
     unsigned long long target = (unsigned long long)(u * (double)total);
     if (total > 0ull && target >= total) target = total - 1ull;
@@ -938,38 +1103,58 @@ static int sample_by_cluster = 1;
 // 0: always the one-block-per-row kernel (for comparisons); 1: a cluster per row where it fits (the default).
 NI_EXPORT int ni_sample_set_cluster(int on) { sample_by_cluster = on; return NI_OK; }
 
+static int sc_slice(int vocab) { return (((vocab + SC_RANKS - 1) / SC_RANKS) + 31) & ~31; }
+// a cluster per row while a block's slice of the vocabulary fits its shared memory
+static bool sc_takes(int vocab) { return sample_by_cluster && vocab >= 4096 && sc_slice(vocab) <= SC_MAX_SLICE; }
+
+template <typename ARGS>
+static int sc_launch(const float* logits, int* out, const ARGS& args, int n_rows, int vocab, cudaStream_t stream) {
+    const int slice = sc_slice(vocab);
+    const size_t sc_smem = (size_t)slice * sizeof(float) + (size_t)(SC_HISTS + 2 * SC_RANKS) * 256 * sizeof(unsigned long long);
+    static size_t sc_configured = 0;
+    if (sc_configured < sc_smem) {
+        cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel<ARGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_smem);
+        if (e != cudaSuccess) return (int)e;
+        sc_configured = sc_smem;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n_rows * SC_RANKS);
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.dynamicSmemBytes = sc_smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SC_RANKS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<ARGS>, logits, out, args, vocab, slice);
+    return e == cudaSuccess ? NI_OK : (int)e;
+}
+
+// The same for up to SC_VALUE_ROWS rows whose parameters are on the host: they travel with the launch, so that the caller needs no
+// copy to the device, no pinned buffer and no event.  words: seeds (64 bits) of all rows, counters (64 bits), temperatures, top_ps
+// (float), top_ks (int), side by side; read before the call returns.  Other batches and vocabularies: NI_ERR_UNSUPPORTED_SIZE.
+NI_EXPORT int ni_sample_values(const float* logits, int* out, const char* words, int n_rows, int vocab, cudaStream_t stream) {
+    if (n_rows <= 0) return NI_OK;
+    if (vocab <= 0) return NI_ERR_BAD_ARGUMENT;
+    if (n_rows > SC_VALUE_ROWS || !sc_takes(vocab)) return NI_ERR_UNSUPPORTED_SIZE;
+    ScValues v;
+    memset(&v, 0, sizeof(v));
+    const auto take = [&](void* dst, size_t size) { memcpy(dst, words, size * n_rows); words += size * n_rows; };
+    take(v.seeds, 8); take(v.counters, 8); take(v.temperatures, 4); take(v.top_ps, 4); take(v.top_ks, 4);
+    return sc_launch(logits, out, v, n_rows, vocab, stream);
+}
+
 NI_EXPORT int ni_sample(const float* logits, int* out, const float* temperatures, const int* top_ks,
                         const float* top_ps, const unsigned long long* seeds,
                         const unsigned long long* counters, int n_rows, int vocab, cudaStream_t stream) {
     if (n_rows <= 0) return NI_OK;
     if (vocab <= 0) return NI_ERR_BAD_ARGUMENT;
     if (vocab > (1 << 25)) return NI_ERR_UNSUPPORTED_SIZE;  // fixed-point mass would overflow
-    // a cluster per row while a block's slice of the vocabulary fits its shared memory
-    const int slice = (((vocab + SC_RANKS - 1) / SC_RANKS) + 31) & ~31;
-    if (sample_by_cluster && vocab >= 4096 && slice <= SC_MAX_SLICE) {
-        const size_t sc_smem = (size_t)slice * sizeof(float) + (size_t)(SC_HISTS + 2 * SC_RANKS) * 256 * sizeof(unsigned long long);
-        static size_t sc_configured = 0;
-        if (sc_configured < sc_smem) {
-            cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_smem);
-            if (e != cudaSuccess) return (int)e;
-            sc_configured = sc_smem;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)n_rows * SC_RANKS);
-        cfg.blockDim = dim3(SC_THREADS);
-        cfg.dynamicSmemBytes = sc_smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = SC_RANKS;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits, out, temperatures, top_ks, top_ps, seeds,
-                                           counters, vocab, slice);
-        return e == cudaSuccess ? NI_OK : (int)e;
-    }
+    if (sc_takes(vocab))
+        return sc_launch(logits, out, ScArrays{temperatures, top_ks, top_ps, seeds, counters}, n_rows, vocab, stream);
     const size_t smem = (size_t)(SAMPLE_THREADS / 32) * 256 * sizeof(unsigned long long);
     static bool configured = false;
     if (!configured) {

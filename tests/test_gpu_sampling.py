@@ -215,3 +215,37 @@ def test_draws_follow_the_distribution_and_do_not_depend_on_the_batch():
     assert alone == got[17].item()
     mixed = sampler.sample(l[:3].to(DEV), [SamplingParams.greedy(), sp, SamplingParams(seed=9)], [0, 5, 9], [0, 17, 3])
     assert mixed[1].item() == alone and mixed[0].item() == 0
+
+
+@pytest.mark.parametrize("vocab", [4096, 4100, 6000, 16384, 16388, 50257, 128256])
+def test_candidates_of_rows_of_every_range(vocab):
+    """What the slices send as candidates of a row with top-k depends on the range of its logits: signed zeros, rows around
+    zero, rows of huge and of tiny spread, one far token, infinities, short last slices, slices of fewer than k tokens."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(vocab)
+    base = torch.randn(vocab, generator=g)
+    far, most, zeros = base.clone(), torch.full((vocab,), torch.finfo(torch.float32).min), torch.zeros(vocab)
+    far[vocab // 3] = 1e30
+    most[torch.randperm(vocab, generator=g)[:700]] = base[:700]
+    zeros[torch.randperm(vocab, generator=g)[:vocab // 2]] *= -1.0
+    zeros[torch.randperm(vocab, generator=g)[:30]] = base[:30]
+    last = base.clone()
+    last[-100:] += 40.0
+    inf = base.clone()
+    inf[5] = float("inf")
+    rows = [base, base * 1e-30, base * 1e30, base - 3.0, base * 0.1 - 1.0, far, most, zeros, last, -base.abs(), inf, base.round()]
+    l = torch.stack(rows).to(DEV)
+    n = len(rows)
+    seeds, counters = torch.arange(n, device=DEV) * 31 + 7, torch.arange(n, device=DEV)
+    temps = torch.full((n,), 0.9, device=DEV)
+    for k in (1, 50, 300, 504, 505):
+        for p in (1.0, 0.9):
+            outs = []
+            for cluster in (True, False):
+                ops.sample_by_cluster(cluster)
+                out = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+                ops.sample(l, out, temps, torch.full((n,), k, dtype=torch.int32, device=DEV), torch.full((n,), p, device=DEV), seeds, counters)
+                outs.append(out.tolist())
+            ops.sample_by_cluster(True)
+            assert outs[0] == outs[1], (k, p)
+
