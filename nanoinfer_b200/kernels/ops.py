@@ -182,6 +182,7 @@ _SIGNATURES = {
         "ni_argmax": [_P, _P, _I, _I, _P, _P],
         "ni_repetition_penalty": [_P, _P, _P, _I, _I, _I, _P],
         "ni_sample": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _P],
+        "ni_sample_values": [_P, _P, ctypes.c_char_p, _I, _I, _P],
         "ni_sample_set_cluster": [_I],
     },
 }
@@ -2093,6 +2094,22 @@ def sample(logits, out, temperatures, top_ks, top_ps, seeds, counters) -> None:
         _dev(temperatures, "temperatures", torch.float32), _dev(top_ks, "top_ks", torch.int32),
         _dev(top_ps, "top_ps", torch.float32), _dev(seeds, "seeds", torch.int64),
         _dev(counters, "counters", torch.int64), n, v, _stream()), "sample")
+
+
+SAMPLE_VALUE_ROWS = 64         # rows whose parameters can travel with the launch
+
+
+def sample_values(logits: torch.Tensor, out: torch.Tensor, words: bytes) -> bool:
+    """sample() for parameters that are on the host, packed as the kernel's launcher wants them (seeds, counters int64, temperatures,
+    top_ps float32, top_ks int32 of all rows).  False where it does not take the batch or the vocabulary: nothing was launched."""
+    n, v = logits.shape
+    if n > SAMPLE_VALUE_ROWS or len(words) != 28 * n or out.numel() != n:
+        return False
+    rc = load("sampling").ni_sample_values(_dev(logits, "logits", torch.float32), _dev(out, "out", torch.int32), words, n, v, _stream())
+    if rc == -2:
+        return False
+    _check(rc, "sample")
+    return True
 
 
 # ---- the fused decode step ---------------------------------------------------------------------------

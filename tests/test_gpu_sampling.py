@@ -249,3 +249,24 @@ def test_candidates_of_rows_of_every_range(vocab):
             ops.sample_by_cluster(True)
             assert outs[0] == outs[1], (k, p)
 
+
+@pytest.mark.parametrize("rows, vocab, taken", [(1, 4096, True), (64, 4096, True), (65, 4096, False), (3, 4095, False), (2, 400000, False)])
+def test_parameters_that_travel_with_the_launch(rows, vocab, taken):
+    """The same tokens whether a batch's parameters are arguments of the launch or arrays on the device."""
+    import struct
+    from nanoinfer_b200.kernels import ops
+    from nanoinfer_b200.sampling import Sampler, SamplingParams
+    g = torch.Generator().manual_seed(rows)
+    l = (torch.randn(rows, vocab, generator=g) * 3).to(DEV)
+    params = [SamplingParams(temperature=[0.7, 0.0, 1.3][r % 3], top_k=[-1, 20, 300][r % 3 if r % 2 else 0], top_p=[0.9, 1.0][r % 2]) for r in range(rows)]
+    seeds, at = [2 ** 63 + r for r in range(rows)], [5 * r for r in range(rows)]
+    words = struct.pack(f"<{rows}Q{rows}q{rows}f{rows}f{rows}i", *seeds, *at, *(p.temperature for p in params), *(p.top_p for p in params),
+                        *(p.top_k for p in params))
+    out, want = torch.full((rows,), -1, dtype=torch.int32, device=DEV), torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+    assert ops.sample_values(l, out, words) == taken
+    sampler = Sampler(vocab, torch.device(DEV))
+    s, c, t, p, k = sampler._upload(l.device, params, seeds, at)
+    ops.sample(l, want, t, k, p, s, c)
+    assert not taken or torch.equal(out, want)
+    assert torch.equal(sampler.sample(l, params, seeds, at), want)
+    assert sampler.h2d_bytes == 2 * 28 * rows
