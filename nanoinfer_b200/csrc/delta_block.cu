@@ -1,5 +1,6 @@
 // The gated delta rule with one decay per head over prompt portions, four tokens at a time, FP32 throughout (formula and
-// layouts of delta_rule.cu, which walks the tokens one by one).
+// layouts of delta_rule.cu, which walks the tokens one by one; longer portions of key heads of 128 go sixteen tokens at a time,
+// delta_tile.cu).
 //
 // A request's tokens are taken in blocks of four from its portion's start on.  With S the state before a block, P(t, s) the
 // product of the decays of tokens s + 1 .. t of the block and c_t that of tokens 0 .. t:

@@ -111,6 +111,9 @@ _SIGNATURES = {
     "delta_block": {
         "ni_delta_block": [_P, _I, _P, _P, _P, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P],
     },
+    "delta_tile": {
+        "ni_delta_tile": [_P, _I, _P, _P, _P, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
+    },
     "delta_chunk": {
         "ni_delta_chunk_recurrence": [_P, _I, _I, _P, _P, _P, _P, _I, _P, _LL, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _LL, _P, _P, _P],
         "ni_delta_chunk_set_wait": [_LL, _I],
@@ -731,10 +734,18 @@ def delta_block_pays(n_tokens: int, n_seqs: int, max_q_len: int, n_heads: int, d
         (n_tokens >= 8 * n_seqs and (max_q_len >= 26 or n_seqs * size >= full))
 
 
+def delta_tile_pays(n_tokens: int, n_seqs: int, dim: int, vdim: int) -> bool:
+    """Whether delta_block_recurrence takes sixteen tokens at a time (csrc/delta_tile.cu: key heads of 128, value heads a multiple of
+    16): a request costs whole tiles however few its tokens are.  us in blocks of four / in tiles, 16 heads of 128: a portion of 64
+    21.9 / 22.2, four of 32 22.1 / 22.6, three of 100 42.2 / 37.3, 32 of 16 59.2 / 51.5, 16 of 8 27.5 / 32.0; 256 beside 64 single tokens 87 /
+    105, 512 beside 200 207 / 282, 1,024 beside 200 296 / 308."""
+    return dim == 128 and vdim % 16 == 0 and n_tokens >= 192 and n_tokens >= 16 * n_seqs
+
+
 def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
-                           vdim, taps, out) -> None:
+                           vdim, taps, out, tiles: Optional[bool] = None) -> None:
     """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another
-    order of sums): ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the
+    order of sums) or sixteen (``tiles``; None: where delta_tile_pays; FP32 numbers cut in three for the tensor cores): ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the
     decay at ``b_col`` and ``a_col``.  delta_gated_norm must follow (it moves the convolution history on)."""
     f32, i32 = torch.float32, torch.int32
     n = proj.shape[0]
@@ -743,6 +754,22 @@ def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, sta
             proj.shape[1] < max(col0 + c, b_col + n_heads, a_col + n_heads) or min(b_col, a_col) < col0 or \
             state.shape[1] != n_heads * dim * vdim + (taps - 1) * c or cu_q.numel() != n_seqs + 1 or slots.numel() != n_seqs:
         raise KernelError("delta_block_recurrence: shapes do not agree")
+    if delta_tile_pays(n, n_seqs, dim, vdim) if tiles is None else tiles:
+        if dim != 128:
+            raise KernelError("delta_block_recurrence: sixteen tokens at a time are for key heads of 128")
+        lib = load("delta_tile")
+        sizes = []
+        for name, args in (("values", (n, n_heads, vdim)), ("keys", (n, n_seqs, n_q_heads_kv)), ("coefs", (n, n_seqs, n_heads))):
+            f = getattr(lib, "ni_delta_tile_" + name)
+            f.restype, f.argtypes = _LL, [_I] * 3
+            sizes.append(f(*args))
+        values, keys, coef = (torch.empty(b, dtype=torch.uint8, device=proj.device) for b in sizes)
+        _check(lib.ni_delta_tile(
+            _dev(proj, "proj") + col0 * proj.element_size(), _code(proj, "proj"), _dev(conv_w, "conv_w", f32), _dev(a_log, "a_log", f32),
+            _dev(dt_bias, "dt_bias", f32), _dev(state, "state", f32), state.shape[1], _dev(cu_q, "cu_q", i32), _dev(slots, "slots", i32), n,
+            n_seqs, n_q_heads_kv, n_heads, vdim, taps, proj.shape[1], b_col - col0, a_col - col0, values.data_ptr(), keys.data_ptr(),
+            coef.data_ptr(), _dev(out, "out", f32), _stream()), "delta_block_recurrence")
+        return
     qkv = torch.empty(n, c, dtype=f32, device=proj.device)
     lib = load("delta_block")
     lib.ni_delta_block_coefs.restype, lib.ni_delta_block_coefs.argtypes = _LL, [_I] * 3

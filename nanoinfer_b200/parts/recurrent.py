@@ -33,8 +33,8 @@ class GatedDeltaRule(Part):
     second, block-diagonal product turns (W_a1 x, W_g1 x) into the logits of decay and gate in FP32.  Everything from there
     to the gated norm is FP32 on the device; in bfloat16 a step of single tokens with both options is one launch (from an
     FP32 projection, thin products included), and portions of CHUNK_FROM tokens and more run in chunks on the tensor cores
-    (csrc/delta_chunk.cu); with a decay per head steps of long portions run by blocks of four tokens (csrc/delta_block.cu,
-    ops.delta_block_pays).  A request's state is one FP32 vector: M of every head, then the last
+    (csrc/delta_chunk.cu); with a decay per head steps of long portions run by blocks of four or tiles of sixteen tokens
+    (csrc/delta_block.cu, csrc/delta_tile.cu, ops.delta_block_pays, ops.delta_tile_pays).  A request's state is one FP32 vector: M of every head, then the last
     conv_taps - 1 inputs of every convolved channel.  A step's kernels run exactly once, so the state advances by exactly
     the step's tokens.
 
@@ -158,7 +158,7 @@ class GatedDeltaRule(Part):
         if self.chunked:
             self.kernel_modules = ("delta_chunk",)
         if self.in_blocks:
-            self.kernel_modules = ("delta_block",)
+            self.kernel_modules = ("delta_block", "delta_tile")
 
     def cache_need(self):
         return StateNeed((self.H * self.D * self.V + (self.taps - 1) * self.channels,), "float32")

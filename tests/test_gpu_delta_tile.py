@@ -1,0 +1,101 @@
+"""The gated delta rule sixteen tokens at a time against the kernel that walks the tokens one by one and against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _inputs(G, H, V, taps, lens, fast, seed, dtype=torch.float32, col0=0):
+    g = torch.Generator().manual_seed(seed)
+    C = 2 * G * 128 + H * V
+    b_col = col0 + C + 4
+    a_col = b_col + H
+    N = -(-(b_col + 2 * H) // 4) * 4
+    i32 = dict(dtype=torch.int32, device=DEV)
+    return dict(G=G, H=H, V=V, taps=taps, C=C, b_col=b_col, a_col=a_col, col0=col0, n=sum(lens), n_seqs=len(lens),
+                proj=torch.randn(sum(lens), N, generator=g).to(DEV, dtype), conv_w=(torch.randn(C, taps, generator=g) * 0.6).to(DEV),
+                a_log=(torch.randn(H, generator=g) + fast).to(DEV), dt_bias=torch.randn(H, generator=g).to(DEV),
+                cu=torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), **i32), slots=torch.randperm(len(lens) + 3, generator=g)[:len(lens)].int().to(DEV),
+                seq=torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().to(DEV),
+                state=torch.randn(len(lens) + 3, H * 128 * V + (taps - 1) * C, generator=g).to(DEV) * 0.2)
+
+
+def _tiles(ops, x, tiles=True):
+    state, out = x["state"].clone(), torch.full((x["n"], x["H"] * x["V"]), float("nan"), device=DEV)
+    ops.delta_block_recurrence(x["proj"], x["col0"], x["b_col"], x["a_col"], x["conv_w"], x["a_log"], x["dt_bias"], state, x["cu"], x["slots"],
+                               x["n_seqs"], x["G"], x["H"], 128, x["V"], x["taps"], out, tiles=tiles)
+    return out, state
+
+
+def _tokens(ops, x):
+    state, out = x["state"].clone(), torch.empty(x["n"], x["H"] * x["V"], device=DEV)
+    qkv, gates = torch.empty(x["n"], x["C"], device=DEV), torch.empty(x["n"], x["H"], 2, device=DEV)
+    ops.delta_prepare(x["proj"], x["conv_w"], x["a_log"], x["dt_bias"], state, x["seq"], x["cu"], x["slots"], x["n_seqs"], x["G"], x["H"], 128,
+                      x["V"], x["taps"], qkv, gates, col0=x["col0"], b_col=x["b_col"])
+    ops.delta_recurrence(qkv, gates, state, x["cu"], x["slots"], x["n_seqs"], x["G"], x["H"], 128, x["V"], out)
+    return out, state, qkv, gates
+
+
+@pytest.mark.parametrize("G, H, V, taps, fast", [(1, 1, 128, 4, -2.0), (2, 6, 48, 4, -2.0), (4, 4, 32, 1, 4.0), (1, 3, 16, 6, 4.0), (2, 2, 80, 3, -6.0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_portions_of_every_length(G, H, V, taps, fast, dtype):
+    """Portions around multiples of sixteen, shorter than the convolution's history, none at all, slots out of order; decays
+    that reach zero within a tile and that hardly forget."""
+    from nanoinfer_b200.kernels import ops
+    x = _inputs(G, H, V, taps, [17, 1, 0, 67, 2, 16, 31, 33, 130, 15], fast, G + 10 * H + V, dtype)
+    out, state = _tiles(ops, x)
+    want, want_state, _, _ = _tokens(ops, x)
+    # sums of 128 terms in another order, carried along at most 130 tokens whose state neither rule lets grow
+    torch.testing.assert_close(out, want, rtol=2e-5, atol=2e-5 * want.abs().max().item())
+    torch.testing.assert_close(state, want_state, rtol=2e-5, atol=2e-5 * want_state.abs().max().item())
+    others = torch.ones(state.shape[0], dtype=torch.bool)
+    others[x["slots"].long().cpu()] = False
+    assert torch.equal(state[others], x["state"][others])
+
+
+def _in_64_bits(x):
+    G, H, V, taps, C, cu = x["G"], x["H"], x["V"], x["taps"], x["C"], x["cu"].tolist()
+    proj, want, ends = x["proj"].double(), [], []
+    decay = torch.exp(-torch.exp(x["a_log"].double()) * torch.nn.functional.softplus(proj[:, x["a_col"]:x["a_col"] + H] + x["dt_bias"].double()))
+    beta = torch.sigmoid(proj[:, x["b_col"]:x["b_col"] + H])
+    for r in range(x["n_seqs"]):
+        kept = x["state"][x["slots"][r].long()].double()
+        s, L = kept[:H * 128 * V].view(H, 128, V).clone(), cu[r + 1] - cu[r]
+        rows = torch.cat([kept[H * 128 * V:].view(taps - 1, C), proj[cu[r]:cu[r + 1], x["col0"]:x["col0"] + C]])
+        y = torch.nn.functional.silu(sum(rows[i:i + L] * x["conv_w"][:, i].double() for i in range(taps)))
+        q, k = (z / torch.sqrt((z * z).sum(-1, keepdim=True) + 1e-6) for z in (y[:, :G * 128].view(L, G, 128), y[:, G * 128:2 * G * 128].view(L, G, 128)))
+        q, k, v = q.repeat_interleave(H // G, 1) * 128 ** -0.5, k.repeat_interleave(H // G, 1), y[:, 2 * G * 128:].view(L, H, V)
+        for t in range(L):
+            s = s * decay[cu[r] + t][:, None, None]
+            s = s + k[t][:, :, None] * (beta[cu[r] + t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], s)))[:, None, :]
+            want.append(torch.einsum("hd,hdv->hv", q[t], s).reshape(-1))
+        ends.append(s.reshape(-1))
+    return torch.stack(want), torch.stack(ends)
+
+
+@pytest.mark.parametrize("fast", [-4.0, -1.0, 2.0])
+def test_errors_against_64_bits_stay_where_they_were(fast):
+    """Read-outs and states no further from 64 bits than in blocks of four, but for what differs from input to input: the last states
+    are those of 12 heads, whose errors have a spread of a tenth or two of their mean."""
+    from nanoinfer_b200.kernels import ops
+    x = _inputs(4, 4, 64, 4, [200, 130, 70], fast, 5)
+    want, ends = _in_64_bits(x)
+    errors = []
+    for tiles in (True, False):
+        out, state = _tiles(ops, x, tiles)
+        end = state[x["slots"].long(), :4 * 128 * 64].double()
+        errors.append((((out - want).norm() / want.norm()).item(), ((end - ends).norm() / ends.norm()).item()))
+    assert all(a <= 1.25 * b for a, b in zip(*errors)), errors
+
+
+def test_refused_and_chosen():
+    from nanoinfer_b200.kernels import ops
+    x = _inputs(1, 1, 20, 4, [200], -2.0, 6)
+    with pytest.raises(ops.KernelError):
+        _tiles(ops, x)                                       # value heads of 20
+    out, _ = _tiles(ops, x, tiles=None)                      # ... go in blocks of four
+    torch.testing.assert_close(out, _tokens(ops, x)[0], rtol=2e-5, atol=2e-5 * out.abs().max().item())
+    x = _inputs(1, 2, 32, 4, [200], -2.0, 7, torch.bfloat16, col0=3)
+    assert ops.delta_tile_pays(200, 1, 128, 32)
+    assert torch.equal(_tiles(ops, x)[0], _tiles(ops, x, tiles=None)[0])

@@ -131,3 +131,11 @@ def test_blocks_that_only_ask_for_weights_hold_nobody_up(cluster):
         assert number(items - 1, n_kv - 1, splits - 1) == own - 1 and number(0, 0, splits) == own
         assert items * n_kv * (splits + more) <= 3 * sms < items * n_kv * (splits + more + (splits if cluster else 1))
     assert some > 20
+
+
+@pytest.mark.parametrize("dim, vdim, lens, tiles", [
+    (128, 128, [64], False), (128, 128, [32] * 4, False), (128, 128, [100] * 3, True), (128, 128, [16] * 32, True), (128, 128, [8] * 16, False),
+    (128, 128, [256] + [1] * 64, False), (128, 128, [512] + [1] * 200, False), (128, 128, [1201, 847], True), (128, 48, [300], True),
+    (128, 20, [300], False), (64, 128, [300], False), (256, 128, [300], False)])
+def test_the_delta_rule_goes_by_tiles_where_they_are_done_first(dim, vdim, lens, tiles):
+    assert ops.delta_tile_pays(sum(lens), len(lens), dim, vdim) == tiles
