@@ -15,14 +15,16 @@
 // The state lies transposed in the warps' accumulator layout, 16 columns of v by 64 of the 128 rows: read as the first operand of the
 // next product it needs no exchange.  k, q, T and A are cut by the preparation, once, and lie as the second operands are read: a
 // lane's numbers of a 16 x 8 piece side by side.  Two warps share 16 columns; they add their halves of R and Q S through shared
-// memory, one barrier per tile.  What bounds a portion is the chain of its tiles, about 3,050 clocks each: 1,010 instructions of a
+// memory, one barrier per tile.  What bounds a portion is the chain of its tiles, about 2,850 clocks each: 1,010 instructions of a
 // lone warp per scheduler, which issues nothing else for 8 clocks while one of its 162 MMAs enters the tensor core.  (Four warps per 16
-// columns: 148 us instead of 129, since their products come in the same phases; FP32 multiply-adds in the same tiles: 183 us.)
+// columns: 148 us instead of 129 at the time, since their products come in the same phases; FP32 multiply-adds in the same tiles: 183 us.)
 //
-// Portions of 1,201 and 847 tokens, 16 heads of 128: 182 us with the preparation (51), against 247 us in blocks of four; 2,048 tokens 267
-// (338), 8 x 512 268 (330), 512 75 (91).  Error against 64 bits of the whole rule, read-outs / states, means over six inputs: decays of a
+// Portions of 1,201 and 847 tokens, 16 heads of 128: 171 us with the preparation (51), against 247 us in blocks of four; 2,048 tokens 248
+// (338), 8 x 512 261 (330), 512 71 (91).  Error against 64 bits of the whole rule, read-outs / states, means over six inputs: decays of a
 // few tokens 1.3e-7 / 1.4e-7 (blocks of four 1.3e-7 / 1.3e-7), of some tens 1.7e-7 / 2.2e-7 (1.9e-7 / 2.7e-7), decays near one 1.1e-6 /
 // 2.0e-6 (1.1e-6 / 2.0e-6: the decays' own rounding).
+#include <type_traits>
+
 #include "common.cuh"
 
 #define DT_TOK 16
@@ -329,6 +331,37 @@ __device__ __forceinline__ DtPiece dt_piece(const uint8_t* pieces, int n_pieces,
     b.c = *reinterpret_cast<const uint2*>(pieces + n_pieces * 512 + piece * 256 + lane * 8);
     return b;
 }
+// Coefficient (t, s) of two pieces that hold T or A: the sum of its parts.
+__device__ __forceinline__ float dt_coefficient(const uint8_t* pieces, int t, int s) {
+    const DtPiece b = dt_piece(pieces, 2, t >> 3, 4 * (t & 7) + ((s & 7) >> 1));
+    const uint32_t p[3] = {s >> 3 ? b.ab.y : b.ab.x, s >> 3 ? b.ab.w : b.ab.z, s >> 3 ? b.c.y : b.c.x};
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 2; k >= 0; --k) sum += __uint_as_float((s & 1) ? p[k] & 0xffff0000u : p[k] << 16);
+    return sum;
+}
+// sum_{s<t} C_ts x_s without the tokens from t on, for the tokens and columns of this lane's numbers: what the tensor core makes of
+// infinities and NaN (its zeros times a later token's) is taken back this way.
+__device__ __noinline__ void dt_masked(const uint8_t* pieces, const float x[8], float y[8]) {
+    const int lane = threadIdx.x & 31, q4 = lane & 3;
+    float acc[8] = {};
+#pragma unroll
+    for (int s = 0; s < DT_TOK; ++s) {
+        const int src = (lane & ~3) + ((s & 7) >> 1);
+        const float a = __shfl_sync(0xffffffffu, x[4 * (s >> 3) + (s & 1)], src), b = __shfl_sync(0xffffffffu, x[4 * (s >> 3) + (s & 1) + 2], src);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 8 * (i >> 1) + 2 * q4 + (i & 1), at = 4 * (i >> 1) + (i & 1);
+            if (s < t) {
+                const float c = dt_coefficient(pieces, t, s);
+                acc[at] = fmaf(c, a, acc[at]);
+                acc[at + 2] = fmaf(c, b, acc[at + 2]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = acc[i];
+}
 #define DT_STAGES 2
 #define DT_VP 36               // row pitch of the values in shared memory
 #define DT_STAGE (DT_KEYS + DT_COEF + DT_TOK * DT_VP * 4)
@@ -366,175 +399,201 @@ delta_tile_recurrence_kernel(const float* __restrict__ values, const uint8_t* __
         asm volatile("cp.async.commit_group;" ::: "memory");   // one group per tile, empty or not
     };
     static_assert(DT_KEYS % 2048 == 0 && DT_COEF % 16 == 0, "whole pieces for every thread");
-    fetch(0);
 
     // state: accumulator i holds columns col, col + 8 by rows 64 half + 8 i + 2 q4, + 1
     const bool there = col0 + 16 * team < V;                   // V is a multiple of 16: all of a team's columns or none
     float* S = state + (size_t)slots[seq] * state_stride + ((size_t)h * DT_D + 64 * half + 2 * q4) * V + col;
     float s[8][4];
+    const auto walk = [&](auto masked) {
+        constexpr bool MASKED = decltype(masked)::value;
+        fetch(0);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[i][e] = there ? S[(size_t)(8 * i + (e & 1)) * V + 8 * (e >> 1)] : 0.f;
+            for (int e = 0; e < 4; ++e) s[i][e] = there ? S[(size_t)(8 * i + (e & 1)) * V + 8 * (e >> 1)] : 0.f;
+        for (int tile = 0; tile < tiles; ++tile) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                                       // the tile is there; every warp has left the one before
+            fetch(tile + 1);
+            const uint8_t* st = dt_smem + (tile % DT_STAGES) * DT_STAGE;
+            const uint8_t* Tm = st + DT_KEYS;
+            const uint8_t* Am = Tm + 2 * DT_PIECE;
+            const float* vec = reinterpret_cast<const float*>(Tm + 4 * DT_PIECE);
+            const float* vs = reinterpret_cast<const float*>(st + DT_KEYS + DT_COEF) + 16 * team + row;
 
-    for (int tile = 0; tile < tiles; ++tile) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                       // the tile is there; every warp has left the one before
-        fetch(tile + 1);
-        const uint8_t* st = dt_smem + (tile % DT_STAGES) * DT_STAGE;
-        const uint8_t* Tm = st + DT_KEYS;
-        const uint8_t* Am = Tm + 2 * DT_PIECE;
-        const float* vec = reinterpret_cast<const float*>(Tm + 4 * DT_PIECE);
-        const float* vs = reinterpret_cast<const float*>(st + DT_KEYS + DT_COEF) + 16 * team + row;
-
-        // R^T and (Q S)^T, this half of the rows: [16 columns] x [tokens 8 j .. 8 j + 7]; j: k, k, q, q
-        float sum[4][4], small[4][4];
+            // R^T and (Q S)^T, this half of the rows: [16 columns] x [tokens 8 j .. 8 j + 7]; j: k, k, q, q
+            float sum[4][4], small[4][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            DtOperand a;
-            dt_operand(s[2 * i], s[2 * i + 1], a);
-            DtPiece b[4];
+            for (int i = 0; i < 4; ++i) {
+                DtOperand a;
+                dt_operand(s[2 * i], s[2 * i + 1], a);
+                DtPiece b[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = dt_piece(st + (j >> 1) * 16 * DT_PIECE, 16, 2 * (4 * half + i) + (j & 1), lane);
-            float big[4][4];
+                for (int j = 0; j < 4; ++j) b[j] = dt_piece(st + (j >> 1) * 16 * DT_PIECE, 16, 2 * (4 * half + i) + (j & 1), lane);
+                float big[4][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dt_mma_zero(big[j], a.p[0], b[j].ab.x, b[j].ab.y);
-            if (i == 0) {
+                for (int j = 0; j < 4; ++j) dt_mma_zero(big[j], a.p[0], b[j].ab.x, b[j].ab.y);
+                if (i == 0) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dt_mma_zero(small[j], a.p[0], b[j].c.x, b[j].c.y);
-            } else {
+                    for (int j = 0; j < 4; ++j) dt_mma_zero(small[j], a.p[0], b[j].c.x, b[j].c.y);
+                } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[0], b[j].c.x, b[j].c.y);
+                    for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[0], b[j].c.x, b[j].c.y);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[2], b[j].ab.x, b[j].ab.y);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[1], b[j].ab.z, b[j].ab.w);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[0], b[j].ab.z, b[j].ab.w);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[1], b[j].ab.x, b[j].ab.y);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[j][e] = i == 0 ? big[j][e] : sum[j][e] + big[j][e];
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[2], b[j].ab.x, b[j].ab.y);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[1], b[j].ab.z, b[j].ab.w);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[0], b[j].ab.z, b[j].ab.w);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) dt_mma(small[j], a.p[1], b[j].ab.x, b[j].ab.y);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) sum[j][e] = i == 0 ? big[j][e] : sum[j][e] + big[j][e];
-        }
+                for (int e = 0; e < 4; ++e) sum[j][e] += small[j][e];
+            exch[(3 * half) * 32 + lane] = make_float4(sum[0][0], sum[0][1], sum[0][2], sum[0][3]);
+            exch[(3 * half + 1) * 32 + lane] = make_float4(sum[1][0], sum[1][1], sum[1][2], sum[1][3]);
+            // the other warp writes the read-outs of tokens 8 (1 - half) ..
+            exch[(3 * half + 2) * 32 + lane] = half ? make_float4(sum[2][0], sum[2][1], sum[2][2], sum[2][3])
+                                                    : make_float4(sum[3][0], sum[3][1], sum[3][2], sum[3][3]);
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + team) : "memory");
+            float o[4], x[2][4];
+            {
+                const float4 y[3] = {exch[(3 * (1 - half)) * 32 + lane], exch[(3 * (1 - half) + 1) * 32 + lane], exch[(3 * (1 - half) + 2) * 32 + lane]};
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sum[j][e] += small[j][e];
-        exch[(3 * half) * 32 + lane] = make_float4(sum[0][0], sum[0][1], sum[0][2], sum[0][3]);
-        exch[(3 * half + 1) * 32 + lane] = make_float4(sum[1][0], sum[1][1], sum[1][2], sum[1][3]);
-        // the other warp writes the read-outs of tokens 8 (1 - half) ..
-        exch[(3 * half + 2) * 32 + lane] = half ? make_float4(sum[2][0], sum[2][1], sum[2][2], sum[2][3])
-                                                : make_float4(sum[3][0], sum[3][1], sum[3][2], sum[3][3]);
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + team) : "memory");
-        float o[4], x[2][4];
-        {
-            const float4 y[3] = {exch[(3 * (1 - half)) * 32 + lane], exch[(3 * (1 - half) + 1) * 32 + lane], exch[(3 * (1 - half) + 2) * 32 + lane]};
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {                      // X: tokens 8 j + 2 q4, + 1 of columns col, col + 8
-                const int t = 8 * j + 2 * q4;
-                const float2 be = *reinterpret_cast<const float2*>(vec + t), bc = *reinterpret_cast<const float2*>(vec + 16 + t);
-                x[j][0] = fmaf(-bc.x, sum[j][0] + y[j].x, be.x * vs[t * DT_VP]);
-                x[j][1] = fmaf(-bc.y, sum[j][1] + y[j].y, be.y * vs[(t + 1) * DT_VP]);
-                x[j][2] = fmaf(-bc.x, sum[j][2] + y[j].z, be.x * vs[t * DT_VP + 8]);
-                x[j][3] = fmaf(-bc.y, sum[j][3] + y[j].w, be.y * vs[(t + 1) * DT_VP + 8]);
+                for (int j = 0; j < 2; ++j) {                      // X: tokens 8 j + 2 q4, + 1 of columns col, col + 8
+                    const int t = 8 * j + 2 * q4;
+                    const float2 be = *reinterpret_cast<const float2*>(vec + t), bc = *reinterpret_cast<const float2*>(vec + 16 + t);
+                    x[j][0] = fmaf(-bc.x, sum[j][0] + y[j].x, be.x * vs[t * DT_VP]);
+                    x[j][1] = fmaf(-bc.y, sum[j][1] + y[j].y, be.y * vs[(t + 1) * DT_VP]);
+                    x[j][2] = fmaf(-bc.x, sum[j][2] + y[j].z, be.x * vs[t * DT_VP + 8]);
+                    x[j][3] = fmaf(-bc.y, sum[j][3] + y[j].w, be.y * vs[(t + 1) * DT_VP + 8]);
+                }
+                o[0] = (half ? sum[3][0] : sum[2][0]) + y[2].x; o[1] = (half ? sum[3][1] : sum[2][1]) + y[2].y;
+                o[2] = (half ? sum[3][2] : sum[2][2]) + y[2].z; o[3] = (half ? sum[3][3] : sum[2][3]) + y[2].w;
             }
-            o[0] = (half ? sum[3][0] : sum[2][0]) + y[2].x; o[1] = (half ? sum[3][1] : sum[2][1]) + y[2].y;
-            o[2] = (half ? sum[3][2] : sum[2][2]) + y[2].z; o[3] = (half ? sum[3][3] : sum[2][3]) + y[2].w;
-        }
-        // U^T = X^T + X^T (T - 1)^T, in both warps
-        float u[2][4];
-        {
-            DtOperand a;
-            dt_operand(x[0], x[1], a);
-            float d[2][4];
-            DtPiece b[2];
+            // U^T = X^T + X^T (T - 1)^T, in both warps
+            float u[2][4];
+            {
+                DtOperand a;
+                dt_operand(x[0], x[1], a);
+                float d[2][4];
+                DtPiece b[2];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                b[m] = dt_piece(Tm, 2, m, lane);
-                dt_mma_zero(u[m], a.p[0], b[m].ab.x, b[m].ab.y);
-                dt_mma_zero(d[m], a.p[0], b[m].c.x, b[m].c.y);
-            }
-#pragma unroll
-            for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[2], b[m].ab.x, b[m].ab.y);
-#pragma unroll
-            for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[1], b[m].ab.z, b[m].ab.w);
-#pragma unroll
-            for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[0], b[m].ab.z, b[m].ab.w);
-#pragma unroll
-            for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[1], b[m].ab.x, b[m].ab.y);
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) u[m][e] = x[m][e] + (u[m][e] + d[m][e]);
-        }
-        // read-outs of tokens 8 half ..: c (Q S) + A U, what FP32 adds to them first
-        {
-            const float2 c = *reinterpret_cast<const float2*>(vec + 32 + 8 * half + 2 * q4), own = *reinterpret_cast<const float2*>(vec + 64 + 8 * half + 2 * q4);
-            o[0] = fmaf(c.x, o[0], own.x * (half ? u[1][0] : u[0][0])); o[1] = fmaf(c.y, o[1], own.y * (half ? u[1][1] : u[0][1]));
-            o[2] = fmaf(c.x, o[2], own.x * (half ? u[1][2] : u[0][2])); o[3] = fmaf(c.y, o[3], own.y * (half ? u[1][3] : u[0][3]));
-        }
-        // S^T <- c_15 S^T + (U P(15, .))^T K
-        {
-            float w[2][4];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const float2 tail = *reinterpret_cast<const float2*>(vec + 48 + 8 * j + 2 * q4);
-                w[j][0] = u[j][0] * tail.x; w[j][1] = u[j][1] * tail.y; w[j][2] = u[j][2] * tail.x; w[j][3] = u[j][3] * tail.y;
-            }
-            DtOperand a;
-            dt_operand(w[0], w[1], a);
-            const float all = vec[32 + 15];
-#pragma unroll
-            for (int i0 = 0; i0 < 8; i0 += 4) {
-                DtPiece b[4];
-                float big[4][4], d[4][4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    b[i] = dt_piece(st + 32 * DT_PIECE, 16, 8 * half + i0 + i, lane);
-                    dt_mma_zero(big[i], a.p[0], b[i].ab.x, b[i].ab.y);
-                    dt_mma_zero(d[i], a.p[0], b[i].c.x, b[i].c.y);
+                for (int m = 0; m < 2; ++m) {
+                    b[m] = dt_piece(Tm, 2, m, lane);
+                    dt_mma_zero(u[m], a.p[0], b[m].ab.x, b[m].ab.y);
+                    dt_mma_zero(d[m], a.p[0], b[m].c.x, b[m].c.y);
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[2], b[i].ab.x, b[i].ab.y);
+                for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[2], b[m].ab.x, b[m].ab.y);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[1], b[i].ab.z, b[i].ab.w);
+                for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[1], b[m].ab.z, b[m].ab.w);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[0], b[i].ab.z, b[i].ab.w);
+                for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[0], b[m].ab.z, b[m].ab.w);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[1], b[i].ab.x, b[i].ab.y);
+                for (int m = 0; m < 2; ++m) dt_mma(d[m], a.p[1], b[m].ab.x, b[m].ab.y);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int m = 0; m < 2; ++m)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) s[i0 + i][e] = fmaf(all, s[i0 + i][e], big[i][e] + d[i][e]);
+                    for (int e = 0; e < 4; ++e) u[m][e] = x[m][e] + (u[m][e] + d[m][e]);
+            }
+            float later[4] = {0.f, 0.f, 0.f, 0.f};                 // what A U is without the tensor core
+            if (MASKED) {
+                float in[8], sums[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) in[i] = x[i >> 2][i & 3];
+                dt_masked(Tm, in, sums);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) in[i] = u[i >> 2][i & 3] = x[i >> 2][i & 3] + sums[i];
+                dt_masked(Am, in, sums);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) later[e] = half ? sums[4 + e] : sums[e];
+            }
+            // read-outs of tokens 8 half ..: c (Q S) + A U, what FP32 adds to them first
+            {
+                const float2 c = *reinterpret_cast<const float2*>(vec + 32 + 8 * half + 2 * q4), own = *reinterpret_cast<const float2*>(vec + 64 + 8 * half + 2 * q4);
+                o[0] = fmaf(c.x, o[0], own.x * (half ? u[1][0] : u[0][0])); o[1] = fmaf(c.y, o[1], own.y * (half ? u[1][1] : u[0][1]));
+                o[2] = fmaf(c.x, o[2], own.x * (half ? u[1][2] : u[0][2])); o[3] = fmaf(c.y, o[3], own.y * (half ? u[1][3] : u[0][3]));
+            }
+            // S^T <- c_15 S^T + (U P(15, .))^T K
+            {
+                float w[2][4];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float2 tail = *reinterpret_cast<const float2*>(vec + 48 + 8 * j + 2 * q4);
+                    w[j][0] = u[j][0] * tail.x; w[j][1] = u[j][1] * tail.y; w[j][2] = u[j][2] * tail.x; w[j][3] = u[j][3] * tail.y;
+                }
+                DtOperand a;
+                dt_operand(w[0], w[1], a);
+                const float all = vec[32 + 15];
+#pragma unroll
+                for (int i0 = 0; i0 < 8; i0 += 4) {
+                    DtPiece b[4];
+                    float big[4][4], d[4][4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        b[i] = dt_piece(st + 32 * DT_PIECE, 16, 8 * half + i0 + i, lane);
+                        dt_mma_zero(big[i], a.p[0], b[i].ab.x, b[i].ab.y);
+                        dt_mma_zero(d[i], a.p[0], b[i].c.x, b[i].c.y);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[2], b[i].ab.x, b[i].ab.y);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[1], b[i].ab.z, b[i].ab.w);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[0], b[i].ab.z, b[i].ab.w);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dt_mma(d[i], a.p[1], b[i].ab.x, b[i].ab.y);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) s[i0 + i][e] = fmaf(all, s[i0 + i][e], big[i][e] + d[i][e]);
+                }
+            }
+            // ... and A U
+            {
+                DtOperand a;
+                dt_operand(u[0], u[1], a);
+                const DtPiece b = dt_piece(Am, 2, half, lane);
+                float big[4], d[4];
+                dt_mma_zero(big, a.p[0], b.ab.x, b.ab.y);
+                dt_mma_zero(d, a.p[0], b.c.x, b.c.y);
+                dt_mma(d, a.p[2], b.ab.x, b.ab.y);
+                dt_mma(d, a.p[1], b.ab.z, b.ab.w);
+                dt_mma(d, a.p[0], b.ab.z, b.ab.w);
+                dt_mma(d, a.p[1], b.ab.x, b.ab.y);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] += MASKED ? later[e] : big[e] + d[e];
+                const int t = 8 * half + 2 * q4, tok = tile * DT_TOK + t;
+                float* dst = out + (size_t)(first + tok) * dm.H * V + (size_t)h * V + col;
+                if (there && tok < n) {
+                    dst[0] = o[0];
+                    dst[8] = o[2];
+                }
+                if (there && tok + 1 < n) {
+                    dst[(size_t)dm.H * V] = o[1];
+                    dst[(size_t)dm.H * V + 8] = o[3];
+                }
             }
         }
-        // ... and A U
-        {
-            DtOperand a;
-            dt_operand(u[0], u[1], a);
-            const DtPiece b = dt_piece(Am, 2, half, lane);
-            float big[4], d[4];
-            dt_mma_zero(big, a.p[0], b.ab.x, b.ab.y);
-            dt_mma_zero(d, a.p[0], b.c.x, b.c.y);
-            dt_mma(d, a.p[2], b.ab.x, b.ab.y);
-            dt_mma(d, a.p[1], b.ab.z, b.ab.w);
-            dt_mma(d, a.p[0], b.ab.z, b.ab.w);
-            dt_mma(d, a.p[1], b.ab.x, b.ab.y);
-            const int t = 8 * half + 2 * q4, tok = tile * DT_TOK + t;
-            float* dst = out + (size_t)(first + tok) * dm.H * V + (size_t)h * V + col;
-            if (there && tok < n) {
-                dst[0] = o[0] + (big[0] + d[0]);
-                dst[8] = o[2] + (big[2] + d[2]);
-            }
-            if (there && tok + 1 < n) {
-                dst[(size_t)dm.H * V] = o[1] + (big[1] + d[1]);
-                dst[(size_t)dm.H * V + 8] = o[3] + (big[3] + d[3]);
-            }
-        }
-    }
+    };
+    walk(std::false_type{});
+    // An infinity or a NaN in U: the tensor core has given it (0 times it) to the tokens before its own in its tile, too.  It has reached
+    // the state's column as well, and stays there: then once more, T and A times nothing but earlier tokens.  (Looked for in every tile:
+    // 3 to 7 us of 131.)
+    float zero = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) zero += s[i][e] - s[i][e];
+    if (__syncthreads_or(zero != 0.f)) walk(std::true_type{});
     if (there) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)

@@ -99,3 +99,22 @@ def test_refused_and_chosen():
     x = _inputs(1, 2, 32, 4, [200], -2.0, 7, torch.bfloat16, col0=3)
     assert ops.delta_tile_pays(200, 1, 128, 32)
     assert torch.equal(_tiles(ops, x)[0], _tiles(ops, x, tiles=None)[0])
+
+
+@pytest.mark.parametrize("poison", [float("inf"), float("nan")])
+@pytest.mark.parametrize("what", ["value", "key", "query", "beta", "decay"])
+def test_what_is_not_finite_stays_with_its_own_and_later_tokens(poison, what):
+    """An infinity or a NaN in the middle of a tile: tokens before it, other requests and (a value) other columns as if it were not there."""
+    from nanoinfer_b200.kernels import ops
+    x = _inputs(2, 2, 32, 4, [45, 40], -2.0, 11)
+    clean, clean_state = _tiles(ops, x)
+    column = {"value": 2 * 2 * 128 + 32 + 5, "key": 2 * 128 + 128 + 7, "query": 128 + 3, "beta": x["b_col"] + 1, "decay": x["a_col"] + 1}[what]
+    x["proj"][22, column] = poison                            # head 1 of request 0
+    out, state = _tiles(ops, x)
+    hit = torch.zeros_like(clean, dtype=torch.bool)
+    hit[22:45, 32 + 5 if what == "value" else slice(32, 64)] = True
+    torch.testing.assert_close(out[~hit], clean[~hit], rtol=1e-6, atol=1e-6 * clean.abs().max().item())
+    want, want_state, _, _ = _tokens(ops, x)
+    keep = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(out)[~hit], keep[~hit]) and not torch.isfinite(out[~keep]).any()
+    torch.testing.assert_close(state[x["slots"][1].long()], clean_state[x["slots"][1].long()], rtol=0, atol=0)
