@@ -745,8 +745,9 @@ def delta_tile_pays(n_tokens: int, n_seqs: int, dim: int, vdim: int) -> bool:
 def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
                            vdim, taps, out, tiles: Optional[bool] = None) -> None:
     """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another
-    order of sums) or sixteen (``tiles``; None: where delta_tile_pays; FP32 numbers cut in three for the tensor cores): ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the
-    decay at ``b_col`` and ``a_col``.  delta_gated_norm must follow (it moves the convolution history on)."""
+    order of sums) or sixteen (``tiles``; None: where delta_tile_pays; FP32 numbers cut in three for the tensor cores):
+    ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the decay at ``b_col`` and
+    ``a_col``.  delta_gated_norm must follow (it moves the convolution history on)."""
     f32, i32 = torch.float32, torch.int32
     n = proj.shape[0]
     c = 2 * n_q_heads_kv * dim + n_heads * vdim
