@@ -1,35 +1,38 @@
 // out[M, N] = x[M, K] . w[N, K]^T of FP32 matrices with long rows on the fifth-generation tensor cores, with errors smaller than
-// those of a chain of FP32 multiply-adds.  Every FP32 number is cut in two: its upper 11 bits of mantissa (what the tensor core's
-// tf32 keeps of an operand) and what is left (13 bits, of which it keeps 11 again):
+// those of a chain of FP32 multiply-adds.  Every FP32 number is the sum of three bfloat16 numbers, each what is left rounded to nearest
+// (24 bits in all, so none is lost), and six of the nine products of parts are taken:
 //
-//     x w = xh wh + (xh wl + xl wh)  [+ xl wl, 2^-22 of x w and left out; xh is rounded, wh cut, so its mean is zero]
+//     x w = xa wa + (xa wb + xb wa + xb wb + xa wc + xc wa)     [+ xb wc + xc wb + xc wc: 2^-23 of x w at most, 2^-25 in the mean square]
 //
-// The tensor core adds into its FP32 accumulator by cutting, a bias that grows with the number of additions (-1.3e-7 after 32
-// columns, -2.9e-7 after 64).  So the accumulator of the large products (xh wh) is emptied every 64 columns into registers, where it
-// is added with rounding to nearest, and the small ones, 2^-11 of the large, have an accumulator of their own that is emptied every
-// 256:
+// The tensor core adds into its FP32 accumulator by cutting, a bias that grows with the number of additions.  So the accumulator of the
+// large products (xa wa) is emptied every 64 columns into registers, where it is added with rounding to nearest, and the small ones,
+// 2^-8 of the large, have an accumulator of their own that is emptied every 256:
 //     slice s of 256:  sum_s = (((hh_0 + hh_1) + hh_2) + hh_3) + small          result = (sum_0 + sum_1) + ...
 // This order is the same for every tile size, number of rows and split of K, so an element's bits depend on its two rows alone.
-// Relative error against 64 bits, normal (positive) numbers: 3.0e-7 (3.7e-7) at 1,024 columns where the chain has 5.7e-7 (4.9e-7),
-// 3.1e-7 (3.6e-7) at 8,192 where it has 1.6e-6 (1.3e-6).
+// Relative error against 64 bits, here / of the chain: normal numbers 0.9e-7 / 5.7e-7 at 1,024 columns, 1.3e-7 / 1.6e-6 at 8,192;
+// positive ones 0.9e-7 / 4.9e-7 and 1.2e-7 / 1.4e-6; rows of ten terms 0.56e-7 / 0.65e-7, of one 2.6e-8 / 2.5e-8; a number that meets
+// ones and zeros comes back bit for bit.  (Two tf32 parts and three products, which lose two of the 24 bits: 3.0e-7 and 3.7e-7,
+// rows of ten terms 1.8e-7, of one 1.7e-7.)
 //
-// What bounds it: at many rows the cutting and the MMAs' reads of shared memory (2,048 x 16,384 weights and 1,087 rows: 418 us, 175
-// TFLOP/s; chains on CUDA cores 1,417); at few the weights, [128256, 2048] 174 us (6.0 TB/s; the ring of chains 177, at 8 rows 239),
-// and for small matrices the way of one block: 6 us of start, first load and last sum, 0.65 us for 64 columns ([2048, 2048] 12.4 us
-// alone, less behind a kernel that lets it start early).
+// What bounds it: at many rows shared memory (the boxes, the parts of x and the MMAs' reads of them) and the cutting: 1,087 rows and
+// [16384, 2048] 416 us (175 TFLOP/s; two tf32 parts 418, chains on CUDA cores 1,417), 177 rows 107 (116); at few the weights,
+// [128256, 2048] 174 us (6.0 TB/s; 174; the ring of chains 177, at 8 rows 239), and for small matrices the way of one block: 6 us
+// of start, first load and last sum, 0.7 us for 64 columns ([2048, 2048] 13.0 us alone (12.1), less behind a kernel that lets it start
+// early).
 //
 // The 128 lanes of the tcgen05 tile are weight rows, its columns BT rows of x (16 .. 128): few rows read the weights once, at
 // many rows 128 x 128 tiles.  Blocks are persistent; a block's warps:
-//   0 - ..  cut: GROUPS groups take turns at the stages of 32 columns that TMA has filled: the numbers stay where they are (the
-//           tensor core ignores the bits that it does not keep), what is left goes beside them.  Those of x lie so that xh and
-//           xl, or xl and xh, are 2 BT rows of one operand
-//   then    empty the accumulators, 4 or 8 warps
+//   0 - ..  cut: GROUPS groups of four take turns at the boxes of 32 columns that TMA has filled.  The weights' parts go to tensor memory,
+//           from where the MMAs read them (in shared memory they are written and read five times by MMAs of few columns: 230 us for
+//           the vocabulary); those of x to shared memory, so that xa and xb, or xb and xa, are 2 BT rows of one operand
+//   then    empty the accumulators, 4 to 16 warps
 //   last    two: the MMAs, and TMA
 // A product with few weight rows cuts the slices of K over the blocks of a cluster; their sums go to the block that owns the row
 // of x (through its shared memory, once all MMAs are done) and are added there in the order of the slices.
 //
-// An element that is not finite is computed once more as one chain of fused multiply-adds: inf - inf among the parts of an
-// infinite operand, or an overflow that only the order of these sums has, does not show.
+// A sum that is not finite, not below 2^100, or below 2^-80 (but no zero) is computed once more as one chain of fused multiply-adds:
+// inf - inf among the parts of an infinite operand, a part that rounds beyond FP32's range, or third parts that bfloat16 cannot hold
+// (of numbers below 2^-110), do not show.  Beside ordinary numbers such small ones lose 2^-133 at most.
 #include <cuda.h>
 
 #include <mutex>
@@ -37,7 +40,7 @@
 #include "common.cuh"
 
 #define GT_ROWS 128            // weight rows of a tile
-#define GT_HALF 32             // columns of a box in shared memory: 128 bytes
+#define GT_BOX 32              // columns of a box as TMA brings it: 128 bytes of FP32, 64 of a part
 #define GT_BK 64               // k-block: what the accumulator of large products adds up
 #define GT_SLICE 4             // k-blocks of a slice
 #define GT_ERR_LOAD 51
@@ -45,27 +48,25 @@
 #define GT_ERR_MMA 53
 #define GT_ERR_SUMS 54
 
-// RAW stages of SUB boxes of 32 columns as they are loaded, STAGES of cut ones (PLACE: the same stages, the rests beside the numbers);
-// GROUPS of GROUP cutting warps; ACC warps that empty accumulators; COLS of tensor memory (3 BT for the accumulators, the rest for
-// sums of slices)
+// RAW boxes as loaded; STAGES of cut ones, the weights' parts in tensor memory, those of x in shared memory; GROUPS of four cutting
+// warps; ACC warps that empty accumulators; HH accumulators of large products
 template <int BT> struct GtCfg;
-template <> struct GtCfg<16> { static constexpr int RAW = 4, STAGES = 2, SUB = 2, GROUPS = 2, GROUP = 8, ACC = 4, COLS = 256; static constexpr bool PLACE = false; };
-template <> struct GtCfg<32> { static constexpr int RAW = 3, STAGES = 2, SUB = 2, GROUPS = 2, GROUP = 8, ACC = 4, COLS = 512; static constexpr bool PLACE = false; };
-template <> struct GtCfg<64> { static constexpr int RAW = 4, STAGES = 4, SUB = 1, GROUPS = 4, GROUP = 2, ACC = 8, COLS = 512; static constexpr bool PLACE = true; };
-template <> struct GtCfg<128> { static constexpr int RAW = 3, STAGES = 3, SUB = 1, GROUPS = 3, GROUP = 4, ACC = 16, COLS = 512; static constexpr bool PLACE = true; };
+template <> struct GtCfg<16> { static constexpr int RAW = 11, STAGES = 4, GROUPS = 4, ACC = 4, HH = 2; };
+template <> struct GtCfg<32> { static constexpr int RAW = 9, STAGES = 4, GROUPS = 4, ACC = 4, HH = 2; };
+template <> struct GtCfg<64> { static constexpr int RAW = 6, STAGES = 4, GROUPS = 4, ACC = 8, HH = 1; };
+template <> struct GtCfg<128> { static constexpr int RAW = 4, STAGES = 2, GROUPS = 2, ACC = 16, HH = 1; };
 template <int BT> struct GtSizes {
     using C = GtCfg<BT>;
-    static constexpr int A = GT_ROWS * 128, B = BT * 128;                            // bytes of a box of weights and of x
-    // A loaded stage: weights, x.  A cut one: rests of the weights, per box of x numbers and rests.  In place: weights, their rests,
-    // per box of x room for both.
-    static constexpr int RAW_STAGE = C::SUB * (C::PLACE ? 2 * A + 2 * B : A + B), STAGE = C::SUB * (C::PLACE ? 2 * A + 2 * B : A + 2 * B);
-    static constexpr int RAW_X = C::SUB * (C::PLACE ? 2 * A : A), REST_A = C::PLACE ? C::SUB * A : 0, CUT_X = C::SUB * (C::PLACE ? 2 * A : A);
-    static constexpr int CUT_RING = C::PLACE ? 0 : C::RAW * RAW_STAGE;               // where the stages of cut numbers begin
-    static constexpr int RING = C::RAW * RAW_STAGE + (C::PLACE ? 0 : C::STAGES * STAGE), SMEM = 1024 + RING + 256;
-    static constexpr int REGIONS = C::COLS / BT - 3;                                 // sums of slices that a block can keep
-    static constexpr int CUT = C::GROUPS * C::GROUP, THREADS = (CUT + C::ACC + 2) * 32;
-    static_assert(C::GROUPS <= C::STAGES && C::RAW >= C::STAGES && (!C::PLACE || C::RAW == C::STAGES), "see the cutting warps' waits");
-    static_assert(SMEM <= 232448, "shared memory");
+    static constexpr int A = GT_ROWS * 128, B = BT * 128, BOX = A + B;               // bytes of a box of weights and of x
+    static constexpr int PART = BT * 64, XRING = C::RAW * BOX;                       // of a part of a box of x; where those begin
+    static constexpr int RING = XRING + C::STAGES * 3 * PART, SMEM = 1024 + RING + 512;
+    // tensor memory: accumulators (the first of large products, small ones, the other of large ones), sums of slices, weights
+    static constexpr int SUMS = (1 + C::HH) * BT, WSTAGE = 3 * GT_BOX / 2, WPARTS = 512 - C::STAGES * WSTAGE;
+    static constexpr int REGIONS = (WPARTS - SUMS) / BT;                             // sums of slices that a block can keep, but for its last
+    static constexpr int CUT = 4 * C::GROUPS, THREADS = (CUT + C::ACC + 2) * 32;
+    static_assert(C::GROUPS <= C::STAGES && C::RAW >= C::STAGES, "see the cutting warps' waits");
+    static_assert(REGIONS >= 1 && BOX % 1024 == 0 && PART % 1024 == 0, "the swizzle goes by the address");
+    static_assert((2 * C::RAW + 2 * C::STAGES + 6) * 8 <= 512 && SMEM <= 232448, "shared memory");
 };
 
 __device__ __forceinline__ uint32_t gt_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -130,24 +131,24 @@ __device__ __forceinline__ void gt_tma_3d(void* dst, const CUtensorMap* map, int
 }
 __device__ __forceinline__ void gt_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void gt_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ uint64_t gt_desc(const void* tile) {   // K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t gt_desc(const void* tile) {              // K-major, 64-byte swizzle, 8-row groups 512 bytes apart
     const uint32_t addr = gt_smem(tile);
     uint64_t d = 0;
     d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
     d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)(512 >> 4) << 32;
     d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
+    d |= (uint64_t)4 << 61;
     return d;
 }
-__host__ __device__ constexpr uint32_t gt_idesc(int n) {          // TF32 x TF32 -> FP32, M = 128, N = n
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(GT_ROWS >> 4) << 24);
+__host__ __device__ constexpr uint32_t gt_idesc(int n) {          // BF16 x BF16 -> FP32, M = 128, N = n
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(GT_ROWS >> 4) << 24);
 }
-__device__ __forceinline__ void gt_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void gt_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void gt_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
@@ -166,6 +167,9 @@ __device__ __forceinline__ void gt_st16(uint32_t taddr, const float* r) {
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n"
         ::"f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]),
           "f"(r[8]), "f"(r[9]), "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void gt_st4(uint32_t taddr, const uint4& a) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};\n" ::"r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void gt_pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void gt_cluster_sync() {
@@ -191,16 +195,22 @@ __device__ __forceinline__ GtPair gt_fma(GtPair a, GtPair b, GtPair c) {
     return r;
 }
 __device__ __forceinline__ GtPair gt_sub(GtPair a, GtPair b) { return gt_fma(b, gt_pair(-1.f, -1.f), a); }
-// Rounded to 11 bits of mantissa by Veltkamp's splitting (the larger part of v's two): t = (2^13 + 1) v, t - (t - v).  What is not
-// finite, or overflows in t, ends as NaN.
-__device__ __forceinline__ GtPair gt_rounded(GtPair v) {
-    const GtPair t = gt_fma(v, gt_pair(8192.f, 8192.f), v);
-    return gt_sub(t, gt_sub(t, v));
-}
-// What the tensor core does not keep of two numbers, where it cuts them.
-__device__ __forceinline__ GtPair gt_rest_of_cut(float a, float b) {
-    const float ca = __uint_as_float(__float_as_uint(a) & 0xffffe000u), cb = __uint_as_float(__float_as_uint(b) & 0xffffe000u);
-    return gt_sub(gt_pair(a, b), gt_pair(ca, cb));
+// The three parts of eight numbers, in pairs of bfloat16.  Each is what is left rounded to nearest, so that three hold all 24 bits.  What
+// is not finite, or rounds beyond bfloat16's range, has a NaN among its parts.
+__device__ __forceinline__ void gt_cut(const float4& a, const float4& b, uint4 part[3]) {
+    GtPair v[4] = {gt_pair(a.x, a.y), gt_pair(a.z, a.w), gt_pair(b.x, b.y), gt_pair(b.z, b.w)};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v[j]));
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h[j]) : "f"(hi), "f"(lo));
+            if (i < 2) v[j] = gt_sub(v[j], gt_pair(__uint_as_float(h[j] << 16), __uint_as_float(h[j] & 0xffff0000u)));
+        }
+        part[i] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
 }
 // Four columns of a row in global memory, one by one (zeros beyond K): rows that TMA does not take.
 __device__ __forceinline__ float4 gt_load4(const float* __restrict__ p, int k, int K, bool live) {
@@ -212,19 +222,43 @@ __device__ __forceinline__ float4 gt_load4(const float* __restrict__ p, int k, i
     return v;
 }
 
-// A sum that is not finite, as one chain (NaN stays NaN, so the chain may end there).
-__device__ __forceinline__ float gt_chain(const float* __restrict__ x, const float* __restrict__ w, int K) {
-    float a = 0.f;
-    for (int k = 0; k < K && a == a; ++k) a = fmaf(x[k], w[k], a);
-    return a;
+// Whether a sum stands as it is: zero, or from 2^-80 to 2^100.
+__device__ __forceinline__ bool gt_stands(float v) {
+    const uint32_t magnitude = __float_as_uint(v) & 0x7fffffffu;
+    return magnitude == 0u || magnitude - (47u << 23) < (180u << 23);
 }
-__device__ __forceinline__ bool gt_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+// Up to four sums of one weight row (out, ldo apart) as chains where they do not stand.  VEC: rows lie on 16 bytes, K is a multiple of 4.
+// (Number by number, with one sum at a time: 143 ms for 1,087 rows of infinities and [16384, 2048].)
+template <bool VEC>
+__device__ __forceinline__ void gt_chains(const float* __restrict__ x, int ldx, int rows, const float* __restrict__ w, int K, float* out, int ldo) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int k = 0; k < K; k += 4) {
+        float xs[4][4], ws[4];
+        auto load = [&](const float* from, float v[4]) {
+            const float4 q = VEC ? *reinterpret_cast<const float4*>(from + k) : gt_load4(from, k, K, true);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        };
+        load(w, ws);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load(x + (size_t)(i < rows ? i : 0) * ldx, xs[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (VEC || k + j < K) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = fmaf(xs[i][j], ws[j], a[i]);
+            }
+        if (a[0] != a[0] && a[1] != a[1] && a[2] != a[2] && a[3] != a[3]) break;         // NaN stays NaN
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (i < rows && !gt_stands(out[(size_t)i * ldo])) out[(size_t)i * ldo] = a[i];
+}
 
 struct GtParams {
     const float* x;
     const float* w;
     float* out;
-    int M, N, K, H, ldx, ldo, splits;
+    int M, N, K, H, ldx, ldo, splits, early;
     int* error;
 };
 
@@ -245,16 +279,17 @@ template <int BT, bool TMA>
 __global__ void __launch_bounds__(GtSizes<BT>::THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GtParams p) {
     using S = GtSizes<BT>;
-    constexpr int RAW = GtCfg<BT>::RAW, STAGES = GtCfg<BT>::STAGES, GROUPS = GtCfg<BT>::GROUPS, ACC = GtCfg<BT>::ACC;
-    constexpr int SUB = GtCfg<BT>::SUB, P = GT_BK / GT_HALF / SUB;                           // stages of a k-block
+    using C = GtCfg<BT>;
+    constexpr int RAW = C::RAW, STAGES = C::STAGES, GROUPS = C::GROUPS, ACC = C::ACC, HH = C::HH;
+    constexpr int P = GT_BK / GT_BOX;                                                        // boxes of a k-block
     constexpr int CPT = BT * 4 / ACC;                                                        // columns of an emptying thread
     extern __shared__ uint8_t gt_smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>(((uintptr_t)gt_smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* loaded = reinterpret_cast<uint64_t*>(ring + S::RING);
-    uint64_t* full = loaded + RAW;
+    uint64_t* raw_empty = loaded + RAW;
+    uint64_t* full = raw_empty + RAW;
     uint64_t* empty = full + STAGES;
-    uint64_t* raw_empty = GtCfg<BT>::PLACE ? empty : empty + STAGES;
-    uint64_t* hh_full = raw_empty + RAW;
+    uint64_t* hh_full = empty + STAGES;
     uint64_t* hh_empty = hh_full + 2;
     uint64_t* small_empty = hh_empty + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(small_empty + 1);
@@ -267,109 +302,109 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int n_units = ((p.M + BT - 1) / BT) * ((p.N + GT_ROWS - 1) / GT_ROWS) * p.H;
     const int unit0 = blockIdx.x / splits, step = gridDim.x / splits;                        // (split: one unit per cluster)
 
-    const int steps = (b1 - b0) * P;                                                         // stages of a unit
+    const int steps = (b1 - b0) * P;                                                         // boxes of a unit
     auto tma_load = [&](int i, int n0, int m0, int head, int k, bool weights, bool x) {
-        const int rs = i % RAW, buf = i / P & 1;
-        uint8_t* a = ring + rs * S::RAW_STAGE;
-        uint8_t* b = a + S::RAW_X + (GtCfg<BT>::PLACE && buf ? S::B : 0);
-        if (weights) gt_expect_tx(&loaded[rs], SUB * (S::A + S::B));
-#pragma unroll
-        for (int h = 0; h < SUB; ++h) {                             // (a box beyond K is zeros)
-            if (weights) gt_tma_2d(a + h * S::A, &map_w, k + h * GT_HALF, head * p.N + n0, &loaded[rs]);
-            if (x) gt_tma_3d(b + (GtCfg<BT>::PLACE ? 2 : 1) * h * S::B, &map_x, k + h * GT_HALF, head, m0, &loaded[rs]);
-        }
+        uint8_t* box = ring + i % RAW * S::BOX;
+        uint64_t* bar = &loaded[i % RAW];
+        if (weights) gt_expect_tx(bar, S::BOX);
+        if (weights) gt_tma_2d(box, &map_w, k, head * p.N + n0, bar);                       // (columns beyond K are zeros)
+        if (x) gt_tma_3d(box + S::A, &map_x, k, head, m0, bar);
     };
-    const int ahead = !TMA || unit0 >= n_units ? 0 : steps < RAW ? steps : RAW;              // stages asked for at once
+    // boxes whose weights are asked for at once
+    const int ahead = !TMA || !p.early || unit0 >= n_units ? 0 : steps < RAW ? steps : RAW;
     if (threadIdx.x == (S::CUT + ACC + 1) * 32) {
-        for (int s = 0; s < STAGES; ++s) { gt_init(&full[s], GtCfg<BT>::GROUP); gt_init(&empty[s], 1); }
-        for (int s = 0; s < RAW; ++s) { gt_init(&loaded[s], 1); if (!GtCfg<BT>::PLACE) gt_init(&raw_empty[s], 1); }
+        for (int s = 0; s < RAW; ++s) { gt_init(&loaded[s], 1); gt_init(&raw_empty[s], 4); }
+        for (int s = 0; s < STAGES; ++s) { gt_init(&full[s], 4); gt_init(&empty[s], 1); }
         for (int a = 0; a < 2; ++a) { gt_init(&hh_full[a], 1); gt_init(&hh_empty[a], ACC); }
         gt_init(small_empty, ACC);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        // The first weights are asked for before the kernel in front has ended, and before the block is set up: they depend on
-        // nothing.
+        // Weights that the caller says the kernel in front does not write are asked for before that kernel has ended, and before the
+        // block is set up.
         const GtUnit<BT> u(p, unit0);
-        for (int j = 0; j < ahead; ++j) tma_load(j, u.n0, u.m0, u.head, b0 * GT_BK + j * SUB * GT_HALF, true, false);
+        for (int j = 0; j < ahead; ++j) tma_load(j, u.n0, u.m0, u.head, b0 * GT_BK + j * GT_BOX, true, false);
     }
     if (warp == S::CUT + ACC) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     ::"r"(gt_smem(tmem_slot)), "r"(GtCfg<BT>::COLS) : "memory");
+                     ::"r"(gt_smem(tmem_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     gt_fence_before();
     __syncthreads();
     gt_fence_after();
     const uint32_t tmem = *tmem_slot;
+    bool stands = true;                                             // every sum that this thread has written
     gt_pdl_wait();                                                  // x is there, and nobody reads what out was
 
     if (warp < S::CUT) {
-        // ---- cut: stage number i of this block is group i % GROUPS's.  A thread takes 16 bytes wherever they lie in the swizzle;
-        // only numbers from global memory need their row and columns ----
-        constexpr int T = 32 * GtCfg<BT>::GROUP, AU = S::A / 16 / T, BU = (S::B / 16 + T - 1) / T;
-        constexpr int AB = AU < 8 ? AU : 8, BB = BU < 8 ? BU : 8;                   // 16-byte pieces read before the first is written
-        static_assert(AU % AB == 0 && BU % BB == 0, "whole batches");
-        static_assert(S::B / 16 < T || S::B / 16 % T == 0, "a thread has the same pieces of x as the others, or one or none");
-        const int group = warp / GtCfg<BT>::GROUP, t = threadIdx.x % T;
-        int first = 0;                                             // number of the unit's first stage
+        // ---- cut: box number i of this block is group i % GROUPS's.  Of the weights a warp has the 32 rows of its quarter of tensor
+        // memory, a lane one row; of x eight columns of a row (eight lanes next to each other have different rows: no two meet in a
+        // bank) ----
+        const int group = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane, r = lane & 7, c = lane >> 3;
+        const uint32_t wparts = tmem + ((uint32_t)(quarter * 32) << 16) + S::WPARTS;
+        int first = 0;                                             // number of the unit's first box
         bool ok = true;
         for (int unit = unit0; unit < n_units && ok; unit += step, first += steps) {
             const GtUnit<BT> u(p, unit);
             for (int i = first + (group + GROUPS - first % GROUPS) % GROUPS; i < first + steps; i += GROUPS) {
-                const int rs = i % RAW, stage = i % STAGES, buf = i / P & 1;
-                // (In this order: MMAs end in order, so every stage up to i - STAGES has been cut, and the loaded stage cannot be
+                const int s = i % STAGES, buf = HH > 1 ? i / P & 1 : 0;
+                // (In this order: MMAs end in order, so every box up to i - STAGES has been cut, and the loaded one cannot be
                 // waiting for number i - RAW still, whose phase has the other parity.)
-                ok = gt_wait(&empty[stage], ((i / STAGES) & 1) ^ 1, p.error, GT_ERR_CUT);
-                ok = ok && gt_wait(TMA ? &loaded[rs] : &raw_empty[rs], (i / RAW & 1) ^ (TMA ? 0 : 1), p.error, GT_ERR_CUT);
+                ok = gt_wait(&empty[s], ((i / STAGES) & 1) ^ 1, p.error, GT_ERR_CUT);
+                if (TMA) ok = ok && gt_wait(&loaded[i % RAW], (i / RAW) & 1, p.error, GT_ERR_CUT);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
+                gt_fence_after();
+                const uint8_t* raw = ring + i % RAW * S::BOX;
+                const int k0 = b0 * GT_BK + (i - first) * GT_BOX;
 #pragma unroll
-                for (int h = 0; h < SUB; ++h) {
-                    uint8_t* a = ring + rs * S::RAW_STAGE + h * S::A + 16 * t;
-                    uint8_t* a_rest = ring + S::CUT_RING + stage * S::STAGE + S::REST_A + h * S::A + 16 * t;
-                    const uint8_t* x = ring + rs * S::RAW_STAGE + S::RAW_X + (GtCfg<BT>::PLACE ? 2 * h * S::B + (buf ? S::B : 0) : h * S::B) + 16 * t;
-                    uint8_t* b = ring + S::CUT_RING + stage * S::STAGE + S::CUT_X + 2 * h * S::B + 16 * t;
-                    uint8_t* b_rest = b + (buf ? 0 : S::B);
-                    b += buf ? S::B : 0;                           // (x before its rests, or behind them)
-                    auto load = [&](const float* base, int ld, int rows, int at) -> float4 {
-                        const int row = at >> 3, k = b0 * GT_BK + ((i - first) * SUB + h) * GT_HALF + 4 * ((at & 7) ^ (row & 7));
-                        return gt_load4(base + (size_t)row * ld, k, K, row < rows);
-                    };
-#pragma unroll
-                    for (int j0 = 0; j0 < AU; j0 += AB) {
-                        float4 v[AB];
-#pragma unroll
-                        for (int j = 0; j < AB; ++j)
-                            if (TMA) v[j] = *reinterpret_cast<const float4*>(a + (j0 + j) * 16 * T);
-                            else v[j] = load(p.w + ((size_t)u.head * p.N + u.n0) * K, K, p.N - u.n0, t + (j0 + j) * T);
-#pragma unroll
-                        for (int j = 0; j < AB; ++j) {
-                            if (!TMA) *reinterpret_cast<float4*>(a + (j0 + j) * 16 * T) = v[j];
-                            *reinterpret_cast<ulonglong2*>(a_rest + (j0 + j) * 16 * T) =
-                                make_ulonglong2(gt_rest_of_cut(v[j].x, v[j].y), gt_rest_of_cut(v[j].z, v[j].w));
-                        }
+                for (int k = 0; k < GT_BOX; k += 8) {
+                    float4 a, b;
+                    if (TMA) {
+                        a = *reinterpret_cast<const float4*>(raw + row * 128 + (((k / 4) ^ r) << 4));
+                        b = *reinterpret_cast<const float4*>(raw + row * 128 + (((k / 4 + 1) ^ r) << 4));
+                    } else {
+                        const float* from = p.w + ((size_t)u.head * p.N + u.n0 + row) * K;
+                        a = gt_load4(from, k0 + k, K, u.n0 + row < p.N);
+                        b = gt_load4(from, k0 + k + 4, K, u.n0 + row < p.N);
                     }
-                    if (S::B / 16 >= T || t < S::B / 16) {
+                    uint4 part[3];
+                    gt_cut(a, b, part);
 #pragma unroll
-                        for (int j0 = 0; j0 < BU; j0 += BB) {
-                            float4 v[BB];
-#pragma unroll
-                            for (int j = 0; j < BB; ++j)
-                                if (TMA) v[j] = *reinterpret_cast<const float4*>(x + (j0 + j) * 16 * T);
-                                else v[j] = load(p.x + (size_t)u.head * K + (size_t)u.m0 * p.ldx, p.ldx, p.M - u.m0, t + (j0 + j) * T);
-#pragma unroll
-                            for (int j = 0; j < BB; ++j) {
-                                const GtPair v0 = gt_pair(v[j].x, v[j].y), v1 = gt_pair(v[j].z, v[j].w);
-                                const GtPair h0 = gt_rounded(v0), h1 = gt_rounded(v1);
-                                *reinterpret_cast<ulonglong2*>(b + (j0 + j) * 16 * T) = make_ulonglong2(h0, h1);
-                                *reinterpret_cast<ulonglong2*>(b_rest + (j0 + j) * 16 * T) =
-                                    make_ulonglong2(gt_sub(v0, h0), gt_sub(v1, h1));
-                            }
-                        }
-                    }
+                    for (int j = 0; j < 3; ++j) gt_st4(wparts + s * S::WSTAGE + j * (GT_BOX / 2) + k / 2, part[j]);
                 }
+                uint8_t* parts = ring + S::XRING + s * 3 * S::PART;
+                uint8_t* x0 = parts + (buf ? S::PART : 0);                                   // (first parts before second ones, or behind them)
+                uint8_t* x1 = parts + (buf ? 0 : S::PART);
+#pragma unroll
+                for (int j = 0; j < (BT / 8 + 3) / 4; ++j) {
+                    const int eight = quarter + 4 * j, row = 8 * eight + r;
+                    if (BT / 8 % 4 && eight >= BT / 8) break;
+                    if (BT == 16 && u.m0 + 8 * eight >= p.M) break;                          // rows that nobody has; up to 8: 26.3 us instead of 26.7
+                    float4 a, b;
+                    if (TMA) {
+                        a = *reinterpret_cast<const float4*>(raw + S::A + row * 128 + (((2 * c) ^ r) << 4));
+                        b = *reinterpret_cast<const float4*>(raw + S::A + row * 128 + (((2 * c + 1) ^ r) << 4));
+                    } else {
+                        const float* x = p.x + (size_t)u.head * K + (size_t)(u.m0 + row) * p.ldx;
+                        const int k = k0 + 8 * c;
+                        a = gt_load4(x, k, K, u.m0 + row < p.M);
+                        b = gt_load4(x, k + 4, K, u.m0 + row < p.M);
+                    }
+                    uint4 part[3];
+                    gt_cut(a, b, part);
+                    const int at = row * 64 + ((c ^ (r >> 1)) << 4);
+                    *reinterpret_cast<uint4*>(x0 + at) = part[0];
+                    *reinterpret_cast<uint4*>(x1 + at) = part[1];
+                    *reinterpret_cast<uint4*>(parts + 2 * S::PART + at) = part[2];
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // the MMAs read through the other proxy
+                gt_fence_before();
                 __syncwarp();
-                if (lane == 0) gt_arrive(&full[stage]);
+                if (lane == 0) {
+                    gt_arrive(&full[s]);
+                    if (TMA) gt_arrive(&raw_empty[i % RAW]);
+                }
             }
         }
         __syncwarp();
@@ -380,70 +415,92 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             bool ok = true;
             if (ahead) {
                 const GtUnit<BT> u(p, unit0);
-                for (int j = 0; j < ahead; ++j) tma_load(j, u.n0, u.m0, u.head, b0 * GT_BK + j * SUB * GT_HALF, false, true);
+                for (int j = 0; j < ahead; ++j) tma_load(j, u.n0, u.m0, u.head, b0 * GT_BK + j * GT_BOX, false, true);
             }
             for (int unit = unit0; unit < n_units && ok; unit += step) {
                 const GtUnit<BT> u(p, unit);
                 for (int j = 0; j < steps; ++j, ++i) {
                     if (i < ahead) continue;
                     if (!gt_wait(&raw_empty[i % RAW], ((i / RAW) & 1) ^ 1, p.error, GT_ERR_LOAD)) { ok = false; break; }
-                    tma_load(i, u.n0, u.m0, u.head, b0 * GT_BK + j * SUB * GT_HALF, true, true);
+                    tma_load(i, u.n0, u.m0, u.head, b0 * GT_BK + j * GT_BOX, true, true);
                 }
             }
+            for (int j = i < RAW ? 0 : i - RAW; j < i; ++j)         // loads in flight end before the block may
+                gt_wait(&loaded[j % RAW], (j / RAW) & 1, p.error, GT_ERR_LOAD);
         }
         __syncwarp();
     } else if (warp == S::CUT + ACC) {
         // ---- MMAs: warp-uniform loop, one elected lane issues ----
         constexpr uint32_t one = gt_idesc(BT), two = gt_idesc(2 * BT);
-        constexpr uint64_t BL = S::B >> 4;
         uint32_t elected;
         asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}\n" : "=r"(elected));
         const bool leader = elected != 0;
-        const uint64_t da0 = gt_desc(ring), dr0 = gt_desc(ring + S::CUT_RING + S::REST_A), db0 = gt_desc(ring + S::CUT_RING + S::CUT_X);
-        int rs = 0, stage = 0, buf = 0;
-        uint32_t phase = 0, small_phase = 1, hh_phase = 1;         // (the accumulators alternate: one phase for a pair of them)
+        const uint64_t x0 = gt_desc(ring + S::XRING);
+        constexpr uint64_t PART = S::PART >> 4;
+        int stage = 0, buf = 0, last = -1;
+        uint32_t phase = 0, small_phase = 1, hh_phase = 1;         // (two accumulators alternate: one phase for the pair)
         bool ok = true;
         for (int unit = unit0; unit < n_units && ok; unit += step) {
             for (int i = 0; i < steps; ++i) {
-                const bool begins = P == 1 || i % P == 0, ends = P == 1 || i % P == P - 1, first = i % (P * GT_SLICE) == 0;
-                // (A k-block in the middle asks for one barrier twice rather than for two.)
-                ok = gt_ended(&full[stage], phase, begins ? &hh_empty[buf] : &full[stage], begins ? hh_phase : phase,
+                const bool begins = i % P == 0, ends = i % P == P - 1, first = i % (P * GT_SLICE) == 0, hh = begins && HH > 1;
+                // (A box in the middle of a k-block asks for one barrier three times rather than for three.)
+                ok = gt_ended(&full[stage], phase, hh ? &hh_empty[buf] : &full[stage], hh ? hh_phase : phase,
                               first ? small_empty : &full[stage], first ? small_phase : phase);
                 if (!__all_sync(0xffffffffu, ok)) {
-                    ok = !begins || gt_wait(&hh_empty[buf], hh_phase, p.error, GT_ERR_MMA);
+                    ok = !hh || gt_wait(&hh_empty[buf], hh_phase, p.error, GT_ERR_MMA);
                     ok = ok && (!first || gt_wait(small_empty, small_phase, p.error, GT_ERR_MMA));
                     ok = __all_sync(0xffffffffu, ok && gt_wait(&full[stage], phase, p.error, GT_ERR_MMA));
                 }
                 if (first) small_phase ^= 1;
                 if (!ok) break;
                 gt_fence_after();
+                const uint32_t w = tmem + S::WPARTS + stage * S::WSTAGE, d_small = tmem + BT, d_hh = tmem + (buf ? 2 * BT : 0);
+                const uint64_t x = x0 + (uint64_t)stage * 3 * PART;
                 if (leader) {
-                    const uint64_t da = da0 + (uint64_t)((rs * S::RAW_STAGE) >> 4);
-                    const uint64_t dr = dr0 + (uint64_t)((stage * S::STAGE) >> 4), db = db0 + (uint64_t)((stage * S::STAGE) >> 4);
-                    const uint32_t d_hh = tmem + (buf ? 2 * BT : 0), d_small = tmem + BT, d_both = tmem + (buf ? BT : 0);
 #pragma unroll
-                    for (int k = 0; k < SUB * GT_HALF / 8; ++k) {
-                        const int h = k / (GT_HALF / 8);
-                        const uint64_t o = (uint64_t)((k * 32 % 128) >> 4);
-                        const uint64_t a = da + h * (S::A >> 4) + o, b = db + 2 * h * BL + o, bh = b + (buf ? BL : 0), bl = b + (buf ? 0 : BL);
-                        if (k == 0 && begins && !first) {           // the large ones begin anew, the small ones go on
-                            gt_mma(d_hh, a, bh, one, 0u);
-                            gt_mma(d_small, a, bl, one, 1u);
+                    for (int k = 0; k < GT_BOX / 16; ++k) {
+                        const uint32_t wa = w + 8 * k, wb = wa + GT_BOX / 2, wc = wb + GT_BOX / 2;                  // parts of the weights
+                        const uint64_t xa = x + 2 * k + (buf ? PART : 0), xb = x + 2 * k + (buf ? 0 : PART), xc = x + 2 * k + 2 * PART;
+                        if (HH == 1) {                              // the large ones follow below
+                            gt_mma(d_small, wa, xb, one, k == 0 && first ? 0u : 1u);
+                        } else if (k == 0 && begins && !first) {    // the large ones begin anew, the small ones go on
+                            gt_mma(d_hh, wa, xa, one, 0u);
+                            gt_mma(d_small, wa, xb, one, 1u);
                         } else {
-                            gt_mma(d_both, a, b, two, k == 0 && first ? 0u : 1u);
+                            gt_mma(tmem + (buf ? BT : 0), wa, x + 2 * k, two, k == 0 && first ? 0u : 1u);
                         }
-                        gt_mma(d_small, dr + h * (S::A >> 4) + o, bh, one, 1u);
+                        gt_mma(d_small, wb, xa, one, 1u);
+                        gt_mma(d_small, wb, xb, one, 1u);
+                        gt_mma(d_small, wa, xc, one, 1u);
+                        gt_mma(d_small, wc, xa, one, 1u);
                     }
+                }
+                if (HH == 1) {                                      // (the one accumulator has been emptied meanwhile)
+                    __syncwarp();
+                    if (begins) {
+                        ok = __all_sync(0xffffffffu, gt_wait(&hh_empty[0], hh_phase, p.error, GT_ERR_MMA));
+                        gt_fence_after();
+                    }
+                    if (leader && ok) {
+#pragma unroll
+                        for (int k = 0; k < GT_BOX / 16; ++k) gt_mma(d_hh, w + 8 * k, x + 2 * k, one, k == 0 && begins ? 0u : 1u);
+                    }
+                }
+                if (leader) {
                     gt_commit(&empty[stage]);
-                    if (!GtCfg<BT>::PLACE) gt_commit(&raw_empty[rs]);
                     if (ends) gt_commit(&hh_full[buf]);
                 }
                 __syncwarp();
-                if (ends) { hh_phase ^= buf; buf ^= 1; }
-                if (++rs == RAW) rs = 0;
+                last = 2 * stage + (int)phase;
+                if (!ok) break;
+                if (ends) {
+                    hh_phase ^= HH > 1 ? buf : 1;
+                    if (HH > 1) buf ^= 1;
+                }
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
+        if (last >= 0) gt_wait(&empty[last >> 1], last & 1, p.error, GT_ERR_MMA);           // nor do MMAs outlive their tensor memory
         __syncwarp();
     } else {
         // ---- empty the accumulators: a warp reads the lanes of its quarter (warp & 3), CPT of the columns ----
@@ -455,9 +512,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const GtUnit<BT> u(p, unit);
             float s[CPT];
             for (int kb = b0; kb < b1; ++kb, ++i) {
-                const int buf = i & 1, slice = kb / GT_SLICE;
+                const int buf = HH > 1 ? i & 1 : 0, slice = kb / GT_SLICE;
                 const bool first = kb % GT_SLICE == 0, end = kb == b1 - 1, last = end || kb % GT_SLICE == GT_SLICE - 1;
-                ok = __all_sync(0xffffffffu, gt_wait(&hh_full[buf], (i >> 1) & 1, p.error, GT_ERR_SUMS));
+                ok = __all_sync(0xffffffffu, gt_wait(&hh_full[buf], (HH > 1 ? i >> 1 : i) & 1, p.error, GT_ERR_SUMS));
                 if (!ok) break;
                 gt_fence_after();
                 uint32_t v[16];
@@ -486,9 +543,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     if (last) gt_arrive(small_empty);
                 }
                 if (!last) continue;
-                if (splits > 1) {                                   // kept until the cluster's MMAs are all done
+                if (splits > 1) {                                   // kept until the cluster's MMAs are all done (the last where
+                                                                    // large products were: this block's have ended)
 #pragma unroll
-                    for (int c = 0; c < CPT; c += 16) gt_st16(t + (3 + slice - s0) * BT + c, s + c);
+                    for (int c = 0; c < CPT; c += 16) gt_st16(t + (end ? 0 : S::SUMS + (slice - s0) * BT) + c, s + c);
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                     continue;
                 }
@@ -496,39 +554,31 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (slice > 0) {
 #pragma unroll
                     for (int c = 0; c < CPT; c += 16) {
-                        gt_ld16(t + 3 * BT + c, v);
+                        gt_ld16(t + S::SUMS + c, v);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) s[c + j] = __uint_as_float(v[j]) + s[c + j];
                     }
                 }
                 if (!end) {
 #pragma unroll
-                    for (int c = 0; c < CPT; c += 16) gt_st16(t + 3 * BT + c, s + c);
+                    for (int c = 0; c < CPT; c += 16) gt_st16(t + S::SUMS + c, s + c);
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 }
             }
             const int n = u.n0 + quarter * 32 + lane;
             if (splits == 1 && ok && n < p.N) {
-                const float* x = p.x + (size_t)u.head * K;
-                const float* w = p.w + ((size_t)u.head * p.N + n) * K;
                 float* out = p.out + (size_t)u.head * p.N + n;
-                bool finite = true;
 #pragma unroll
                 for (int c = 0; c < CPT; ++c) {
                     const int m = u.m0 + c0 + c;
                     if (m < p.M) {
                         out[(size_t)m * p.ldo] = s[c];
-                        finite = finite && gt_finite(s[c]);
+                        stands = stands && gt_stands(s[c]);
                     }
-                }
-                if (!finite) {
-#pragma unroll 1
-                    for (int m = u.m0 + c0; m < u.m0 + c0 + CPT && m < p.M; ++m)
-                        if (!gt_finite(out[(size_t)m * p.ldo])) out[(size_t)m * p.ldo] = gt_chain(x + (size_t)m * p.ldx, w, K);
                 }
             }
         }
-        if (gt_extra_wait) gt_wait(&hh_full[i & 1], (i >> 1) & 1, p.error, GT_ERR_SUMS);       // tests: a wait that runs out
+        if (gt_extra_wait) gt_wait(&hh_full[HH > 1 ? i & 1 : 0], (HH > 1 ? i >> 1 : i) & 1, p.error, GT_ERR_SUMS);       // tests: a wait that runs out
         __syncwarp();
     }
     if (splits > 1) {
@@ -545,7 +595,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll 1
                 for (int c = 0; c < CPT && c0 + c < rows; c += 16) {
                     uint32_t v[16];
-                    gt_ld16(t + (3 + s - s0) * BT + c, v);
+                    gt_ld16(t + (s == s1 - 1 ? 0 : S::SUMS + (s - s0) * BT) + c, v);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         if (c0 + c + j < rows)
@@ -565,18 +615,33 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 for (int s = 1; s < slices; ++s) v += mine[((size_t)s * per + l) * GT_ROWS];
                 const int m = u.m0 + rank * per + l;
                 if (n < p.N) {
-                    if (!gt_finite(v))
-                        v = gt_chain(p.x + (size_t)u.head * K + (size_t)m * p.ldx, p.w + ((size_t)u.head * p.N + n) * K, K);
                     p.out[(size_t)u.head * p.N + n + (size_t)m * p.ldo] = v;
+                    stands = stands && gt_stands(v);
                 }
             }
         }
     }
     gt_fence_before();
-    __syncthreads();
+    const bool again = __syncthreads_or(!stands);
     if (warp == S::CUT + ACC) {
         gt_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(GtCfg<BT>::COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
+    }
+    if (again) {                                                    // all warps look through what the block has written, four rows of x at a time
+        for (int unit = unit0; unit < n_units; unit += step) {
+            const GtUnit<BT> u(p, unit);
+            const int all = p.M - u.m0 < BT ? p.M - u.m0 : BT, per = (all + splits - 1) / splits;
+            const int m0 = u.m0 + rank * per, m1 = m0 + per < u.m0 + all ? m0 + per : u.m0 + all;
+            for (int item = warp; item < (per + 3) / 4 * 4; item += S::THREADS / 32) {
+                const int m = m0 + item / 4 * 4, rows = m1 - m < 4 ? m1 - m : 4, n = u.n0 + (item & 3) * 32 + lane;
+                if (n >= p.N) continue;
+                float* out = p.out + (size_t)u.head * p.N + n + (size_t)m * p.ldo;
+                bool four = true;
+                for (int i = 0; i < rows; ++i) four = four && gt_stands(out[(size_t)i * p.ldo]);
+                if (!four)
+                    gt_chains<TMA>(p.x + (size_t)u.head * K + (size_t)m * p.ldx, p.ldx, rows, p.w + ((size_t)u.head * p.N + n) * K, K, out, p.ldo);
+            }
+        }
     }
 }
 
@@ -598,7 +663,7 @@ template <int BT>
 static bool gt_can_split(int M, int K, int splits) {
     if (splits == 1) return true;
     const int slices = gt_slices(K), rows = M < BT ? M : BT;
-    return splits <= 8 && splits <= slices && (slices + splits - 1) / splits <= GtSizes<BT>::REGIONS &&
+    return splits <= 8 && splits <= slices && (slices + splits - 1) / splits <= GtSizes<BT>::REGIONS + 1 &&
            (long long)slices * ((rows + splits - 1) / splits) * GT_ROWS * 4 <= GtSizes<BT>::RING;
 }
 
@@ -622,7 +687,7 @@ static GtEncodeTiledFn gt_encode_tiled() {
 // 32 columns (128 bytes, 128-byte swizzle) of `box_rows` rows: of the weights [rows, K], or of one head of x [M, H, K].
 static int gt_map_w(CUtensorMap* map, const float* w, long long rows, int K) {
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)K * 4};
-    const cuuint32_t box[2] = {GT_HALF, GT_ROWS}, elem[2] = {1, 1};
+    const cuuint32_t box[2] = {GT_BOX, GT_ROWS}, elem[2] = {1, 1};
     GtEncodeTiledFn enc = gt_encode_tiled();
     if (!enc) return NI_ERR_BAD_ARGUMENT;
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(w), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -631,7 +696,7 @@ static int gt_map_w(CUtensorMap* map, const float* w, long long rows, int K) {
 }
 static int gt_map_x(CUtensorMap* map, const float* x, int M, int H, int K, int ldx, int box_rows) {
     const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)H, (cuuint64_t)M}, strides[2] = {(cuuint64_t)K * 4, (cuuint64_t)ldx * 4};
-    const cuuint32_t box[3] = {GT_HALF, 1, (cuuint32_t)box_rows}, elem[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {GT_BOX, 1, (cuuint32_t)box_rows}, elem[3] = {1, 1, 1};
     GtEncodeTiledFn enc = gt_encode_tiled();
     if (!enc) return NI_ERR_BAD_ARGUMENT;
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(x), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -701,10 +766,10 @@ static int gt_clusters(int splits) {
     return cached[dev][splits];
 }
 
-// The tile and the split of K that are done first by what they measured: a k-block of 64 takes a block 0.65, 0.95, 1.10 and 1.62 us
+// The tile and the split of K that are done first by what they measured: a k-block of 64 takes a block 0.70, 0.82, 1.02 and 1.55 us
 // with 16, 32, 64 and 128 rows of x (128 weight rows; 0.74 us is what memory gives every SM for its 32 KB), a launch 6 us besides, and
-// a cluster 1.7 us and 0.02 us for every row and slice of a block's sums.  [2048, 2048] and 177 rows: 30.9 us in two slices of 64-row
-// tiles, 43 whole; [2048, 8192] and 1 row: 24.5 in six slices, 29.7 in four, 89 whole.
+// a cluster 1.5 us, 0.045 us for every row and 0.01 for every row and slice of a block's sums.  [2048, 2048] and 120 rows: 19.2 us in
+// four slices of 64-row tiles, 38 whole; [2048, 8192] and 2 rows: 26.6 in six slices, 31.9 in four, 98 whole.
 static void gt_choose(const GtParams& p, int& bt, int& splits) {
     const int slices = gt_slices(p.K);
     const long long n_tiles = (long long)((p.N + GT_ROWS - 1) / GT_ROWS) * p.H;
@@ -714,7 +779,7 @@ static void gt_choose(const GtParams& p, int& bt, int& splits) {
     for (int i = 0; i < 4; ++i) {
         const int b = 16 << i;
         if (want_bt ? b != want_bt : (b > 16 && b >= 2 * p.M)) continue;
-        const double per_block = i == 0 ? 0.65 : i == 1 ? 0.95 : i == 2 ? 1.10 : 1.62;
+        const double per_block = i == 0 ? 0.70 : i == 1 ? 0.82 : i == 2 ? 1.02 : 1.55;
         const long long units = n_tiles * ((p.M + b - 1) / b);
         for (int sp = 1; sp <= 8; ++sp) {
             if (want_splits ? sp != want_splits : sp > 1 && units * sp > 4LL * ni_sm_count()) continue;
@@ -722,7 +787,7 @@ static void gt_choose(const GtParams& p, int& bt, int& splits) {
                   : b == 64 ? gt_can_split<64>(p.M, p.K, sp) : gt_can_split<128>(p.M, p.K, sp))) continue;
             const long long at_once = sp == 1 ? ni_sm_count() : gt_clusters(sp), waves = (units + at_once - 1) / at_once;
             const int mine = (slices + sp - 1) / sp, rows = p.M < b ? p.M : b;
-            const double once = sp == 1 ? 0.0 : 1.7 + 0.02 * rows * mine;
+            const double once = sp == 1 ? 0.0 : 1.5 + 0.045 * rows + 0.01 * rows * mine;
             const double us = 6.0 + waves * (once + per_block * GT_SLICE * mine);
             if (!bt || us < best) { best = us; bt = b; splits = sp; }
         }
@@ -732,10 +797,10 @@ static void gt_choose(const GtParams& p, int& bt, int& splits) {
 // One product per head: out[m, h, :] = x[m, h, :] . w[h]^T with x [M, H, K] (rows ldx floats apart), w [H, N, K], out [M, H, N].
 // bt (16, 32, 64, 128) and splits (blocks that share K): 0 leaves the choice to the sizes; every choice gives the same bits.
 NI_EXPORT int ni_gemm_f32_tc(const float* x, int ldx, const float* w, float* out, int M, int N, int K, int H, int bt, int splits,
-                             int* error, cudaStream_t stream) {
+                             int early, int* error, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || H <= 0) return NI_OK;
     if (K <= 0 || error == nullptr || (long long)ldx < (long long)H * K || bt < 0 || splits < 0) return NI_ERR_BAD_ARGUMENT;
-    GtParams p = {x, w, out, M, N, K, H, ldx, H * N, splits, error};
+    GtParams p = {x, w, out, M, N, K, H, ldx, H * N, splits, early, error};
     gt_choose(p, bt, p.splits);
     switch (bt) {
         case 16: return gt_launch_loads<16>(p, stream);

@@ -48,7 +48,7 @@ _SIGNATURES = {
         "ni_gemm_f32_heads": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
     },
     "gemm_f32_tc": {
-        "ni_gemm_f32_tc": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+        "ni_gemm_f32_tc": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
         "ni_gemm_f32_tc_set_wait": [_LL, _I],
     },
     "pointwise": {
@@ -559,17 +559,18 @@ def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
 
 
 def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int = 0, splits: int = 0) -> None:
-    """gemm_f32_heads on the tensor cores, every number cut in two (csrc/gemm_f32_tc.cu); w may be [N, K] for one head.  ``rows`` (16,
+    """gemm_f32_heads on the tensor cores, every number cut in three (csrc/gemm_f32_tc.cu); w may be [N, K] for one head.  ``rows`` (16,
     32, 64, 128: rows of x in a tile) and ``splits`` (blocks that share K, up to 8): 0 leaves them to the sizes; the bits are the
     same."""
     args = _heads_of(x, w if w.dim() == 3 else w.unsqueeze(0), out, "gemm_f32_tc")
-    _check(load("gemm_f32_tc").ni_gemm_f32_tc(*args, int(rows), int(splits), _error_word(x.device).data_ptr(), _stream()), "gemm_f32_tc")
+    _check(load("gemm_f32_tc").ni_gemm_f32_tc(*args, int(rows), int(splits), 1, _error_word(x.device).data_ptr(), _stream()), "gemm_f32_tc")
 
 
-# Rows of at least this many columns go to the tensor cores as numbers cut in two, shorter ones to the chains of csrc/gemm_f32.cu.  The
+# Rows of at least this many columns go to the tensor cores as numbers cut in three, shorter ones to the chains of csrc/gemm_f32.cu.  The
 # rule looks at nothing but the row's length, so that a row's bits depend on no other row.  Relative error against 64 bits, cut in
-# two / as a chain: normal numbers 3.0e-7 / 4.1e-7 at 512 columns, 3.0e-7 / 5.7e-7 at 1,024, 3.1e-7 / 1.6e-6 at 8,192; positive numbers
-# 3.6e-7 / 3.1e-7, 3.7e-7 / 4.9e-7, 3.6e-7 / 1.3e-6.  Below the line the chain is as close, and short rows have little to gain.
+# three / as a chain: normal numbers 0.9e-7 / 4.1e-7 at 512 columns, 0.9e-7 / 5.7e-7 at 1,024, 1.3e-7 / 1.6e-6 at 8,192; rows of a
+# single term 2.6e-8 / 2.5e-8.  us for 2,048 weight rows: 512 columns, 1 row of x 8.7 / 3.8, 177 rows 12.7 / 22.7; 1,024 columns 8.6 / 5.3 and
+# 19.7 / 38.6.  Below the line single tokens lose more than the prompts' products are worth.
 F32_CUT_COLUMNS = 1024
 
 

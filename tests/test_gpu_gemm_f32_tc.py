@@ -1,4 +1,4 @@
-"""The FP32 product on the tensor cores (numbers cut in two): bits that do not depend on tile, split or neighbours, errors
+"""The FP32 product on the tensor cores (numbers cut in three): bits that do not depend on tile, split or neighbours, errors
 against 64 bits, rows that TMA does not take, infinities and overflows, a wait that runs out."""
 import pytest
 import torch
@@ -17,25 +17,33 @@ def _exact(x, w):
 
 
 def _bound(k, total):
-    """Of an element's error, from the sum of |x| |w|: the rests lose up to 3 of 2^23 parts of w and 1 of x, the product of rests
-    is 2^-21 at most; 9 cuts (of 2^-23) while 64 columns are added up, a rounding (2^-24) per 64 and per 256 columns."""
-    return total * (4 * 2.0 ** -23 + 2.0 ** -21 + 9 * 2.0 ** -23 + (k / 64 + k / 256 + 4) * 2.0 ** -24) + 1e-30
+    """Of an element's error, from the sum of |x| |w|: second parts are 2^-8 of a number at most, third ones 2^-16, so what is left out
+    is 2^-23; 9 cuts (of 2^-23) of the large products while 64 columns are added up, 160 of the small ones, 2^-7 of them, in 256
+    columns; a rounding (2^-24) per 64 and per 256 columns."""
+    return total * (2.0 ** -23 + 9 * 2.0 ** -23 + 1.25 * 2.0 ** -23 + (k / 64 + k / 256 + 4) * 2.0 ** -24) + 1e-30
+
+
+def _taken(m, k, rows, splits):
+    """Whether a tile takes a split: a slice of 256 columns for each block, room for a block's sums and for those that arrive."""
+    slices, (regions, ring) = -(-k // 256), {16: (18, 215040), 32: (8, 208896), 64: (4, 196608), 128: (2, 180224)}[rows]
+    return splits == 1 or (splits <= slices and -(-slices // splits) <= regions
+                           and slices * -(-min(m, rows) // splits) * 512 <= ring)
 
 
 def _choices(ops, x, w, out):
-    """Every tile and split that takes the product."""
+    """Every tile and split that takes the product; the others, and no others, are refused."""
     for rows in (16, 32, 64, 128):
-        for splits in (1, 2, 3, 5, 8):
-            try:
-                ops.gemm_f32_tc(x, w, out, rows, splits)
-            except ops.KernelError:
-                assert splits > 1
+        for splits in (1, 2, 3, 4, 5, 8):
+            if not _taken(x.shape[0], x.shape[1], rows, splits):
+                with pytest.raises(ops.KernelError, match="bad argument"):
+                    ops.gemm_f32_tc(x, w, out, rows, splits)
                 continue
+            ops.gemm_f32_tc(x, w, out, rows, splits)
             yield rows, splits
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (2, 128, 32), (15, 129, 64), (16, 127, 68), (17, 300, 256), (33, 5, 260), (64, 256, 1024),
-                                   (65, 130, 1028), (130, 96, 2048), (3, 257, 8192), (129, 140, 4096), (40, 33, 1023)])
+                                   (64, 128, 2048), (128, 128, 2048), (177, 256, 2048), (65, 130, 1028), (130, 96, 2048), (3, 257, 8192), (129, 140, 4096), (40, 33, 1023)])
 def test_every_tile_and_split_gives_the_same_bits(m, n, k):
     from nanoinfer_b200.kernels import ops
     x, w = _randn(m, k, seed=1), _randn(n, k, seed=2)
@@ -65,6 +73,66 @@ def test_errors_are_smaller_than_those_of_a_chain(k, positive):
     ops.linear_f32(x, w, cut)
     ops.gemm_f32(x, w, chain)
     assert (cut.double() - want).norm() < (chain.double() - want).norm()
+
+
+def _rows_of_few(kind, k):
+    x, w = torch.zeros(64, k, device=DEV), _randn(320, k, seed=14)
+    at = torch.arange(64, device=DEV)
+    if kind == "one of 1":
+        x[at, at * 13 % k] = 1.0
+    elif kind == "one":
+        x[at, at * 13 % k] = _randn(64, seed=13)
+    elif kind == "ten":
+        x = _randn(64, k, seed=13) * (torch.rand(64, k, generator=torch.Generator().manual_seed(15)).to(DEV) < 10 / k)
+    elif kind == "one dominates":
+        x = _randn(64, k, seed=13, scale=1e-4)
+        x[at, at * 13 % k] = 3.0
+    else:
+        x, w = _randn(64, k, seed=13), torch.eye(320, k, device=DEV)
+    return x, w
+
+
+@pytest.mark.parametrize("k", [1024, 2048, 8192])
+@pytest.mark.parametrize("kind", ["one of 1", "one", "ten", "one dominates", "identity"])
+def test_rows_of_few_terms_are_as_exact_as_a_chain(kind, k):
+    """Parts that hold whole numbers: a single product is rounded once, and weights (or activations) that meet a one come back as they
+    were.  1.05: what is left out of a product, 2^-25 of it in the mean square, beside a rounding's 2^-24 / sqrt(3)."""
+    from nanoinfer_b200.kernels import ops
+    x, w = _rows_of_few(kind, k)
+    want, _ = _exact(x, w)
+    cut, chain = torch.empty(64, 320, device=DEV), torch.empty(64, 320, device=DEV)
+    ops.linear_f32(x, w, cut)
+    ops.gemm_f32(x, w, chain)
+    assert (cut.double() - want).norm() <= 1.05 * (chain.double() - want).norm()
+    if kind in ("one of 1", "identity"):
+        assert torch.equal(cut, chain)
+
+
+@pytest.mark.parametrize("rows,splits", [(16, 1), (16, 2), (32, 4), (64, 4), (128, 1), (128, 8)])
+def test_numbers_near_the_ends_of_the_range(rows, splits):
+    """Third parts of numbers below 2^-110 are beyond bfloat16: sums below 2^-80 (and from 2^100 on) are chains; beside ordinary
+    numbers such ones lose 2^-133 at most."""
+    from nanoinfer_b200.kernels import ops
+    m, n, k = 40, 140, 2048
+    x, w = _randn(m, k, seed=16), _randn(n, k, seed=17)
+    x[3] *= 2.0 ** -120
+    x[4] *= 2.0 ** -140                              # subnormal
+    x[5] *= 2.0 ** 110
+    x[6, ::2] *= 2.0 ** -122
+    w[7, ::3] *= 2.0 ** -125
+    w[8] = 0
+    got, chain = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops.gemm_f32_tc(x, w, got, rows, splits)
+    ops.gemm_f32(x, w, chain)
+    live = torch.arange(n, device=DEV) != 8
+    for i in (3, 5):
+        assert torch.equal(got[i, live], chain[i, live])
+    assert (got[:, 8] == 0).all()
+    want, total = _exact(x, w)
+    lost = 2.0 ** -133 * (x.double().abs().sum(1)[:, None] + w.double().abs().sum(1)[None])
+    ordinary = torch.ones(m, dtype=torch.bool, device=DEV)
+    ordinary[5] = False
+    assert bool(((got.double() - want).abs() <= _bound(k, total) - 1e-30 + lost)[ordinary].all())
 
 
 @pytest.mark.parametrize("m,k,offset", [(3, 1040, 1), (20, 1036, 2), (70, 1024, 4), (5, 1031, 0)])
