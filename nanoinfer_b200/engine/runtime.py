@@ -165,7 +165,8 @@ class Runtime:
 
     def linear(self, x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                residual: Optional[torch.Tensor] = None, warm=None, handoff=None, affine=None):
-        """y[M, N] = x[M, K] . w[N, K]^T.  ``out_dtype`` float32 asks for FP32 results
+        """y[M, N] = x[M, K] . w[N, K]^T; w is a weight, not the work of the kernel in front (it may be read before that one has
+        ended).  ``out_dtype`` float32 asks for FP32 results
         (logits); the default is the compute dtype.  With ``residual`` (the FP32 residual
         stream) the kernel MAY add the product into it and return None; otherwise the product
         is returned and the caller adds it.  ``affine`` (scale, shift), float32 per column, either may be None: what is
@@ -175,7 +176,7 @@ class Runtime:
         out_dtype = out_dtype or self.dtype
         if self.dtype == torch.float32:
             out = self.empty(m, n, dtype=torch.float32)
-            ops.linear_f32(x, w, out)
+            ops.linear_f32(x, w, out, constant_w=True)
             return out if affine is None else ops.ScaledAddition(out, *affine)
         if residual is None and self.swapped_gemm(m, n, x.shape[1]):
             out = self.empty(m, n, dtype=out_dtype)
@@ -185,13 +186,13 @@ class Runtime:
 
     def heads_linear(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """One product per head: y[t, h, :] = x[t, h, :] . w[h]^T for x [T, H K] (some columns of a wider
-        matrix will do) and w [H, N, K]; returns [T, H N] in the compute dtype.  float32: the package's own kernels, an order
+        matrix will do) and w [H, N, K], a weight as in linear; returns [T, H N] in the compute dtype.  float32: the package's own kernels, an order
         of sums that the row's length fixes; bfloat16: a library batched product (FP32 accumulation) written straight into y."""
         n_heads, n, k = w.shape
         t = x.shape[0]
         y = self.empty(t, n_heads * n)
         if self.dtype == torch.float32:
-            ops.linear_f32(x, w, y)
+            ops.linear_f32(x, w, y, constant_w=True)
         else:
             torch.bmm(x.view(t, n_heads, k).transpose(0, 1), w.transpose(1, 2), out=y.view(t, n_heads, n).transpose(0, 1))
         return y

@@ -558,12 +558,20 @@ def gemm_f32_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _check(load("gemm_f32").ni_gemm_f32_heads(*_heads_of(x, w, out, "gemm_f32_heads"), _stream()), "gemm_f32_heads")
 
 
-def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int = 0, splits: int = 0) -> None:
-    """gemm_f32_heads on the tensor cores, every number cut in three (csrc/gemm_f32_tc.cu); w may be [N, K] for one head.  ``rows`` (16,
-    32, 64, 128: rows of x in a tile) and ``splits`` (blocks that share K, up to 8): 0 leaves them to the sizes; the bits are the
-    same."""
-    args = _heads_of(x, w if w.dim() == 3 else w.unsqueeze(0), out, "gemm_f32_tc")
-    _check(load("gemm_f32_tc").ni_gemm_f32_tc(*args, int(rows), int(splits), 1, _error_word(x.device).data_ptr(), _stream()), "gemm_f32_tc")
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int = 0, splits: int = 0, constant_w: bool = False) -> None:
+    """gemm_f32 (w [N, K]) or gemm_f32_heads (w [H, N, K]) on the tensor cores, every number cut in three (csrc/gemm_f32_tc.cu).
+    ``rows`` (16, 32, 64, 128: rows of x in a tile) and ``splits`` (blocks that share K, up to 8): 0 leaves them to the sizes; the bits
+    are the same.  ``constant_w``: the kernel in front on this stream does not write w (a weight that was laid out long ago), so that
+    it may be read before that kernel has ended."""
+    if w.dim() == 2:
+        (m, k), n = x.shape, w.shape[0]
+        if w.shape[1] != k or out.shape != (m, n):
+            raise KernelError("gemm_f32_tc: shapes do not agree")
+        args = (_dev(x, "x", torch.float32), k, _dev(w, "w", torch.float32), _dev(out, "out", torch.float32), m, n, k, 1)
+    else:
+        args = _heads_of(x, w, out, "gemm_f32_tc")
+    _check(load("gemm_f32_tc").ni_gemm_f32_tc(*args, int(rows), int(splits), 1 if constant_w else 0, _error_word(x.device).data_ptr(),
+                                              _stream()), "gemm_f32_tc")
 
 
 # Rows of at least this many columns go to the tensor cores as numbers cut in three, shorter ones to the chains of csrc/gemm_f32.cu.  The
@@ -574,11 +582,11 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int =
 F32_CUT_COLUMNS = 1024
 
 
-def linear_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def linear_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, constant_w: bool = False) -> None:
     """The 32-bit path's product: out = x . w^T with w [N, K], or one per head with w [H, N, K] (see gemm_f32_heads).  A row of out
-    depends on its row of x alone, whatever lies beside it."""
+    depends on its row of x alone, whatever lies beside it.  ``constant_w``: see gemm_f32_tc."""
     if w.shape[-1] >= F32_CUT_COLUMNS:
-        gemm_f32_tc(x, w, out)
+        gemm_f32_tc(x, w, out, constant_w=constant_w)
     elif w.dim() == 3:
         gemm_f32_heads(x, w, out)
     else:

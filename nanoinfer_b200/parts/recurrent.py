@@ -192,7 +192,7 @@ class GatedDeltaRule(Part):
         x = proj[:, col0 + self.thin_col:col0 + self.thin_col + self.thin_k]
         if rt.dtype == torch.float32:
             z = rt.empty(n, self.w_thin.shape[0])
-            ops.linear_f32(x, self.w_thin.view(1, *self.w_thin.shape), z)
+            ops.linear_f32(x, self.w_thin.view(1, *self.w_thin.shape), z, constant_w=True)
             return z
         if x.dtype != torch.bfloat16 or rt.skinny(n, self.thin_k):
             x = x.to(torch.bfloat16).contiguous()

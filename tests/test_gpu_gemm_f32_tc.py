@@ -177,6 +177,19 @@ def test_what_is_not_finite_or_overflows_in_between(rows, splits):
     assert bool(((got.double() - want).abs()[fine] <= _bound(k, total)[fine]).all())
 
 
+def test_rows_that_a_chain_takes_or_refuses():
+    """One product's x is contiguous whatever its length; the strides of a single row do not matter."""
+    from nanoinfer_b200.kernels import ops
+    w = _randn(140, 1024, seed=18)
+    with pytest.raises(ops.KernelError, match="contiguous"):
+        ops.linear_f32(_randn(5, 1040, seed=19)[:, :1024], w, torch.empty(5, 140, device=DEV))
+    column = _randn(1024, 1, seed=20)
+    out, want = torch.empty(1, 140, device=DEV), torch.empty(1, 140, device=DEV)
+    ops.linear_f32(column.t(), w, out)                # [1, 1024], strides 1 and 1
+    ops.linear_f32(column.view(1, 1024), w, want)
+    assert torch.equal(out, want)
+
+
 def test_a_rule_by_the_length_of_a_row_alone():
     from nanoinfer_b200.kernels import ops
     for k in (1020, 1024):

@@ -139,3 +139,26 @@ def test_blocks_that_only_ask_for_weights_hold_nobody_up(cluster):
     (128, 20, [300], False), (64, 128, [300], False), (256, 128, [300], False)])
 def test_the_delta_rule_goes_by_tiles_where_they_are_done_first(dim, vdim, lens, tiles):
     assert ops.delta_tile_pays(sum(lens), len(lens), dim, vdim) == tiles
+
+
+def test_only_constant_weights_are_read_ahead_of_the_kernel_in_front(monkeypatch):
+    """A product by itself takes any w, the work of the kernel in front included; the runtime's weights are constant."""
+    import torch
+
+    from nanoinfer_b200.engine.runtime import Runtime
+    asked = []
+    monkeypatch.setattr(ops, "load", lambda module: SimpleNamespace(ni_gemm_f32_tc=lambda *a: asked.append(a[10]) or 0))
+    monkeypatch.setattr(ops, "_dev", lambda t, name, dtype=None: t.data_ptr())
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "_error_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(ops, "_heads_of", lambda x, w, out, what: (x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), 3, 8, 1024, 2))
+    x, w, out = torch.zeros(3, 1024), torch.zeros(8, 1024), torch.zeros(3, 8)
+    ops.linear_f32(x, w, out)
+    ops.linear_f32(torch.zeros(3, 2048), torch.zeros(2, 8, 1024), torch.zeros(3, 16))
+    ops.gemm_f32_tc(x, w, out)
+    assert asked == [0, 0, 0]
+    rt = object.__new__(Runtime)
+    rt.dtype, rt.device = torch.float32, torch.device("cpu")
+    rt.linear(x, w)
+    rt.heads_linear(torch.zeros(3, 2048), torch.zeros(2, 8, 1024))
+    assert asked[3:] == [1, 1]
