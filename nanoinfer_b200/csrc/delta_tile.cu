@@ -19,10 +19,12 @@
 // lone warp per scheduler, which issues nothing else for 8 clocks while one of its 162 MMAs enters the tensor core.  (Four warps per 16
 // columns: 148 us instead of 129 at the time, since their products come in the same phases; FP32 multiply-adds in the same tiles: 183 us.)
 //
-// Portions of 1,201 and 847 tokens, 16 heads of 128: 171 us with the preparation (51), against 247 us in blocks of four; 2,048 tokens 248
-// (338), 8 x 512 261 (330), 512 71 (91).  Error against 64 bits of the whole rule, read-outs / states, means over six inputs: decays of a
-// few tokens 1.3e-7 / 1.4e-7 (blocks of four 1.3e-7 / 1.3e-7), of some tens 1.7e-7 / 2.2e-7 (1.9e-7 / 2.7e-7), decays near one 1.1e-6 /
-// 2.0e-6 (1.1e-6 / 2.0e-6: the decays' own rounding).
+// Portions of 1,201 and 847 tokens, 16 heads of 128: 178 us with the preparation (53), against 251 us in blocks of four; 2,048 tokens 255
+// (342), 8 x 512 269 (335), 512 75 (94).  Error against 64 bits of the whole rule, read-outs / states, means over eight inputs of up to
+// 1,100 tokens: decays of a few tokens 1.2e-7 / 1.1e-7 (blocks of four 1.3e-7 / 1.2e-7), of some tens 1.1e-7 / 1.2e-7 (1.4e-7 / 1.5e-7),
+// of some hundreds 1.3e-7 / 1.5e-7 (3.0e-7 / 4.5e-7), decays near one 1.6e-7 / 1.8e-7 (1.7e-6 / 2.7e-6).  Decays and beta in 64 bits and
+// the keys' norms with one step of Newton's method are worth more than what the cuts cost (in FP32: states 1.07 times the error of
+// blocks of four where a decay lasts a few tokens); they take 2 us.
 #include <type_traits>
 
 #include "common.cuh"
@@ -44,7 +46,13 @@ struct DtDims {
 };
 
 __device__ __forceinline__ float dt_silu(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dt_softplus(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
+__device__ __forceinline__ double dt_softplus(double z) { return z > 20.0 ? z : log1p(exp(z)); }
+// 1 / sqrt(s): the error of the division and the root (a factor of all of a row's numbers) is put right by one step of Newton's method
+// whose residual is exact.
+__device__ __forceinline__ float dt_rsqrt(float s) {
+    const float r = 1.0f / sqrtf(s), h = s * r, left = fmaf(-h, r, 1.0f) - fmaf(s, r, -h) * r;
+    return fmaf(0.5f * r, left, r);
+}
 
 // Tiles before request `seq` (all of a warp's lanes get it).
 __device__ __forceinline__ int dt_tiles_before(const int* __restrict__ cu_q, int seq) {
@@ -194,7 +202,7 @@ delta_tile_prepare_kernel(const T* __restrict__ proj, const float* __restrict__ 
         dt_conv<T, TAPS>(proj, conv_w, hist, dm, first, at, live, c, y);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            const float r = (1.0f / sqrtf(ni_warp_sum(dt_dot4(y[t], y[t], 0.f)) + 1e-6f)) * (which ? 1.0f : 1.0f / sqrtf((float)DT_D));
+            const float r = dt_rsqrt((ni_warp_sum(dt_dot4(y[t], y[t], 0.f)) + 1e-6f) * (which ? 1.0f : (float)DT_D));
             y[t].x *= r; y[t].y *= r; y[t].z *= r; y[t].w *= r;
             *reinterpret_cast<float4*>(which ? &ks[4 * warp + t][4 * lane] : &qs[4 * warp + t][4 * lane]) = y[t];
         }
@@ -242,20 +250,21 @@ delta_tile_prepare_kernel(const T* __restrict__ proj, const float* __restrict__ 
     __syncthreads();
     const int per = dm.H / dm.G, j = lane & 15;
     for (int h = g * per + warp; h < (g + 1) * per; h += 4) {
-        float decay = 1.f, beta = 0.f;                         // lane t < 16: token t's
+        // lane t < 16: token t's decay and beta, in 64 bits: their errors are factors of all of the state
+        double decay = 1.0, beta = 0.0;
         if (lane < DT_TOK && lane < left) {
             const T* row = proj + (size_t)(first + tile0 + lane) * dm.ld;
-            decay = expf(-expf(a_log[h]) * dt_softplus(ni_to_float(row[dm.a_off + h]) + dt_bias[h]));
-            beta = 1.0f / (1.0f + expf(-ni_to_float(row[dm.b_off + h])));
+            decay = exp(-exp((double)a_log[h]) * dt_softplus((double)ni_to_float(row[dm.a_off + h]) + (double)dt_bias[h]));
+            beta = 1.0 / (1.0 + exp(-(double)ni_to_float(row[dm.b_off + h])));
         }
         uint8_t* o = coef + ((size_t)blockIdx.x * dm.H + h) * DT_COEF;
         float* vec = reinterpret_cast<float*>(o + 4 * DT_PIECE);
-        // lane j (and j + 16): column j of A and L, running down the tokens; c and P(15, .) on the way.  Products of decays are
-        // kept in 64 bits: their error is common to all of the state, so that it would not average out along a portion.
+        // lane j (and j + 16): column j of A and L, running down the tokens; c and P(15, .) on the way.  Products of decays stay in
+        // 64 bits, since their error would not average out along a portion.
         double p = 1.0, c = 1.0, ct = 1.0;
 #pragma unroll
         for (int t = 0; t < DT_TOK; ++t) {
-            const float dt = __shfl_sync(0xffffffffu, decay, t), bt = __shfl_sync(0xffffffffu, beta, t);
+            const double dt = __shfl_sync(0xffffffffu, decay, t), bt = __shfl_sync(0xffffffffu, beta, t);
             c *= dt;
             if (t == j) ct = c;
             p = t > j ? p * dt : 1.0;
@@ -275,7 +284,7 @@ delta_tile_prepare_kernel(const T* __restrict__ proj, const float* __restrict__ 
                 x[t] = t == j ? 1.f : t > j ? -a : 0.f;
                 ts[warp][t][j] = t > j ? x[t] : 0.f;
             }
-            vec[j] = beta;
+            vec[j] = (float)beta;
             vec[16 + j] = (float)(beta * ct);
             vec[32 + j] = (float)ct;
             vec[48 + j] = (float)p;                            // P(15, j)

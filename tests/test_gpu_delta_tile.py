@@ -74,19 +74,22 @@ def _in_64_bits(x):
     return torch.stack(want), torch.stack(ends)
 
 
-@pytest.mark.parametrize("fast", [-4.0, -1.0, 2.0])
-def test_errors_against_64_bits_stay_where_they_were(fast):
-    """Read-outs and states no further from 64 bits than in blocks of four, but for what differs from input to input: the last states
-    are those of 12 heads, whose errors have a spread of a tenth or two of their mean."""
+@pytest.mark.parametrize("lens", [[200, 130, 70], [1100]])
+@pytest.mark.parametrize("fast", [-6.0, -4.0, -1.0, 2.0, 4.0])
+def test_errors_against_64_bits_stay_where_they_were(fast, lens):
+    """Read-outs and states no further from 64 bits than in blocks of four, in the mean over four inputs: decays near one, whose own
+    errors add up along a long portion, to decays of a token or two, where every product's rounding shows."""
     from nanoinfer_b200.kernels import ops
-    x = _inputs(4, 4, 64, 4, [200, 130, 70], fast, 5)
-    want, ends = _in_64_bits(x)
-    errors = []
-    for tiles in (True, False):
-        out, state = _tiles(ops, x, tiles)
-        end = state[x["slots"].long(), :4 * 128 * 64].double()
-        errors.append((((out - want).norm() / want.norm()).item(), ((end - ends).norm() / ends.norm()).item()))
-    assert all(a <= 1.25 * b for a, b in zip(*errors)), errors
+    sums = {True: [0.0, 0.0], False: [0.0, 0.0]}
+    for seed in range(4):
+        x = _inputs(4, 4, 64, 4, lens, fast, 100 + seed)
+        want, ends = _in_64_bits(x)
+        for tiles, at in sums.items():
+            out, state = _tiles(ops, x, tiles)
+            end = state[x["slots"].long(), :4 * 128 * 64].double()
+            at[0] += ((out - want).norm() / want.norm()).item()
+            at[1] += ((end - ends).norm() / ends.norm()).item()
+    assert all(a <= b for a, b in zip(sums[True], sums[False])), sums
 
 
 def test_refused_and_chosen():
