@@ -7,7 +7,7 @@ missing CUDA library or a tensor on the CPU is an error, never a fallback.
 from __future__ import annotations
 
 import ctypes
-from typing import Dict, Optional
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -743,20 +743,39 @@ def delta_block_pays(n_tokens: int, n_seqs: int, max_q_len: int, n_heads: int, d
         (n_tokens >= 8 * n_seqs and (max_q_len >= 26 or n_seqs * size >= full))
 
 
-def delta_tile_pays(n_tokens: int, n_seqs: int, dim: int, vdim: int) -> bool:
+def delta_tile_pays(n_tokens: int, n_seqs: int, dim: int, vdim: int, n_heads: int = 16, max_q_len: Optional[int] = None) -> bool:
     """Whether delta_block_recurrence takes sixteen tokens at a time (csrc/delta_tile.cu: key heads of 128, value heads a multiple of
-    16): a request costs whole tiles however few its tokens are.  us in blocks of four / in tiles, 16 heads of 128: a portion of 64
-    21.9 / 22.2, four of 32 22.1 / 22.6, three of 100 42.2 / 37.3, 32 of 16 59.2 / 51.5, 16 of 8 27.5 / 32.0; 256 beside 64 single tokens 87 /
-    105, 512 beside 200 207 / 282, 1,024 beside 200 296 / 308."""
-    return dim == 128 and vdim % 16 == 0 and n_tokens >= 192 and n_tokens >= 16 * n_seqs
+    16).  ``max_q_len``: the longest portion (None: the mean).  A request costs whole tiles however few its tokens are, and tiles take 4 us more
+    to start, which portions of 96 tokens win back, or enough work for all SMs.  us in blocks of four / in tiles, 16 heads of 128 unless
+    said: a portion of 64 25.6 / 26.5, three of 100 44 / 43, eight of 32 36 / 34, 16 of 16 37.9 / 39.1, 32 of 16 61 / 58, 256 beside 40 single
+    tokens 78 / 79; 4 heads, eight of 32 20.7 / 23.4, 32 of 16 27.5 / 29.8.  With many heads a single token's tile costs 4.8 us (64 heads), a block
+    2.7, and nothing hides it behind a long portion: 64 heads, 512 beside 31 260 / 284, 1,024 beside 63 508 / 567, but 16 of 16 116 / 102;
+    32 heads, 1,024 beside 63 350 / 286."""
+    size = n_heads * vdim / 2048                               # the work of a token, in 16 heads of 128
+    longest = n_tokens / max(n_seqs, 1) if max_q_len is None else max_q_len
+    short = n_seqs > 1 and n_tokens - longest < 8 * (n_seqs - 1)           # what lies beside the longest portion: fewer than eight tokens each
+    return dim == 128 and vdim % 16 == 0 and n_tokens >= 192 and n_tokens >= 16 * n_seqs and \
+        (longest >= 96 or n_tokens * size >= 256) and (not short or n_tokens >= 8 * size * n_seqs)
+
+
+def delta_tile_bytes(n_tokens: int, n_seqs: int, n_q_heads_kv: int, n_heads: int, vdim: int) -> Tuple[int, int, int]:
+    """Bytes of what delta_block_recurrence keeps in its buffer between the two kernels of tiles: values, keys, coefficients."""
+    lib = load("delta_tile")
+    sizes = []
+    for name, args in (("values", (n_tokens, n_heads, vdim)), ("keys", (n_tokens, n_seqs, n_q_heads_kv)), ("coefs", (n_tokens, n_seqs, n_heads))):
+        f = getattr(lib, "ni_delta_tile_" + name)
+        f.restype, f.argtypes = _LL, [_I] * 3
+        sizes.append(-(-f(*args) // 512) * 512)
+    return tuple(sizes)
 
 
 def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, state, cu_q, slots, n_seqs, n_q_heads_kv, n_heads, dim,
-                           vdim, taps, out, tiles: Optional[bool] = None) -> None:
+                           vdim, taps, out, tiles: Optional[bool] = None, buf: Optional[torch.Tensor] = None) -> None:
     """What delta_prepare and delta_recurrence do with a decay per head, four tokens at a time (FP32 throughout; another
     order of sums) or sixteen (``tiles``; None: where delta_tile_pays; FP32 numbers cut in three for the tensor cores):
     ``proj`` [T, *] float32 or bfloat16, q | k | v from column ``col0`` on, the logits of beta and of the decay at ``b_col`` and
-    ``a_col``.  delta_gated_norm must follow (it moves the convolution history on)."""
+    ``a_col``.  ``buf``: for tiles, at least delta_tile_bytes bytes on the device (default: allocated here).  delta_gated_norm must
+    follow (it moves the convolution history on)."""
     f32, i32 = torch.float32, torch.int32
     n = proj.shape[0]
     c = 2 * n_q_heads_kv * dim + n_heads * vdim
@@ -764,21 +783,23 @@ def delta_block_recurrence(proj, col0, b_col, a_col, conv_w, a_log, dt_bias, sta
             proj.shape[1] < max(col0 + c, b_col + n_heads, a_col + n_heads) or min(b_col, a_col) < col0 or \
             state.shape[1] != n_heads * dim * vdim + (taps - 1) * c or cu_q.numel() != n_seqs + 1 or slots.numel() != n_seqs:
         raise KernelError("delta_block_recurrence: shapes do not agree")
-    if delta_tile_pays(n, n_seqs, dim, vdim) if tiles is None else tiles:
+    if delta_tile_pays(n, n_seqs, dim, vdim, n_heads) if tiles is None else tiles:
         if dim != 128:
             raise KernelError("delta_block_recurrence: sixteen tokens at a time are for key heads of 128")
         lib = load("delta_tile")
-        sizes = []
-        for name, args in (("values", (n, n_heads, vdim)), ("keys", (n, n_seqs, n_q_heads_kv)), ("coefs", (n, n_seqs, n_heads))):
-            f = getattr(lib, "ni_delta_tile_" + name)
-            f.restype, f.argtypes = _LL, [_I] * 3
-            sizes.append(f(*args))
-        values, keys, coef = (torch.empty(b, dtype=torch.uint8, device=proj.device) for b in sizes)
+        sizes = delta_tile_bytes(n, n_seqs, n_q_heads_kv, n_heads, vdim)
+        if buf is None:
+            buf = torch.empty(sum(sizes), dtype=torch.uint8, device=proj.device)
+        elif buf.numel() * buf.element_size() < sum(sizes):
+            raise KernelError("delta_block_recurrence: the buffer is too small")
+        values = _dev(buf, "buf")
+        keys = values + sizes[0]
+        coef = keys + sizes[1]
         _check(lib.ni_delta_tile(
             _dev(proj, "proj") + col0 * proj.element_size(), _code(proj, "proj"), _dev(conv_w, "conv_w", f32), _dev(a_log, "a_log", f32),
             _dev(dt_bias, "dt_bias", f32), _dev(state, "state", f32), state.shape[1], _dev(cu_q, "cu_q", i32), _dev(slots, "slots", i32), n,
-            n_seqs, n_q_heads_kv, n_heads, vdim, taps, proj.shape[1], b_col - col0, a_col - col0, values.data_ptr(), keys.data_ptr(),
-            coef.data_ptr(), _dev(out, "out", f32), _stream()), "delta_block_recurrence")
+            n_seqs, n_q_heads_kv, n_heads, vdim, taps, proj.shape[1], b_col - col0, a_col - col0, values, keys, coef,
+            _dev(out, "out", f32), _stream()), "delta_block_recurrence")
         return
     qkv = torch.empty(n, c, dtype=f32, device=proj.device)
     lib = load("delta_block")

@@ -221,8 +221,11 @@ class GatedDeltaRule(Part):
                                        ctx.cu_q, ctx.slots, ctx.n_seqs, ctx.max_q_len, g, h, d, v, self.taps, buf, o)
         elif self.in_blocks and ops.delta_block_takes(proj, col0, cache.state) and \
                 ops.delta_block_pays(n, ctx.n_seqs, ctx.max_q_len, h, d, v):
+            tiles, buf = ops.delta_tile_pays(n, ctx.n_seqs, d, v, h, ctx.max_q_len), None
+            if tiles:
+                buf = rt.workspace("delta_tiles", sum(ops.delta_tile_bytes(n, ctx.n_seqs, g, h, v)), torch.uint8)  # one buffer for all layers
             ops.delta_block_recurrence(proj, col0, col0 + self.b_col, col0 + self.b_col + h, self.conv_w, self.a_log, self.dt_bias,
-                                       cache.state, ctx.cu_q, ctx.slots, ctx.n_seqs, g, h, d, v, self.taps, o)
+                                       cache.state, ctx.cu_q, ctx.slots, ctx.n_seqs, g, h, d, v, self.taps, o, tiles=tiles, buf=buf)
         else:
             qkv = rt.empty(n, self.channels, dtype=f32)
             gates = rt.empty(n, h, 2, dtype=f32)

@@ -104,6 +104,41 @@ def test_refused_and_chosen():
     assert torch.equal(_tiles(ops, x)[0], _tiles(ops, x, tiles=None)[0])
 
 
+def test_a_buffer_of_the_caller_s_gives_the_same_bits():
+    from nanoinfer_b200.kernels import ops
+    x = _inputs(2, 4, 48, 4, [33, 180, 7], -2.0, 8)
+    want, want_state = _tiles(ops, x)
+    need = sum(ops.delta_tile_bytes(x["n"], x["n_seqs"], 2, 4, 48))
+    buf = torch.full((need + 64,), 255, dtype=torch.uint8, device=DEV)       # (NaN wherever it is read before it is written)
+    state, out = x["state"].clone(), torch.empty_like(want)
+    args = (x["proj"], 0, x["b_col"], x["a_col"], x["conv_w"], x["a_log"], x["dt_bias"], state, x["cu"], x["slots"], x["n_seqs"], 2, 4, 128, 48, 4, out)
+    with pytest.raises(ops.KernelError, match="too small"):
+        ops.delta_block_recurrence(*args, tiles=True, buf=buf[:need - 1])
+    ops.delta_block_recurrence(*args, tiles=True, buf=buf)
+    assert torch.equal(out, want) and torch.equal(state, want_state) and (buf[need:] == 255).all()
+
+
+def test_layers_and_captured_steps_share_one_buffer():
+    """The part takes its scratch from the runtime: a second call, or another layer's, allocates none."""
+    import types
+
+    from nanoinfer_b200.kernels import ops
+    from nanoinfer_b200.parts.recurrent import GatedDeltaRule
+    x = _inputs(2, 2, 32, 4, [200, 60], -2.0, 9, torch.bfloat16)
+    asked = []
+    rt = types.SimpleNamespace(dtype=torch.bfloat16, empty=lambda *s, dtype=None: torch.zeros(s, device=DEV, dtype=dtype or torch.bfloat16),
+                               workspace=lambda name, n, dtype, zero=False: asked.append((name, n)) or torch.empty(n, dtype=dtype, device=DEV))
+    part = object.__new__(GatedDeltaRule)
+    part.__dict__.update(rt=rt, G=2, H=2, D=128, V=32, taps=4, channels=x["C"], b_col=x["b_col"], gate_col=0, wants_f32_tokens=False, w_thin=None,
+                         channel=False, chunked=False, in_blocks=True, thin_gate=False, conv_w=x["conv_w"], a_log=x["a_log"], dt_bias=x["dt_bias"],
+                         norm_w=torch.ones(32, device=DEV), eps=1e-6, output_scale=1.0)
+    ctx = types.SimpleNamespace(max_q_len=200, n_seqs=2, cu_q=x["cu"], slots=x["slots"], seq_of_token=x["seq"])
+    out = torch.empty(260, 64, dtype=torch.bfloat16, device=DEV)
+    for _ in range(2):
+        part.between(x["proj"], 0, ctx, types.SimpleNamespace(state=x["state"].clone()), out)
+    assert asked == [("delta_tiles", sum(ops.delta_tile_bytes(260, 2, 2, 2, 32)))] * 2
+
+
 @pytest.mark.parametrize("poison", [float("inf"), float("nan")])
 @pytest.mark.parametrize("what", ["value", "key", "query", "beta", "decay"])
 def test_what_is_not_finite_stays_with_its_own_and_later_tokens(poison, what):

@@ -139,6 +139,15 @@ def test_blocks_that_only_ask_for_weights_hold_nobody_up(cluster):
     (128, 20, [300], False), (64, 128, [300], False), (256, 128, [300], False)])
 def test_the_delta_rule_goes_by_tiles_where_they_are_done_first(dim, vdim, lens, tiles):
     assert ops.delta_tile_pays(sum(lens), len(lens), dim, vdim) == tiles
+    assert ops.delta_tile_pays(sum(lens), len(lens), dim, vdim, 16, max(lens)) == tiles
+
+
+@pytest.mark.parametrize("heads, lens, tiles", [
+    (4, [32] * 8, False), (4, [16] * 32, False), (4, [100] * 3, True), (4, [256] + [1] * 15, True), (4, [128] * 8, True), (8, [16] * 16, False), (8, [16] * 32, True),
+    (16, [32] * 8, True), (32, [256] + [1] * 15, True), (32, [1024] + [1] * 63, True), (64, [256] + [1] * 15, False), (64, [512] + [1] * 31, False),
+    (64, [1024] + [1] * 63, False), (64, [16] * 16, True), (64, [512] * 8, True), (64, [2048], True)])
+def test_tiles_are_weighed_with_the_heads_and_the_longest_portion(heads, lens, tiles):
+    assert ops.delta_tile_pays(sum(lens), len(lens), 128, 128, heads, max(lens)) == tiles
 
 
 def test_only_constant_weights_are_read_ahead_of_the_kernel_in_front(monkeypatch):
