@@ -434,11 +434,14 @@ struct ScScratch {
 // value that the largest tokens of at least k threads reach (few threads have two of the k) the block sends its tokens to the
 // cluster's first block, which finds the k-th largest, the top-p floor and the draw among those alone - with the same keys, the
 // same 64-bit masses and the same rules, so the same token.  (Before, every token was counted by the leading 12 bits of its key while
-// it was loaded: 32 shared-memory additions per thread instead of one, and half again as many candidates.)  A slice with fewer than
-// four tokens per thread counts them all.  A slice with more than SC_CANDIDATES tokens from its coarse value on (a large k, rows of
-// equal logits), or fewer than k threads with a finite token, sends the whole row down the general path below.
+// it was loaded: 32 shared-memory additions per thread instead of one, and half again as many candidates.)  Of 512 threads' largest
+// tokens the k largest leave about 512 ln(512 / (512 - k)) of the slice's from the k-th on, 423 for k = 288 but all 504 for k = 320: with
+// a larger k than 9/16 of the threads every token is counted that is no less than the least of the threads' largest (at least 512
+// are; under a fifth of the slice), so that little more than k go.  A slice with fewer than four tokens per thread counts them all.  A
+// slice with more than SC_CANDIDATES tokens from its coarse value on (a k near 504, rows of equal logits), or fewer than k threads with a
+// finite token, sends the whole row down the general path below.
 // 8 rows of 128,256 logits, top-k 50 and top-p 0.9: 14.3 us (21.2 as above), against 102 us as eleven passes of the cluster over the
-// row; k = 200 21.7 (27.0); 64 rows, k = 50 40.6 (49.6).
+// row; k = 200 21.7 (27.0), 350 35.3 (105 with the threads' largest alone), 500 37.3 (106); 64 rows, k = 50 40.6 (49.6).
 #define SC_COARSE 4096
 // The coarse value of a number: -1 below `lo`.  (Monotonic in v, which is all that counts.)
 struct ScScale {
@@ -904,7 +907,11 @@ sample_cluster_kernel(const float* __restrict__ logits, int* __restrict__ out, c
         };
         if (top < INFINITY) {                                // (an infinite or NaN logit: nothing counted, so the general path)
             if (sparse) {
-                count(z[largest_at]);
+                if (k <= SC_THREADS * 9 / 16) {
+                    count(z[largest_at]);
+                } else {
+                    for (int i = tid; i < n; i += SC_THREADS) count(z[i]);       // (those below s.low[0] are none)
+                }
             } else {
                 for (int i = tid; i < n; i += blockDim.x) count(z[i]);
             }

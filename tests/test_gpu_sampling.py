@@ -270,3 +270,62 @@ def test_parameters_that_travel_with_the_launch(rows, vocab, taken):
     assert not taken or torch.equal(out, want)
     assert torch.equal(sampler.sample(l, params, seeds, at), want)
     assert sampler.h2d_bytes == 2 * 28 * rows
+
+
+def _sample_us(logits, k, top_p=0.9):
+    """Microseconds of one call, by itself in a graph of twenty."""
+    from nanoinfer_b200.kernels import ops
+    n = logits.shape[0]
+    out = torch.empty(n, dtype=torch.int32, device=DEV)
+    rows = torch.arange(n, dtype=torch.int64, device=DEV)
+    args = (torch.full((n,), 0.8, device=DEV), torch.full((n,), k, dtype=torch.int32, device=DEV), torch.full((n,), top_p, device=DEV), rows, rows)
+    ops.sample(logits, out, *args)
+    graph, start, end = torch.cuda.CUDAGraph(), torch.cuda.Event(True), torch.cuda.Event(True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        for _ in range(20):
+            ops.sample(logits, out, *args)
+    times = []
+    for _ in range(4):
+        start.record()
+        graph.replay()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(end) * 50)
+    return min(times)
+
+
+@pytest.mark.parametrize("spread", ["normal", "uniform"])
+def test_a_large_k_stays_with_the_candidates(spread):
+    """Up to a k near what a slice can send, a row goes by its candidates: 8 rows of 128,256 take 35 to 43 us for k = 320 to 490, where
+    passes over the row take 103 to 130."""
+    g = torch.Generator().manual_seed(3)
+    l = (torch.randn(8, 128256, generator=g) * 3 if spread == "normal" else torch.rand(8, 128256, generator=g) * 10).to(DEV)
+    passes = _sample_us(l, 600)                      # more than a slice can send
+    for k in (289, 320, 350, 400, 490):
+        assert _sample_us(l, k) < 0.6 * passes, k
+
+
+@pytest.mark.parametrize("k", [288, 289, 320, 400, 490, 504, 505])
+@pytest.mark.parametrize("vocab", [16384, 50257, 128256])
+def test_a_large_k_draws_the_same_tokens(vocab, k):
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(k)
+    l = torch.randn(8, vocab, generator=g) * 3
+    l[1] = (l[1] * 2).round() / 2                    # ties
+    l[2] = torch.rand(vocab, generator=g)
+    l[3, torch.randperm(vocab, generator=g)[: vocab - 450]] = -float("inf")          # fewer tokens than k, or little more
+    l[4, : vocab // 8] += 30.0                       # all in the first block's slice
+    l[5, 7] = 1e30
+    l[6] = l[6].abs().neg()
+    l = l.to(DEV)
+    rows = torch.arange(8, dtype=torch.int64, device=DEV)
+    for p in (0.9, 1.0):
+        outs = []
+        for cluster in (True, False):
+            ops.sample_by_cluster(cluster)
+            out = torch.full((8,), -1, dtype=torch.int32, device=DEV)
+            ops.sample(l, out, torch.full((8,), 0.9, device=DEV), torch.full((8,), k, dtype=torch.int32, device=DEV), torch.full((8,), p, device=DEV), rows, rows)
+            outs.append(out.tolist())
+        ops.sample_by_cluster(True)
+        assert outs[0] == outs[1], p
