@@ -582,10 +582,12 @@ __device__ uint32_t sc_mass_select(const unsigned long long* list, int n, uint32
 
 // The first block's part: list [SC_RANKS][SC_CANDIDATES] of (key << 32) | id, counts[2 c + 1] of them per block.  The candidates are
 // counted by coarse value once more: those above the value of the k-th largest stay, those of that value (a few) are compared with
-// one another - or, if they are many, all go by passes over their bits.  Up to SC_PAIRS tokens that stay are compared with one
-// another; more (ties at the k-th place: up to 4,032 stay) go by passes over their bits.
+// one another - or, if they are more than the threads, all go by passes over their bits - unless they are one number, which ties are.
+// Up to SC_PAIRS tokens that stay are compared with one another; more (ties at the k-th place: up to 4,032 stay) go by passes over
+// their bits.
 // 8 rows, k = 50, top-p 0.9, us now / every candidate by passes over its bits / as passes of the cluster over the row: without ties
-// 14.3 / 21.2 / 102; 128 tied at the k-th place 22.6 / 28.8 / 178, 480 49.3 / 47.9 / 179, 1,024 63 / 60.5 / 182, 3,920 107 / 94 / 197.
+// 14.4 / 21.3 / 102; 128 tied at the k-th place 20.8 / 25.6 / 178, 480 52.2 / 58.7 / 179, 1,024 71.2 / 74.1 / 182, 3,920 126 / 128 / 197;
+// without top-p 480 22.7 / 27.4, 3,920 90 / 91.  (One number looked for among fewer than 256: 128 tied 21.2.)
 __device__ void sc_pick(unsigned long long* list, const unsigned long long* counts, uint32_t* work, ScScratch& s, float m, int k, float p,
                         unsigned long long seed, unsigned long long counter, int* out) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -635,7 +637,22 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
     const int from = max(0, (int)s.digit_rest[0]), tied = (int)work[from], rest = k - ((int)s.digit_rest[1] - tied);       // of `tied`, `rest` stay
     uint32_t* same = reinterpret_cast<uint32_t*>(s.hist);    // the keys of that value, if they are no more than the block's threads
     uint32_t key_floor = 0u;
-    if (tied <= SC_THREADS) {
+    bool equal = false;                                      // all of that value are one number: they stay
+    if (tied > SC_PAIRS) {
+        bool alike = true;
+#pragma unroll
+        for (int u = 0; u < EACH; ++u)
+            if (u * SC_THREADS < sent && have >> u & 1 && coarse(mine[u]) == from) same[0] = (uint32_t)(mine[u] >> 32);        // (any of them)
+        __syncthreads();
+        const uint32_t one = same[0];
+#pragma unroll
+        for (int u = 0; u < EACH; ++u)
+            if (u * SC_THREADS < sent && have >> u & 1 && coarse(mine[u]) == from) alike = alike && (uint32_t)(mine[u] >> 32) == one;
+        equal = __syncthreads_and(alike);
+    }
+    if (equal) {
+        // nothing to find
+    } else if (tied <= SC_THREADS) {
 #pragma unroll
         for (int u = 0; u < EACH; ++u)
             if (u * SC_THREADS < sent && have >> u & 1 && coarse(mine[u]) == from)
@@ -648,10 +665,18 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
         for (int shift = 24; shift >= 0; shift -= 8) {
             if (tid < 256) bins[tid] = 0u;
             __syncthreads();
-            for (int i = tid; i < SLOTS; i += blockDim.x) {
-                if ((unsigned long long)(i % SC_CANDIDATES) >= counts[2 * (i / SC_CANDIDATES) + 1]) continue;
-                const uint32_t key = (uint32_t)(list[i] >> 32);
-                if ((key & mask) == prefix) atomicAdd(&bins[(key >> shift) & 255u], 1u);
+#pragma unroll
+            for (int u = 0; u < EACH; ++u) {
+                if (u * SC_THREADS >= sent) continue;
+                const uint32_t key = (uint32_t)(mine[u] >> 32), bin = (key >> shift) & 255u;
+                const bool in = (have >> u & 1) && (key & mask) == prefix;
+                const unsigned who = __ballot_sync(0xffffffffu, in);
+                const uint32_t first = __shfl_sync(0xffffffffu, bin, who ? __ffs(who) - 1 : 0);
+                if (__all_sync(0xffffffffu, !in || bin == first)) {
+                    if (lane == 0 && who) atomicAdd(&bins[first], (uint32_t)__popc(who));
+                } else if (in) {
+                    atomicAdd(&bins[bin], 1u);
+                }
             }
             __syncthreads();
             if (warp == 0) {                                 // lane l holds bins 8 l .. 8 l + 7
@@ -683,8 +708,8 @@ __device__ void sc_pick(unsigned long long* list, const unsigned long long* coun
         if (u * SC_THREADS >= sent || !(have >> u & 1)) continue;
         const uint32_t key = (uint32_t)(mine[u] >> 32);
         const int value = coarse(mine[u]);
-        bool stays = tied <= SC_THREADS ? value > from : key >= key_floor;
-        if (tied <= SC_THREADS && value == from) {           // fewer than `rest` of its value are larger
+        bool stays = equal ? value >= from : tied <= SC_THREADS ? value > from : key >= key_floor;
+        if (!equal && tied <= SC_THREADS && value == from) {           // fewer than `rest` of its value are larger
             int larger = 0;
             for (int j = 0; j < tied; ++j) larger += same[j] > key;
             stays = larger < rest;

@@ -329,3 +329,29 @@ def test_a_large_k_draws_the_same_tokens(vocab, k):
             outs.append(out.tolist())
         ops.sample_by_cluster(True)
         assert outs[0] == outs[1], p
+
+
+@pytest.mark.parametrize("tied", [40, 256, 257, 300, 511, 512, 513, 700, 2000, 3900])
+@pytest.mark.parametrize("others", [0, 3])
+def test_tokens_of_one_value_at_the_k_th_place(tied, others):
+    """All of the k-th's coarse value are one number (they stay unlooked at), or a few beside them differ in their last bits."""
+    from nanoinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(tied)
+    l = torch.randn(4, 128256, generator=g)
+    for r in range(4):
+        at = torch.randperm(128256, generator=g)
+        l[r, at[:30]] = 9.0 + torch.rand(30, generator=g)
+        l[r, at[30:30 + tied]] = 8.0
+        for i in range(others):
+            l[r, at[100 + tied + i]] = torch.nextafter(torch.tensor(8.0), torch.tensor(9.0 if i % 2 else 7.0)).item()
+    l = l.to(DEV)
+    rows = torch.arange(4, dtype=torch.int64, device=DEV)
+    for p in (0.95, 1.0):
+        outs = []
+        for cluster in (True, False):
+            ops.sample_by_cluster(cluster)
+            out = torch.full((4,), -1, dtype=torch.int32, device=DEV)
+            ops.sample(l, out, torch.full((4,), 1.5, device=DEV), torch.full((4,), 50, dtype=torch.int32, device=DEV), torch.full((4,), p, device=DEV), rows, rows)
+            outs.append(out.tolist())
+        ops.sample_by_cluster(True)
+        assert outs[0] == outs[1], p
