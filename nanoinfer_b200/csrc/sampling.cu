@@ -1143,11 +1143,13 @@ template <typename ARGS>
 static int sc_launch(const float* logits, int* out, const ARGS& args, int n_rows, int vocab, cudaStream_t stream) {
     const int slice = sc_slice(vocab);
     const size_t sc_smem = (size_t)slice * sizeof(float) + (size_t)(SC_HISTS + 2 * SC_RANKS) * 256 * sizeof(unsigned long long);
-    static size_t sc_configured = 0;
-    if (sc_configured < sc_smem) {
+    static size_t configured[64];                            // what each device allows so far
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
+    if (dev >= 64 || configured[dev] < sc_smem) {
         cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel<ARGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc_smem);
         if (e != cudaSuccess) return (int)e;
-        sc_configured = sc_smem;
+        if (dev < 64) configured[dev] = sc_smem;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_rows * SC_RANKS);
