@@ -29,7 +29,7 @@ class Sampler:
         self._dev = None       # the parameters' place on the device, and the pinned buffers they come from
         self._host, self._events, self._used, self._next = [], [], [], 0
         self._rows, self._parts, self._pairs = -1, (), []      # views of the buffers for a batch of _rows rows
-        self._packed_rows, self._pack = -1, None               # what packs the parameters of a batch of _packed_rows rows
+        self._packer = (-1, None)                              # rows of a batch, and what packs their parameters
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                token_indices: Sequence[int],
@@ -37,7 +37,8 @@ class Sampler:
         """logits float32 [R, V] (modified in place when a penalty applies); ``seeds[r]`` the
         request's resolved seed (>= 0); ``token_indices[r]`` how many tokens the request has
         generated before this one; ``generated[r]`` its generated ids (for the penalty).
-        Returns int32 [R] on the device."""
+        Returns int32 [R] on the device.  The rows' parameters are read now, not when the kernel runs: a CUDA graph that
+        captures this call draws with the same seeds, indices and parameters at every replay."""
         n = logits.shape[0]
         out = torch.empty(n, dtype=torch.int32, device=logits.device)
         if n == 0:
@@ -56,33 +57,34 @@ class Sampler:
                 pen = np.asarray([p.repetition_penalty for p in params], dtype=np.float32)
                 ops.repetition_penalty(logits, torch.from_numpy(ids).to(logits.device),
                                        torch.from_numpy(pen).to(logits.device))
-        if n <= ops.SAMPLE_VALUE_ROWS and self._with_the_launch(logits, out, params, seeds, token_indices):
+        words = self._words(params, seeds, token_indices)
+        if words is not None and ops.sample_values(logits, out, words):
+            self.h2d_bytes += len(words)
             return out
-        seed_t, count_t, temp_t, top_p_t, top_k_t = self._upload(logits.device, params, seeds, token_indices)
+        seed_t, count_t, temp_t, top_p_t, top_k_t = self._upload(logits.device, params, seeds, token_indices, words)
         ops.sample(logits, out, temp_t, top_k_t, top_p_t, seed_t, count_t)
         return out
 
-    # Up to 64 rows' parameters are arguments of the launch: 26 us of host work with the copy below, its buffers and events, 13 so.
-    def _with_the_launch(self, logits, out, params, seeds, token_indices) -> bool:
+    # The parameters side by side: seeds int64 [n], token counters int64 [n], temperature, top_p float32 [n], top_k int32 [n] (None:
+    # something that only numpy's conversions take, or refuse).  Up to 64 rows' are arguments of the launch: 20 us of host work with the
+    # copy below, its buffers and events, 9 so.
+    def _words(self, params, seeds, token_indices):
         n = len(params)
-        if self._packed_rows != n:
-            self._pack, self._packed_rows = struct.Struct(f"<{n}Q{n}q{n}f{n}f{n}i").pack, n
+        rows, pack = self._packer
+        if rows != n:
+            pack = struct.Struct(f"<{n}Q{n}q{n}f{n}f{n}i").pack
+            self._packer = (n, pack)
         try:
-            words = self._pack(*seeds, *token_indices, *[p.temperature for p in params], *[p.top_p for p in params],
-                               *[p.top_k for p in params])
-        except (OverflowError, struct.error, TypeError):        # what only the conversions of numpy take (or refuse)
-            return False
-        if not ops.sample_values(logits, out, words):
-            return False
-        self.h2d_bytes += 28 * n
-        return True
+            return pack(*seeds, *token_indices, *[p.temperature for p in params], *[p.top_p for p in params],
+                        *[p.top_k for p in params])
+        except (OverflowError, struct.error, TypeError):
+            return None
 
-    # More rows' parameters travel in ONE copy from pinned memory (a copy from pageable memory would
-    # hold the host until the stream has run everything before it - the whole step).  Words of 4
-    # bytes: seeds int64 [n], token counters int64 [n], temperature, top_p float32 [n], top_k int32 [n].
+    # More rows' parameters, and those for vocabularies that the kernel does not take so, travel in ONE copy from pinned memory (a
+    # copy from pageable memory would hold the host until the stream has run everything before it - the whole step).
     _RING = 4
 
-    def _upload(self, device, params, seeds, token_indices):
+    def _upload(self, device, params, seeds, token_indices, packed=None):
         n = len(params)
         words = 7 * n
         if self._dev is None or self._dev.numel() < words:
@@ -105,10 +107,10 @@ class Sampler:
             self._pairs = [(d, host[:words], host.numpy()) for host in self._host]
             self._rows = n
         d, h, words_of = self._pairs[i]
-        try:
-            struct.pack_into(f"<{n}Q{n}q{n}f{n}f{n}i", words_of, 0, *seeds, *token_indices, *(p.temperature for p in params),
-                             *(p.top_p for p in params), *(p.top_k for p in params))
-        except (OverflowError, struct.error, TypeError):        # what only the conversions of numpy take (or refuse)
+        packed = self._words(params, seeds, token_indices) if packed is None else packed
+        if packed is not None:
+            words_of[:words] = np.frombuffer(packed, dtype=np.int32)
+        else:
             words_of[0:2 * n].view(np.int64)[:] = np.asarray(seeds, dtype=np.uint64).view(np.int64)
             words_of[2 * n:4 * n].view(np.int64)[:] = np.asarray(token_indices, dtype=np.int64)
             words_of[4 * n:5 * n].view(np.float32)[:] = [p.temperature for p in params]

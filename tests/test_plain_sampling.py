@@ -1,4 +1,5 @@
 """The plain selection itself (no GPU)."""
+import pytest
 import torch
 
 import plain_sampling as ps
@@ -44,3 +45,23 @@ def test_sampler_packs_the_rows_parameters_into_one_buffer():
             assert torch.allclose(top_p_t, torch.tensor([1.0 / (r + 1) for r in range(n)]))
             assert top_k_t.dtype == torch.int32 and top_k_t.tolist() == [r - 1 for r in range(n)]
     assert s.h2d_bytes == 6 * 28 * (1 + 3 + 5 + 70)
+
+
+@pytest.mark.parametrize("rows", [3, 70])
+def test_parameters_are_packed_once_whichever_way_they_travel(rows, monkeypatch):
+    """A vocabulary or a batch that does not take them with the launch gets the same words by the copy."""
+    from nanoinfer_b200.kernels import ops
+    from nanoinfer_b200.sampling import Sampler, SamplingParams
+    params = [SamplingParams(temperature=0.5 + r, top_k=r, top_p=0.25, seed=r) for r in range(rows)]
+    seeds, at = [2 ** 63 + r for r in range(rows)], [5 - r for r in range(rows)]
+    for offered in (False, True):
+        sampler, packs, drawn, taken = Sampler(100, torch.device("cpu")), [], [], []
+        words = sampler._words
+        monkeypatch.setattr(sampler, "_words", lambda *a: packs.append(words(*a)) or packs[-1])
+        monkeypatch.setattr(ops, "sample_values", lambda logits, out, w: taken.append(w) is None and offered)
+        monkeypatch.setattr(ops, "sample", lambda logits, out, t, k, p, s, c: drawn.append((t.tolist(), k.tolist(), p.tolist(), s.tolist(), c.tolist())))
+        monkeypatch.setattr(ops, "current_stream_object", lambda: None)
+        sampler.sample(torch.zeros(rows, 100), params, seeds, at)
+        assert len(packs) == 1 and len(packs[0]) == 28 * rows == sampler.h2d_bytes and taken == packs
+        want = ([p.temperature for p in params], [p.top_k for p in params], [0.25] * rows, [s - 2 ** 64 for s in seeds], at)
+        assert drawn == ([] if offered else [want])
