@@ -14,11 +14,11 @@
 // ones and zeros comes back bit for bit.  (Two tf32 parts and three products, which lose two of the 24 bits: 3.0e-7 and 3.7e-7,
 // rows of ten terms 1.8e-7, of one 1.7e-7.)
 //
-// What bounds it: at many rows shared memory (the boxes, the parts of x and the MMAs' reads of them) and the cutting: 1,087 rows and
-// [16384, 2048] 416 us (175 TFLOP/s; two tf32 parts 418, chains on CUDA cores 1,417), 177 rows 107 (116); at few the weights,
-// [128256, 2048] 174 us (6.0 TB/s; 174; the ring of chains 177, at 8 rows 239), and for small matrices the way of one block: 6 us
-// of start, first load and last sum, 0.7 us for 64 columns ([2048, 2048] 13.0 us alone (12.1), less behind a kernel that lets it start
-// early).
+// What bounds it: at many rows cutting and multiplying, which have two boxes to hand over (tensor pipe busy 53 % of the time, ALU
+// 47 %): 1,087 rows and [16384, 2048] 408 us (179 TFLOP/s; two tf32 parts 418, chains on CUDA cores 1,419), 177 rows 106 (116); at few the weights,
+// [128256, 2048] 169 us (6.2 TB/s; 174; the ring of chains 177, at 8 rows 239), and for small matrices the way of one block: 6 us
+// of start, first load and last sum, 0.66 us for 64 columns ([2048, 2048] 12.5 us alone (12.1; one row as a chain 8.0, whose bits a row among
+// many would not have), less behind a kernel that lets it start early).
 //
 // The 128 lanes of the tcgen05 tile are weight rows, its columns BT rows of x (16 .. 128): few rows read the weights once, at
 // many rows 128 x 128 tiles.  Blocks are persistent; a block's warps:
@@ -182,32 +182,25 @@ __device__ __forceinline__ void gt_st_cluster(const float* mine, uint32_t rank, 
     asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote), "f"(v) : "memory");
 }
 
-// Pairs of numbers, for packed arithmetic.
-typedef unsigned long long GtPair;
-__device__ __forceinline__ GtPair gt_pair(float a, float b) {
-    GtPair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ GtPair gt_fma(GtPair a, GtPair b, GtPair c) {
-    GtPair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ GtPair gt_sub(GtPair a, GtPair b) { return gt_fma(b, gt_pair(-1.f, -1.f), a); }
 // The three parts of eight numbers, in pairs of bfloat16.  Each is what is left rounded to nearest, so that three hold all 24 bits.  What
-// is not finite, or rounds beyond bfloat16's range, has a NaN among its parts.
+// is not finite, or rounds beyond bfloat16's range, has a NaN among its parts.  What is left comes from multiply-adds that read a
+// bfloat16 number as it lies: fewer instructions than packed subtractions of it as FP32, same bits (2 rows and [16384, 2048] 30.4 us
+// instead of 31.7, 1,087 rows 449 instead of 470 in turn).
 __device__ __forceinline__ void gt_cut(const float4& a, const float4& b, uint4 part[3]) {
-    GtPair v[4] = {gt_pair(a.x, a.y), gt_pair(a.z, a.w), gt_pair(b.x, b.y), gt_pair(b.z, b.w)};
+    float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         uint32_t h[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float lo, hi;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v[j]));
+            float &lo = v[2 * j], &hi = v[2 * j + 1];
             asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h[j]) : "f"(hi), "f"(lo));
-            if (i < 2) v[j] = gt_sub(v[j], gt_pair(__uint_as_float(h[j] << 16), __uint_as_float(h[j] & 0xffff0000u)));
+            if (i < 2)
+                asm("{\n.reg .b16 l, h, m;\n"
+                    "mov.b32 {l, h}, %2;\n"
+                    "mov.b16 m, 0xBF80;\n"                          // -1
+                    "fma.rn.f32.bf16 %0, l, m, %0;\n"
+                    "fma.rn.f32.bf16 %1, h, m, %1;\n}\n" : "+f"(lo), "+f"(hi) : "r"(h[j]));
         }
         part[i] = make_uint4(h[0], h[1], h[2], h[3]);
     }
@@ -766,10 +759,10 @@ static int gt_clusters(int splits) {
     return cached[dev][splits];
 }
 
-// The tile and the split of K that are done first by what they measured: a k-block of 64 takes a block 0.70, 0.82, 1.02 and 1.55 us
+// The tile and the split of K that are done first by what they measured: a k-block of 64 takes a block 0.66, 0.77, 1.02 and 1.50 us
 // with 16, 32, 64 and 128 rows of x (128 weight rows; 0.74 us is what memory gives every SM for its 32 KB), a launch 6 us besides, and
-// a cluster 1.5 us, 0.045 us for every row and 0.01 for every row and slice of a block's sums.  [2048, 2048] and 120 rows: 19.2 us in
-// four slices of 64-row tiles, 38 whole; [2048, 8192] and 2 rows: 26.6 in six slices, 31.9 in four, 98 whole.
+// a cluster 1.5 us, 0.045 us for every row and 0.01 for every row and slice of a block's sums.  [2048, 2048] and 120 rows: 18.9 us in
+// four slices of 64-row tiles, 38 whole; [2048, 8192] and 2 rows: 24.4 in six slices, 30 in four, 91 whole.
 static void gt_choose(const GtParams& p, int& bt, int& splits) {
     const int slices = gt_slices(p.K);
     const long long n_tiles = (long long)((p.N + GT_ROWS - 1) / GT_ROWS) * p.H;
@@ -779,7 +772,7 @@ static void gt_choose(const GtParams& p, int& bt, int& splits) {
     for (int i = 0; i < 4; ++i) {
         const int b = 16 << i;
         if (want_bt ? b != want_bt : (b > 16 && b >= 2 * p.M)) continue;
-        const double per_block = i == 0 ? 0.70 : i == 1 ? 0.82 : i == 2 ? 1.02 : 1.55;
+        const double per_block = i == 0 ? 0.66 : i == 1 ? 0.77 : i == 2 ? 1.02 : 1.50;
         const long long units = n_tiles * ((p.M + b - 1) / b);
         for (int sp = 1; sp <= 8; ++sp) {
             if (want_splits ? sp != want_splits : sp > 1 && units * sp > 4LL * ni_sm_count()) continue;

@@ -577,8 +577,8 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int =
 # Rows of at least this many columns go to the tensor cores as numbers cut in three, shorter ones to the chains of csrc/gemm_f32.cu.  The
 # rule looks at nothing but the row's length, so that a row's bits depend on no other row.  Relative error against 64 bits, cut in
 # three / as a chain: normal numbers 0.9e-7 / 4.1e-7 at 512 columns, 0.9e-7 / 5.7e-7 at 1,024, 1.3e-7 / 1.6e-6 at 8,192; rows of a
-# single term 2.6e-8 / 2.5e-8.  us for 2,048 weight rows: 512 columns, 1 row of x 8.7 / 3.8, 177 rows 12.7 / 22.7; 1,024 columns 8.6 / 5.3 and
-# 19.7 / 38.6.  Below the line single tokens lose more than the prompts' products are worth.
+# single term 2.6e-8 / 2.5e-8.  us for 2,048 weight rows: 512 columns, 1 row of x 8.0 / 3.8, 177 rows 11.7 / 22.6; 1,024 columns 8.2 / 5.4 and
+# 18.3 / 38.9.  Below the line single tokens lose more than the prompts' products are worth.
 F32_CUT_COLUMNS = 1024
 
 
