@@ -19,8 +19,8 @@
 // lone warp per scheduler, which issues nothing else for 8 clocks while one of its 162 MMAs enters the tensor core.  (Four warps per 16
 // columns: 148 us instead of 129 at the time, since their products come in the same phases; FP32 multiply-adds in the same tiles: 183 us.)
 //
-// Portions of 1,201 and 847 tokens, 16 heads of 128: 178 us with the preparation (53), against 251 us in blocks of four; 2,048 tokens 255
-// (342), 8 x 512 269 (335), 512 75 (94).  Error against 64 bits of the whole rule, read-outs / states, means over eight inputs of up to
+// Portions of 1,201 and 847 tokens, 16 heads of 128: 170 us with the preparation (51), against 245 us in blocks of four; 2,048 tokens 247
+// (337), 8 x 512 260 (328), 512 69 (89); 2,048 tokens of 4 heads 213 (314), of 64 511 (669).  Error against 64 bits of the whole rule, read-outs / states, means over eight inputs of up to
 // 1,100 tokens: decays of a few tokens 1.2e-7 / 1.1e-7 (blocks of four 1.3e-7 / 1.2e-7), of some tens 1.1e-7 / 1.2e-7 (1.4e-7 / 1.5e-7),
 // of some hundreds 1.3e-7 / 1.5e-7 (3.0e-7 / 4.5e-7), decays near one 1.6e-7 / 1.8e-7 (1.7e-6 / 2.7e-6).  Decays and beta in 64 bits and
 // the keys' norms with one step of Newton's method are worth more than what the cuts cost (in FP32: states 1.07 times the error of

@@ -1,4 +1,5 @@
-// out[M, N] = x[M, K] . w[N, K]^T in true FP32: FFMA on CUDA cores, no tensor-core mode.
+// out[M, N] = x[M, K] . w[N, K]^T in true FP32: FFMA on CUDA cores, no tensor-core mode.  The 32-bit path's products over rows of
+// fewer than 1,024 columns; longer rows go to gemm_f32_tc.cu.
 //
 // The reference calls cublasSgemm with the default math mode for every projection
 // (src/op/kernels/cuda/matmul_kernel.cu:48-89).  These kernels keep the FP32 path free of
@@ -300,7 +301,8 @@ static int gf_launch_ring(const float* x, const float* w, float* out, int M, int
 }
 
 // Up to 16 rows the narrowest ring that holds them all: weights are read once.  Beyond, the ring's 32 x 16 tiles (three
-// blocks per SM) or the 64 x 128 tiles, whichever is done first by what they measured at K = 2,048 (both go with K):
+// blocks per SM) or the 64 x 128 tiles, whichever is done first by what they measured at K = 2,048 (both go with K, which
+// is below 1,024 in the 32-bit path itself):
 // a ring tile takes 34 us alone and 0.077 us each once the SMs are full, a 64 x 128 tile 128 us and 0.64 us.  [2048, K]
 // weights: 64 rows 37 / 130 us, 177 rows 74 / 130 us, 256 rows 99 / 130 us, 512 rows 200 / 130 us; [16384, K]: 17 rows
 // 103 / 130 us, 64 rows 170 / 132 us.  Before (64 x 64 tiles of 4 x 4 outputs per thread, one k-step of 16 at a time): 190 us and

@@ -1,7 +1,9 @@
 """Runtime: device, compute dtype and the matrix products of the forward pass.
 
-float32 is a true 32-bit path: every product runs through the package's own FFMA kernel
-and no reduced-precision tensor-core mode is ever switched on.  bfloat16 keeps weights,
+float32 is a true 32-bit path: every product runs through the package's own kernels - dense
+products over rows of 1,024 and more columns on the tensor cores with every number cut into three
+bfloat16 numbers that hold all of its 24 bits, shorter rows and the experts' products as FFMA
+chains - and no reduced-precision mode is ever switched on.  bfloat16 keeps weights,
 activations and cache in bfloat16 with FP32 accumulation; the residual stream, norm
 statistics, softmax and rotation angles stay FP32 in both.
 """

@@ -23,6 +23,8 @@
     python -m nanoinfer_b200.kernels.microbench hyper --rows 2048 --width 2048 --streams 4 --top 4
     python -m nanoinfer_b200.kernels.microbench attention_prefill --tokens 2048 --q-heads 16 --head-dim 128 --difference
     python -m nanoinfer_b200.kernels.microbench attention_decode --batch 8 --context 2048 --q-heads 16 --head-dim 128 --difference
+    python -m nanoinfer_b200.kernels.microbench gemm_f32 --m 1087 --n 16384 --k 2048
+    python -m nanoinfer_b200.kernels.microbench delta_tile --tokens 1201 847 --heads 16
 
 Each case runs its kernel over several distinct copies of its inputs in turn (together
 larger than the L2 cache, so every run reads from HBM), times it with CUDA events after
@@ -126,6 +128,39 @@ def sample(args) -> None:
     ops.sample_by_cluster(True)
     print(f"sample{' (one block per row)' if args.one_block else ' (a cluster per row)'} rows={n} vocab={v} temperature={args.temperature} "
           f"top_k={args.top_k} top_p={args.top_p}: {us:.1f} us")
+
+
+def gemm_f32(args) -> None:
+    """A product of FP32 matrices: on the tensor cores, every number cut in three, and as chains of multiply-adds."""
+    m, n, k = args.m, args.n, args.k
+    g = torch.Generator(device=DEV).manual_seed(0)
+    copies = max(2, min(24, -(-2 * L2_BYTES // (n * k * 4))))
+    ws = [torch.randn(n, k, device=DEV, generator=g) for _ in range(copies)]
+    x, out = torch.randn(m, k, device=DEV, generator=g), torch.empty(m, n, device=DEV)
+    us = _time([lambda w=w: ops.gemm_f32_tc(x, w, out, args.rows, args.splits, constant_w=True) for w in ws], args.iters)
+    chain = "" if args.no_chain else f"; chains {_time([lambda w=w: ops.gemm_f32(x, w, out) for w in ws], args.iters):.2f} us"
+    print(f"gemm_f32 m={m} n={n} k={k}: cut in three {us:.2f} us ({n * k * 4 / us / 1e3:.0f} GB/s of weights, {2 * m * n * k / us / 1e6:.1f} "
+          f"TFLOP/s){chain} ({copies} weight copies in turn)")
+
+
+def delta_tile(args) -> None:
+    """The gated delta rule with a decay per head over portions of --tokens tokens, preparation included: sixteen tokens at a
+    time and in blocks of four."""
+    G, H, V, taps, n = args.kv_heads or args.heads, args.heads, args.vdim, 4, sum(args.tokens)
+    C = 2 * G * 128 + H * V
+    g = torch.Generator(device=DEV).manual_seed(0)
+    proj = torch.randn(n, C + 2 * H, device=DEV, generator=g)
+    conv_w = torch.randn(C, taps, device=DEV, generator=g) * 0.5
+    a_log, dt_bias = torch.zeros(H, device=DEV), torch.zeros(H, device=DEV)
+    states = [torch.randn(len(args.tokens), H * 128 * V + (taps - 1) * C, device=DEV, generator=g) * 0.1 for _ in range(2)]
+    cu = torch.tensor([0] + [sum(args.tokens[:i + 1]) for i in range(len(args.tokens))], dtype=torch.int32, device=DEV)
+    slots, out = torch.arange(len(args.tokens), dtype=torch.int32, device=DEV), torch.empty(n, H * V, device=DEV)
+    buf = torch.empty(sum(ops.delta_tile_bytes(n, len(args.tokens), G, H, V)), dtype=torch.uint8, device=DEV)
+    tiles, blocks = (_time([lambda st=st: ops.delta_block_recurrence(proj, 0, C, C + H, conv_w, a_log, dt_bias, st, cu, slots, len(args.tokens), G, H,
+                                                                     128, V, taps, out, tiles=t, buf=buf if t else None) for st in states], args.iters)
+                     for t in (True, False))
+    print(f"delta_tile tokens={args.tokens} heads={H}/{G} vdim={V}: sixteen at a time {tiles:.1f} us, four {blocks:.1f} us "
+          f"(chosen: {'sixteen' if ops.delta_tile_pays(n, len(args.tokens), 128, V, H, max(args.tokens)) else 'four'})")
 
 
 def gemm(args) -> None:
@@ -752,6 +787,20 @@ def main() -> None:
     p.add_argument("--top-p", type=float, default=1.0)
     p.add_argument("--one-block", action="store_true")
     p.set_defaults(fn=sample)
+    p = sub.add_parser("gemm_f32")
+    p.add_argument("--m", type=int, default=1087)
+    p.add_argument("--n", type=int, default=16384)
+    p.add_argument("--k", type=int, default=2048)
+    p.add_argument("--rows", type=int, default=0, help="rows of x in a tile (16, 32, 64, 128; 0: by the sizes)")
+    p.add_argument("--splits", type=int, default=0, help="blocks that share K (0: by the sizes)")
+    p.add_argument("--no-chain", action="store_true")
+    p.set_defaults(fn=gemm_f32)
+    p = sub.add_parser("delta_tile")
+    p.add_argument("--tokens", type=int, nargs="+", default=[2048], help="tokens of each request")
+    p.add_argument("--heads", type=int, default=16)
+    p.add_argument("--kv-heads", type=int, default=0, help="heads of q and k (0: as many)")
+    p.add_argument("--vdim", type=int, default=128)
+    p.set_defaults(fn=delta_tile)
     p = sub.add_parser("add_rmsnorm")
     p.add_argument("--rows", type=int, default=2048)
     p.add_argument("--width", type=int, default=2048)
